@@ -10,19 +10,32 @@
 //                  r = I2(x + sum_a N_a u_c[a]) - I1,
 //                the chunk's sum r^2 (double-float) and its 8 nodal gradient
 //                partials sum r * dI2/dx * N_a (FP32), written to the chunk's
-//                own node slots; then it counts its chunks into the node
-//                groups (32 nodes) they touch.  No atomics on data.
-//   node work    the warp that owns a group waits (bounded) until every chunk
-//                of the group has counted, gathers each node's slots, adds the
-//                spring gradient over the neighbour table, writes the trial
-//                gradient, point and direction, and reduces (fixed order) sum
-//                r^2, spring energy, g.g, g.(g - g_cur), g_cur.dir; the warp
-//                that completes a supergroup of 16 groups reduces it, and the
-//                warp that completes a frame's last supergroup runs the CG
-//                control of d2ic/solver_global_cg.py:362-461 (stop test, PR+
-//                beta, restart on g.d >= 0, Armijo with 10 halvings and the
-//                forced 2^-10 step); the frame's round counter releases the
-//                next round.
+//                own node slots as 16-byte records that carry the evaluation's
+//                tag.  No atomics on data, no fence.
+//   node work    the warp that owns a group of 32 nodes polls (bounded) the
+//                group's slots until every chunk that touches it has written
+//                this evaluation's records, adds the spring gradient over the
+//                neighbour table, writes the trial gradient, point and
+//                direction, and reduces (fixed order) sum r^2, spring energy,
+//                g.g, g.(g - g_cur), g_cur.dir; the warp that completes a
+//                supergroup of 16 groups reduces it and publishes its sums as
+//                tagged records.
+//   control      one warp per frame waits for the supergroup records and runs
+//                the CG control of d2ic/solver_global_cg.py:362-461 (stop test,
+//                PR+ beta, restart on g.d >= 0, Armijo with 10 halvings and
+//                the forced 2^-10 step); the round's last frame releases the
+//                next round with one tagged record, which also carries the
+//                next candidate rule when a single frame is active.
+//
+// A round of a small frame is a chain of such hand-overs.  With counters and
+// fences (count the chunks of a group, poll the counter, gather; supergroup
+// and frame counters; state, fence, release word, header and state read back)
+// it took 17.9 us on a 512 x 512 frame with 16-px elements, 23.5 us at
+// 1024 x 1024 and 41.1 us at 2048 x 2048; with tagged records, rolled and
+// smaller once-per-round code and even shares of the chunks 11.6, 14.0 and
+// 31.4 us.  What bounds it now: the L2 round trips of the hand-overs (about
+// 0.7 us each), the fences that order the node data (0.4 us each) and, from
+// 2048 x 2048 on, the pixel pass.
 //
 // Because every partial is written to its own slot and reduced in an order
 // fixed by the frame's own data layout, a frame's result does not depend on
@@ -85,7 +98,7 @@ struct CtlHeader {
     int n_active;
     int total_chunks;
     int total_groups;
-    unsigned rounds_done;   // rounds completed in this launch (released by the round's last frame step)
+    int pad0_;
     int finished;           // a frame finished in this round: the active list is rebuilt before release
     int max_rounds;
     int frames_done;        // frames whose control step ran in the current round
@@ -93,9 +106,10 @@ struct CtlHeader {
     int irq;                // written by the host while a slice runs: end the slice at the next round end
     int list_buf;           // which of the two copies of the active list the current round reads
     unsigned blocks_past;   // block arrivals at round ends: every block has finished a round's list reads
-    int pad_;
+    int pad_[17];
+    uint4 rel;              // the release record of the last completed round, on a cache line of its own
 };
-static_assert(sizeof(CtlHeader) == 64, "control header layout");
+static_assert(sizeof(CtlHeader) == 144 && offsetof(CtlHeader, rel) == 128, "control header layout");
 
 // stop_flags of a slice: end it early
 enum { STOP_ON_FINISH = D2IC_STOP_ON_FINISH,   // after a round in which a frame finished
@@ -165,6 +179,57 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
 
 __device__ __forceinline__ int ld_vol(const int *p) { return *(volatile const int *)p; }
 
+// Orders this thread's earlier accesses (and those it has observed) before its later ones for the GPU:
+// the acquire/release fence, lighter than __threadfence(), which is sequentially consistent.
+__device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
+// Warp sums of five double-floats by a reduce-scatter butterfly: at the exchange distances 16, 8 and 4
+// a lane keeps half of its values and adds its partner's copy of that half, so the five sums take 8
+// double-float additions instead of 25; the additions of each sum are those of df_warp_sum, so the bits
+// are the same.  Lane l returns sum red5_value(l), each sum in four lanes (-1: none).  (This code runs
+// once per round on one warp of an SM: its instruction count is latency.)
+__device__ __forceinline__ int red5_value(int lane) {
+    const int k = lane >> 2;               // lanes 0-3: sum 0, 4-7: 1, 8-11: 2, 16-19: 3, 20-23: 4
+    return k < 3 ? k : (k == 4 ? 3 : (k == 5 ? 4 : -1));
+}
+__host__ __device__ constexpr int red5_lane(int k) { return k < 3 ? 4 * k : 4 * k + 4; }
+__device__ __forceinline__ DF df_shfl_xor(DF v, int o) {
+    return DF{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
+}
+__device__ __forceinline__ DF df_reduce5(const DF q[5], int lane) {
+    const DF z = {0.f, 0.f};
+    const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0, b2 = (lane & 4) != 0;
+    const DF a0 = df_add(b4 ? q[3] : q[0], df_shfl_xor(b4 ? q[0] : q[3], 16));
+    const DF a1 = df_add(b4 ? q[4] : q[1], df_shfl_xor(b4 ? q[1] : q[4], 16));
+    const DF a2 = df_add(b4 ? z : q[2], df_shfl_xor(b4 ? q[2] : z, 16));
+    const DF c0 = df_add(b3 ? a2 : a0, df_shfl_xor(b3 ? a0 : a2, 8));
+    const DF c1 = df_add(b3 ? z : a1, df_shfl_xor(b3 ? a1 : z, 8));
+    DF v = df_add(b2 ? c1 : c0, df_shfl_xor(b2 ? c0 : c1, 4));
+    v = df_add(v, df_shfl_xor(v, 2));
+    return df_add(v, df_shfl_xor(v, 1));
+}
+
+// 16-byte records that carry their own round tag: one 128-bit access is a single memory operation
+// (ld/st.b128 of the PTX memory model), so a reader that finds the tag has the data of the same
+// write.  A producer therefore needs no fence and no counter to hand over a record, and the
+// consumer polls the record itself: one L2 round trip from the store to the value, instead of
+// store, fence, atomic, polled counter, load.
+__device__ __forceinline__ uint4 ld_record(const void *p) {
+    unsigned long long lo, hi;
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(lo), "=l"(hi)
+                 : "l"(p)
+                 : "memory");
+    return make_uint4((unsigned)lo, (unsigned)(lo >> 32), (unsigned)hi, (unsigned)(hi >> 32));
+}
+__device__ __forceinline__ void st_record(void *p, uint4 v) {
+    const unsigned long long lo = (unsigned long long)v.x | ((unsigned long long)v.y << 32);
+    const unsigned long long hi = (unsigned long long)v.z | ((unsigned long long)v.w << 32);
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+                 "l"(lo), "l"(hi)
+                 : "memory");
+}
+
 // Control data is rewritten by other blocks during the launch: read it through
 // L2 (never a possibly stale L1 line).
 __device__ __forceinline__ FrameState load_fs(const FrameState *p) {
@@ -206,7 +271,9 @@ __device__ __forceinline__ float2 cand_value(float2 un, float2 gn, float2 dn, fl
 struct FInfo {
     float alpha, beta;
     int mode, iu, igc, idp, igt;
+    unsigned tag;   // this evaluation's tag: the frame's evaluations so far, plus one (28 bits used)
 };
+constexpr unsigned TAG_MASK = 0x0fffffffu;
 __device__ __forceinline__ FInfo frame_info(const FrameState *S) {
     FInfo fi;
     fi.iu = __ldcg(&S->iu);
@@ -217,8 +284,39 @@ __device__ __forceinline__ FInfo frame_info(const FrameState *S) {
     fi.alpha = __ldcg(&S->alpha);
     fi.beta = __ldcg(&S->beta);
     fi.mode = (st == ST_EVAL) ? 0 : ((rs || k == 0) ? 2 : 1);
+    fi.tag = ((unsigned)__ldcg(&S->n_evals) + 1u) & TAG_MASK;
     return fi;
 }
+
+// The release of a round: one record, polled by one thread of every block.  x: rounds completed in
+// this launch; y: bit 0 the launch's slice ends, bit 1 the candidate rule of the only active frame
+// is in the record (mode, buffer indices in bits 2-9; alpha, beta in z, w), bits 16-31 the version
+// of the active list.  With several active frames the rules are read from the frame states.
+constexpr unsigned REL_STOP = 1u, REL_INLINE = 2u;
+enum { REFRESH_NONE = 0, REFRESH_RULES = 1, REFRESH_LIST = 2 };   // what a block reads after a release
+__device__ __forceinline__ unsigned rel_pack(const FInfo &fi) {
+    return REL_INLINE | ((unsigned)fi.mode << 2) | ((unsigned)fi.iu << 4) | ((unsigned)fi.igc << 5) |
+           ((unsigned)fi.igt << 7) | ((unsigned)fi.idp << 9);
+}
+
+// A candidate rule as a block keeps it in shared memory, 16 bytes.
+struct FRule {
+    float alpha, beta;
+    unsigned packed, tag;   // packed: as in the release record
+    __device__ __forceinline__ FInfo info() const {
+        FInfo fi;
+        fi.alpha = alpha;
+        fi.beta = beta;
+        fi.tag = tag;
+        fi.mode = (int)((packed >> 2) & 3u);
+        fi.iu = (int)((packed >> 4) & 1u);
+        fi.igc = (int)((packed >> 5) & 3u);
+        fi.igt = (int)((packed >> 7) & 3u);
+        fi.idp = (int)((packed >> 9) & 1u);
+        return fi;
+    }
+};
+__device__ __forceinline__ FRule make_rule(const FInfo &fi) { return FRule{fi.alpha, fi.beta, rel_pack(fi), fi.tag}; }
 
 struct Cand {
     const float2 *u, *g, *d;
@@ -409,8 +507,7 @@ struct ChunkMeta {
     int box0, box1, tile;            // packed pixel-box corners and tile origin (col | row << 16)
 };
 
-__device__ __forceinline__ ChunkMeta load_meta(const d2ic_frame_t *frames, int f, int c, int lane) {
-    const d2ic_frame_t &F = frames[f];
+__device__ __forceinline__ ChunkMeta load_meta(const d2ic_frame_t &F, int f, int c, int lane) {
     ChunkMeta m;
     m.s = 0;
     m.f = f;
@@ -454,7 +551,8 @@ __device__ __forceinline__ int atom_acq_rel_add(int *p, int v) {
 
 template <int KIND>
 __device__ __forceinline__ void chunk_compute(const d2ic_frame_t &F, const ChunkMeta &m, float2 uc, const Stage &st,
-                                              const uint4 *srec, const float *tile, int lane) {
+                                              const uint4 *srec, const float *tile, int lane,
+                                              const unsigned *tag_at) {
     const bool staged = st.staged;
     const bool tiled = KIND == D2IC_INTERP_CUBIC && st.tiled;
     const int tw = F.tile_w, th = F.tile_h, tx0 = st.tx0, ty0 = st.ty0;
@@ -549,15 +647,11 @@ __device__ __forceinline__ void chunk_compute(const d2ic_frame_t &F, const Chunk
             const int p = lane + 32 * i;
             if (p < n) one_fast(srec[p]);
         }
-    } else if (staged) {
-#pragma unroll 4
-        for (int i = 0; i < D2IC_CHUNK_MAX / 32; ++i) {
-            const int p = lane + 32 * i;
-            if (p < n) one(srec[p]);
-        }
-        for (int p = lane + D2IC_CHUNK_MAX; p < n; p += 32) one(__ldg(gpix + p));   // beyond the staged buffer
     } else {
-        for (int p = lane; p < n; p += 32) one(__ldg(gpix + p));
+        // boundary chunks and the first pass: one copy of the general per-pixel code (this loop's body
+        // is several times the fast one's; the instruction cache matters more here than its speed)
+#pragma unroll 1
+        for (int p = lane; p < n; p += 32) one(staged && p < D2IC_CHUNK_MAX ? srec[p] : __ldg(gpix + p));
     }
     const DF js = df_warp_sum(DF{jr, 0.f});
     // The 8 nodal partials summed over the warp by a reduce-scatter butterfly: at each of the
@@ -598,24 +692,27 @@ __device__ __forceinline__ void chunk_compute(const d2ic_frame_t &F, const Chunk
     const float gxs = __shfl_sync(0xffffffffu, v1, 8 * ((la >> 1) & 1) + 4 * (la & 1));
     const float gys = __shfl_sync(0xffffffffu, v1, 16 + 8 * ((la >> 1) & 1) + 4 * (la & 1));
     if (lane == 0 && tw > 0) F.chunk_tile[m.c] = tile_origin(m.box0, ux, uy);
-    // lane a stores node a's partial in the chunk's slot of that node; node 0's slot also
-    // carries the chunk's sum of r^2 (double-float), so every chunk is counted exactly once
-    if (lane < 4)
-        reinterpret_cast<float4 *>(F.node_grad)[(size_t)m.slot * F.n_nodes + m.nd] =
-            make_float4(gxs, gys, lane == 0 ? js.hi : 0.f, lane == 0 ? js.lo : 0.f);
+    // Lane a stores node a's partial in the chunk's slot of that node as one tagged record; the slots
+    // of nodes 0 and 1 also carry the two words of the chunk's sum of r^2, so every chunk is counted
+    // exactly once.  The last word holds the evaluation's tag and, for the waiting group (see
+    // gather_slots), whether this is the chunk's first node in its group and how many it has there.
+    {
+        const int grp = m.nd / GN;
+        int cnt = 0;
+        bool first = true;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const bool same = __shfl_sync(0xffffffffu, grp, a) == grp;
+            cnt += same;
+            first = first && !(same && a < lane);
+        }
+        if (lane < 4)
+            st_record(reinterpret_cast<float4 *>(F.node_grad) + (size_t)m.slot * F.n_nodes + m.nd,
+                      make_uint4(__float_as_uint(gxs), __float_as_uint(gys),
+                                 __float_as_uint(lane == 0 ? js.hi : (lane == 1 ? js.lo : 0.f)),
+                                 (*tag_at << 4) | ((unsigned)cnt << 1) | (first ? 1u : 0u)));
+    }
     __syncwarp();                                   // every lane is done with the staged buffers
-}
-
-// One count per distinct node group among a chunk's four nodes; the group's reducer waits
-// until it has as many counts as chunks touch the group.  Each quad of lanes (4 j .. 4 j + 3)
-// holds the node groups of one chunk (grp < 0: no chunk).
-__device__ __forceinline__ void count_chunk_groups_quad(int *group_cnt, int grp, int lane) {
-    const int q0 = lane & ~3, a = lane & 3;
-    const int g0 = __shfl_sync(0xffffffffu, grp, q0), g1 = __shfl_sync(0xffffffffu, grp, q0 + 1),
-              g2 = __shfl_sync(0xffffffffu, grp, q0 + 2);
-    const bool first = a == 0 || (a == 1 && grp != g0) || (a == 2 && grp != g0 && grp != g1) ||
-                       (a == 3 && grp != g0 && grp != g1 && grp != g2);
-    if (grp >= 0 && first) atomicAdd(group_cnt + grp, 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -675,27 +772,84 @@ __device__ __forceinline__ NodePre node_pre(const d2ic_frame_t &F, const FInfo &
     return p;
 }
 
-__device__ __forceinline__ void node_post(const d2ic_frame_t &F, const FInfo &fi, int n, const NodePre &p, DF q[5]) {
+// A node's sums over its K slots (slot order).
+struct SlotSums {
+    float x, y;
+    DF j;
+};
+
+// A bounded wait's periodic check (whole warp): false once the launch is aborted, or aborts it when
+// more than WAIT_NS have passed since the first check (t0, 0 before it).
+__device__ __forceinline__ bool keep_waiting(CtlHeader *H, unsigned long long &t0, int lane) {
+    int go = 1;
+    if (lane == 0) {
+        const unsigned long long now = gtimer();
+        if (t0 == 0) t0 = now;
+        if (ld_vol(&H->abort)) {
+            go = 0;
+        } else if (now - t0 > WAIT_NS) {
+            H->err = D2IC_WAIT_TIMEOUT;
+            atomicExch(&H->abort, 1);
+            go = 0;
+        }
+    }
+    return __shfl_sync(0xffffffffu, go, 0) != 0;
+}
+
+// Gathers the slots of a group's nodes (lane = node n) once every chunk that touches the group has
+// written this evaluation's records (whole warp; false after an abort or WAIT_NS).  The slots
+// themselves are polled: a slot that no chunk owns never carries the tag, so the group is complete
+// when `need` (chunks touching the group) first-node records have arrived and the records they
+// announce -- their chunks' nodes in this group -- are as many as the records that arrived.
+__device__ __forceinline__ bool gather_slots(const d2ic_frame_t &F, int n, int need, unsigned tag, CtlHeader *H,
+                                             SlotSums &s) {
+    const int K = F.node_chunk_k, Nn = F.n_nodes;
+    const float4 *ng = reinterpret_cast<const float4 *>(F.node_grad) + n;
+    constexpr int NB = 4;                              // K of elements that are one chunk each
+    const int lane = threadIdx.x & 31;
+    unsigned long long t0 = 0;
+    auto add = [&](const uint4 &v) {                   // absent records add zeros
+        s.x += __uint_as_float(v.x);
+        s.y += __uint_as_float(v.y);
+        s.j = df_add(s.j, DF{__uint_as_float(v.z), 0.f});
+    };
+    for (unsigned it = 0;; ++it) {
+        int acc = 0;                                   // arrived - announced in the low half, firsts above
+        uint4 v[NB];
+        s.x = s.y = 0.f;
+        s.j = DF{0.f, 0.f};
+        for (int kb = 0; kb < K; kb += NB) {
+#pragma unroll
+            for (int t = 0; t < NB; ++t)
+                v[t] = n < Nn && kb + t < K ? ld_record(ng + (size_t)(kb + t) * Nn) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (int t = 0; t < NB; ++t) {
+                const int x = (v[t].w & 1u) ? 0x10001 - (int)((v[t].w >> 1) & 7u) : 1;
+                acc += (v[t].w >> 4) == tag ? x : 0;
+            }
+            if (K > NB)                                // summed along the way; else once, when complete
+#pragma unroll
+                for (int t = 0; t < NB; ++t) add(v[t]);
+        }
+        const int sum = __reduce_add_sync(0xffffffffu, acc);
+        const int open = (int)(short)(sum & 0xffff), firsts = (sum - open) >> 16;
+        if (open == 0 && firsts >= need) {
+            if (K <= NB)
+#pragma unroll
+                for (int t = 0; t < NB; ++t) add(v[t]);
+            return true;
+        }
+        if ((it & 63) == 63 && !keep_waiting(H, t0, lane)) return false;
+    }
+}
+
+__device__ __forceinline__ void node_post(const d2ic_frame_t &F, const FInfo &fi, int n, const NodePre &p,
+                                          const SlotSums &s, DF q[5]) {
 #pragma unroll
     for (int i = 0; i < 5; ++i) q[i] = DF{0.f, 0.f};
     if (n >= F.n_nodes) return;
-    float sx = 0.f, sy = 0.f;
-    DF sj = {0.f, 0.f};
-    const int K = F.node_chunk_k, Nn = F.n_nodes;
-    const float4 *ng = reinterpret_cast<const float4 *>(F.node_grad) + n;
-    constexpr int NB = 8;
-    for (int kb = 0; kb < K; kb += NB) {
-        float4 v[NB];
-#pragma unroll
-        for (int t = 0; t < NB; ++t) v[t] = (kb + t < K) ? __ldcg(ng + (size_t)(kb + t) * Nn) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int t = 0; t < NB; ++t)
-            if (kb + t < K) {
-                sx += v[t].x;
-                sy += v[t].y;
-                sj = df_add(sj, DF{v[t].z, v[t].w});
-            }
-    }
+    const float sx = s.x, sy = s.y;
+    const DF sj = s.j;
     const float inv_np = 1.0f / (float)max(F.n_pix, 1);
     const float gx = sx * inv_np + F.alpha_reg * p.rx;
     const float gy = sy * inv_np + F.alpha_reg * p.ry;
@@ -712,25 +866,36 @@ __device__ __forceinline__ void node_post(const d2ic_frame_t &F, const FInfo &fi
 }
 
 // ---------------------------------------------------------------------------
-// R step (last block at the end-of-round barrier)
+// Control step (one warp per frame and round)
 // ---------------------------------------------------------------------------
 // The descriptor scalars the control step reads, loaded once at its start.
 struct FConst {
     float *hist;
-    double tol;
-    float alpha_reg;
-    int max_iter, n_pix;
+    double tol, tol2_hi;   // tol2_hi: squares at or above it are certainly not below tol
+    int max_iter;
 };
 
-// Values of a control step that need FP64 division or square root, computed for the whole
-// warp at once (GB300's FP64 pipe is narrow, so each FP64 instruction is costly): the
-// objective J of this round's point, and, for the state after accepting this point, sqrt(g.g)
-// and the PR+ ratio g.(g - g_prev) / (g_prev.g_prev + 1e-16).
+// Values of a control step, computed for the whole warp at once (GB300's FP64 pipe is narrow, so
+// each FP64 instruction is costly): the objective J of this round's point, the squared gradient norm
+// of the state after accepting this point and the PR+ ratio g.(g - g_prev) / (g_prev.g_prev + 1e-16).
 struct StepVals {
-    double J, gnorm, ratio;
+    double J, gg, ratio, armijo;   // armijo: 1e-4 alpha
 };
 
-__device__ void hist_row(const FConst &F, int k, double a, double b, double c) {
+// Tests on the bits of a double (an FP64 comparison costs tens of cycles on GB300).
+__device__ __forceinline__ bool is_nan64(double x) {
+    return ((unsigned long long)__double_as_longlong(x) << 1) > 0xffe0000000000000ull;
+}
+__device__ __forceinline__ bool is_neg64(double x) {   // x < 0 (not for -0 or NaN)
+    const long long b = __double_as_longlong(x);
+    return b < 0 && (b << 1) != 0 && !is_nan64(x);
+}
+__device__ __forceinline__ bool is_nonneg64(double x) {   // x >= 0 (also -0, not NaN)
+    const long long b = __double_as_longlong(x);
+    return (b >= 0 || (b << 1) == 0) && !is_nan64(x);
+}
+
+__device__ __forceinline__ void hist_row(const FConst &F, int k, double a, double b, double c) {
     if (F.hist && k < F.max_iter) {
         F.hist[3 * k + 0] = (float)a;
         F.hist[3 * k + 1] = (float)b;
@@ -738,7 +903,7 @@ __device__ void hist_row(const FConst &F, int k, double a, double b, double c) {
     }
 }
 
-__device__ void accept_point(FrameState &S, double J, double gg, double gdiff) {
+__device__ __forceinline__ void accept_point(FrameState &S, double J, double gg, double gdiff) {
     S.J_cur = J;
     S.gg_prev = S.gg_cur;
     S.gg_cur = gg;
@@ -751,19 +916,23 @@ __device__ void accept_point(FrameState &S, double J, double gg, double gdiff) {
     S.idp = 1 - S.idp;
 }
 
-// Called right after accept_point of this round's point, so v.gnorm = sqrt(S.gg_cur) and
-// v.ratio = S.gdiff_cur / (S.gg_prev + 1e-16).
-__device__ void start_iter(FrameState &S, const FConst &F, const StepVals &v) {
-    S.gnorm = v.gnorm;
-    if (S.gnorm < F.tol) {                       // stop branch: k unchanged
-        hist_row(F, S.k, S.J_cur, S.gnorm, 0.0);
-        S.state = ST_DONE;
-        return;
+// Called right after accept_point of this round's point, so v.gg = S.gg_cur and
+// v.ratio = S.gdiff_cur / (S.gg_prev + 1e-16).  The norm sqrt(g.g) itself is needed only for the stop
+// test and, later, the history: far above the tolerance the test is decided on the squares, and the
+// square root is taken after the release (S.gnorm < 0 marks it as open).
+__device__ __forceinline__ void start_iter(FrameState &S, const FConst &F, const StepVals &v) {
+    S.gnorm = -1.0;
+    if (!(v.gg >= F.tol2_hi)) {
+        S.gnorm = sqrt(v.gg);
+        if (S.gnorm < F.tol) {                   // stop branch: k unchanged
+            hist_row(F, S.k, S.J_cur, S.gnorm, 0.0);
+            S.state = ST_DONE;
+            return;
+        }
     }
     double beta = 0.0;
     if (S.k > 0) {
-        const double x = v.ratio;
-        beta = (x != x) ? x : fmax(x, 0.0);      // jnp.maximum keeps NaN
+        beta = is_neg64(v.ratio) ? 0.0 : v.ratio;   // max(ratio, 0); jnp.maximum keeps NaN
     }
     S.beta = (float)beta;
     S.alpha = 1.0f;
@@ -773,9 +942,9 @@ __device__ void start_iter(FrameState &S, const FConst &F, const StepVals &v) {
     S.state = ST_TRIAL;
 }
 
-__device__ void frame_decide(FrameState &S, const FConst &F, const double *q, const StepVals &v, int eval_only) {
+__device__ __forceinline__ void frame_decide(FrameState &S, const FConst &F, const double *q, const StepVals &v, int eval_only) {
     const double J = v.J;
-    if (J != J || q[P_GG] != q[P_GG]) S.nan_seen = 1;
+    if (is_nan64(J) || is_nan64(q[P_GG])) S.nan_seen = 1;
     S.n_evals += 1;
     // control-flow guard: an iteration takes at most 11 evaluations plus one restart
     if (S.n_evals > 12 * max(F.max_iter, 0) + 4) {
@@ -795,14 +964,14 @@ __device__ void frame_decide(FrameState &S, const FConst &F, const double *q, co
             if (!S.gd_known) {
                 S.gd_known = 1;
                 S.gd = q[P_GD];
-                if (S.gd >= 0.0) {                 // not a descent direction: restart with -g
+                if (is_nonneg64(S.gd)) {           // not a descent direction: restart with -g
                     S.restart = 1;
                     S.gd = -S.gg_cur;
                     S.alpha = 1.0f;
                     return;                        // re-evaluate trial 0 along -g
                 }
             }
-            if (J <= S.J_cur + 1e-4 * (double)S.alpha * S.gd) {
+            if (J <= S.J_cur + v.armijo * S.gd) {
                 hist_row(F, S.k, J, S.gnorm, (double)S.alpha);
                 S.k += 1;
                 accept_point(S, J, q[P_GG], q[P_GDIFF]);
@@ -940,13 +1109,9 @@ __device__ __forceinline__ int wait_blocks_past(CtlHeader *H, unsigned target) {
     return 1;
 }
 
-// The CG control of one frame, run by the warp that reduced the frame's last
-// node group: the group partials are summed in group order (double-float,
-// then FP64) and the frame state advanced.  Nothing else reads the frame's
-// state in this round once all its groups are reduced.
 // Active list rebuilt by one warp (the warp that ends a round): lane l scans a contiguous
 // block of frames, a warp scan gives each block its slot and prefix offsets.
-__device__ void rebuild_active_warp(const d2ic_frame_t *frames, int n_frames, Ctl &C, int lane) {
+__device__ __forceinline__ void rebuild_active_warp(const d2ic_frame_t *frames, int n_frames, Ctl &C, int lane) {
     const int per = (n_frames + 31) / 32;
     const int f0 = min(lane * per, n_frames), f1 = min(f0 + per, n_frames);
     int cnt = 0, ch = 0, gr = 0;
@@ -992,55 +1157,187 @@ __device__ void rebuild_active_warp(const d2ic_frame_t *frames, int n_frames, Ct
     __syncwarp();
 }
 
-__device__ void frame_r(const d2ic_frame_t &F, int f, Ctl &C, int eval_only, int lane) {
+// Supergroup records of a frame, behind its group partials: one tagged 16-byte record per sum.
+constexpr int SG_RECORDS = D2IC_NPART;
+__host__ __device__ inline size_t sg_record_offset(int n_groups) {
+    return ((size_t)n_groups * D2IC_NPART * sizeof(float2) + 15) & ~(size_t)15;
+}
+__device__ __forceinline__ uint4 *sg_records(const d2ic_frame_t &F) {
+    return reinterpret_cast<uint4 *>(reinterpret_cast<char *>(F.group_part) + sg_record_offset(F.n_groups));
+}
+
+// The control step of one frame: waits (bounded) for the frame's supergroup records of this
+// evaluation, reduces them (lane-strided, then a warp sum) and advances the CG state, which lane 0
+// returns in S (shared memory of the block with SHARED, else registers); false after an abort.  Everything that does not need the sums -- the state, one word per
+// lane, and the reciprocals of the two divisions -- is read and computed before the wait, and the
+// square root is left for after the release, so that the path from the last supergroup to the
+// release holds about ten FP64 operations.
+template <bool SHARED>
+__device__ __forceinline__ bool frame_r(const d2ic_frame_t &F, int f, Ctl &C, int eval_only, int lane, unsigned tag,
+                                        FrameState &S) {
+    constexpr int WORDS = sizeof(FrameState) / 8;
+    constexpr int L_HIST = WORDS, L_TOL = WORDS + 1, L_PAR = WORDS + 2;   // lanes of the descriptor's words
+    static_assert(L_PAR < 32, "one word of the state or the descriptor per lane");
+    static_assert(offsetof(d2ic_frame_t, alpha_reg) % 8 == 0 &&
+                      offsetof(d2ic_frame_t, max_iter) == offsetof(d2ic_frame_t, alpha_reg) + 4,
+                  "alpha_reg and max_iter are one word");
     DF q[5] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-    FrameState S;
-    if (lane == 0) S = load_fs(C.fs + f);              // in flight with the partials below
-    FConst fc;
-    fc.hist = F.hist;
-    fc.tol = F.tol;
-    fc.alpha_reg = F.alpha_reg;
-    fc.max_iter = F.max_iter;
-    fc.n_pix = F.n_pix;
+    const unsigned long long *src = reinterpret_cast<const unsigned long long *>(C.fs + f) + lane;
+    if (lane == L_HIST) src = reinterpret_cast<const unsigned long long *>(&F.hist);
+    if (lane == L_TOL) src = reinterpret_cast<const unsigned long long *>(&F.tol);
+    if (lane == L_PAR) src = reinterpret_cast<const unsigned long long *>(&F.alpha_reg);
+    unsigned long long word = 0;
+    if (lane < WORDS) word = __ldcg(src);
+    else if (lane <= L_PAR) word = *src;
+    // lane 0: 0.5 / n_pix; lane 1: 1 / (g.g + 1e-16); lane 2: squares at or above it are certainly not below
+    // tol; lane 3: the Armijo factor
+    const double gg_old = __longlong_as_double(
+        (long long)__shfl_sync(0xffffffffu, word, (int)(offsetof(FrameState, gg_cur) / 8)));
+    const double tol = __longlong_as_double((long long)__shfl_sync(0xffffffffu, word, L_TOL));
+    double inv = (lane == 0 ? 0.5 : 1.0) / (lane == 0 ? (double)max(F.n_pix, 1) : gg_old + 1e-16);
+    const float alpha_old = __uint_as_float((unsigned)(__shfl_sync(0xffffffffu, word, (int)(offsetof(FrameState, alpha) / 8)) >>
+                                                       (8 * (offsetof(FrameState, alpha) % 8))));
+    if (lane == 3) inv = 1e-4 * (double)alpha_old;
+    if (lane == 2) inv = tol > 0.0 ? fmax(tol * tol * (1.0 + 1e-12), 1e-290) : 0.0;
     const int nsg = (F.n_groups + SG - 1) / SG;
-    const float2 *sp = reinterpret_cast<const float2 *>(F.group_part) + (size_t)F.n_groups * D2IC_NPART;
-    for (int g = lane; g < nsg; g += 32) {
-        float2 v[5];
+    const uint4 *rec = sg_records(F);
+    // Every branch of the wait is taken by the whole warp: lanes that left a polling loop one by one
+    // stayed split after it, and the sums below then ran lane by lane (6 us instead of 0.3 us).
+    for (int g0 = 0; g0 < nsg; g0 += 32) {
+        const int g = g0 + lane;
+        uint4 r[SG_RECORDS];
+        unsigned long long t0 = 0;
+        for (unsigned it = 0;; ++it) {
+            bool all = true;
 #pragma unroll
-        for (int i = 0; i < 5; ++i) v[i] = __ldcg(sp + (size_t)g * D2IC_NPART + i);
+            for (int k = 0; k < SG_RECORDS; ++k)
+                r[k] = g < nsg ? ld_record(rec + (size_t)g * SG_RECORDS + k) : make_uint4(0u, 0u, tag, 0u);
 #pragma unroll
-        for (int i = 0; i < 5; ++i) q[i] = df_add(q[i], DF{v[i].x, v[i].y});
+            for (int k = 0; k < SG_RECORDS; ++k) all = all && r[k].z == tag;
+            if (__all_sync(0xffffffffu, all)) break;
+            if ((it & 63) == 63 && !keep_waiting(C.h, t0, lane)) return false;
+        }
+#pragma unroll
+        for (int k = 0; k < SG_RECORDS; ++k)
+            q[k] = df_add(q[k], DF{__uint_as_float(r[k].x), __uint_as_float(r[k].y)});
     }
-#pragma unroll
-    for (int i = 0; i < 5; ++i) q[i] = df_warp_sum(q[i]);
-    // lane i < 5 converts sum i to FP64: one conversion for all five
-    DF sel = q[0];
-#pragma unroll
-    for (int i = 1; i < 5; ++i)
-        if (lane == i) sel = q[i];
-    const double mine = df_to_double(sel);
+    fence_acq_rel();                                   // the groups' node data before this frame's release
+    // the lanes that hold a sum convert it to FP64: one conversion for all five
+    const double mine = df_to_double(df_reduce5(q, lane));
     double qd[5];
 #pragma unroll
-    for (int i = 0; i < 5; ++i) qd[i] = __shfl_sync(0xffffffffu, mine, i);
-    // one division for two quotients: lane 0 the image term of J, lane 1 the PR+ ratio
-    const double gg_old = __shfl_sync(0xffffffffu, lane == 0 ? S.gg_cur : 0.0, 0);
-    const double num = lane == 0 ? 0.5 * qd[P_JSUM] : qd[P_GDIFF];
-    const double den = lane == 0 ? (double)max(fc.n_pix, 1) : gg_old + 1e-16;
-    const double quo = num / den;
+    for (int i = 0; i < 5; ++i) qd[i] = __shfl_sync(0xffffffffu, mine, red5_lane(i));
     StepVals v;
-    v.ratio = __shfl_sync(0xffffffffu, quo, 1);
-    v.gnorm = sqrt(qd[P_GG]);
-    if (lane == 0) {
-        v.J = quo + (double)fc.alpha_reg * qd[P_EREG];
-        frame_decide(S, fc, qd, v, eval_only);
-        C.fs[f] = S;
-        if (S.state == ST_DONE) atomicExch(&C.h->finished, 1);
+    v.gg = qd[P_GG];
+    v.ratio = qd[P_GDIFF] * __shfl_sync(0xffffffffu, inv, 1);
+    v.armijo = __shfl_sync(0xffffffffu, inv, 3);
+    const unsigned long long par = __shfl_sync(0xffffffffu, word, L_PAR);
+    v.J = qd[P_JSUM] * __shfl_sync(0xffffffffu, inv, 0) + (double)__uint_as_float((unsigned)par) * qd[P_EREG];
+    FConst fc;
+    fc.hist = reinterpret_cast<float *>(__shfl_sync(0xffffffffu, word, L_HIST));
+    fc.tol = __longlong_as_double((long long)__shfl_sync(0xffffffffu, word, L_TOL));
+    fc.tol2_hi = __shfl_sync(0xffffffffu, inv, 2);
+    fc.max_iter = (int)(par >> 32);
+    unsigned long long *sw = reinterpret_cast<unsigned long long *>(&S);
+    if (SHARED) {
+        if (lane < WORDS) sw[lane] = word;
+        __syncwarp();
+    } else {
+#pragma unroll
+        for (int i = 0; i < WORDS; ++i) sw[i] = __shfl_sync(0xffffffffu, word, i);
     }
+    if (lane == 0) frame_decide(S, fc, qd, v, eval_only);
+    __syncwarp();
+    return true;
+}
+
+// The rest of a control step (whole warp): the gradient norm if it is still open, and the state.
+template <bool SHARED>
+__device__ __forceinline__ void frame_store(FrameState &S, FrameState *dst, int lane) {
+    if (lane == 0 && S.gnorm < 0.0) S.gnorm = sqrt(S.gg_cur);
+    if (SHARED) {
+        __syncwarp();
+        if (lane < (int)(sizeof(FrameState) / 8))
+            reinterpret_cast<unsigned long long *>(dst)[lane] = reinterpret_cast<const unsigned long long *>(&S)[lane];
+        __syncwarp();
+    } else if (lane == 0) {
+        *dst = S;
+    }
+}
+
+// The candidate rule that follows from a state (as frame_info reads it back).
+__device__ __forceinline__ FInfo info_of(const FrameState &S) {
+    FInfo fi;
+    fi.iu = S.iu;
+    fi.igc = S.igc;
+    fi.idp = S.idp;
+    fi.igt = S.igt;
+    fi.alpha = S.alpha;
+    fi.beta = S.beta;
+    fi.mode = (S.state == ST_EVAL) ? 0 : ((S.restart || S.k == 0) ? 2 : 1);
+    fi.tag = 0;
+    return fi;
+}
+
+// Control step of frame f (one warp), and the round's release if it is the round's last frame.
+template <bool SHARED>
+__device__ __forceinline__ void control_step(const d2ic_frame_t *frames, const d2ic_frame_t &F, int n_frames, Ctl &C, int f, unsigned tag,
+                                             int na, bool blockred, int round, int list_version, int eval_only,
+                                             int stop_flags, unsigned long long *trace, int trace_rounds, int lane,
+                                             FrameState &S) {
+    const bool rt = trace != nullptr && lane == 0 && round < trace_rounds;
+    if (!frame_r<SHARED>(F, f, C, eval_only, lane, tag, S)) return;
+    if (rt) trace[7 * round + 3] = gtimer();
+    // With one active frame whose control stays on this warp the release carries the next candidate
+    // rule, and the state is stored after it.  (A finished frame's state is read by every block after
+    // the release, so it is stored before.)
+    const bool done = SHARED ? S.state == ST_DONE : __shfl_sync(0xffffffffu, lane == 0 ? (S.state == ST_DONE) : 0, 0);
+    const bool inlined = na == 1 && blockred && !done;
+    int last_frame = 1;
+    if (!inlined) frame_store<SHARED>(S, C.fs + f, lane);
+    if (lane == 0 && !inlined) {
+        if (done) atomicExch(&C.h->finished, 1);
+        __threadfence();
+        if (na > 1) last_frame = atom_acq_rel_add(&C.h->frames_done, 1) == na - 1;
+    }
+    __syncwarp();
+    if (__shfl_sync(0xffffffffu, last_frame, 0)) {
+        // every frame of the round has run its control step, so every block's work of the round is
+        // done: rebuild the active list if a frame finished, and release the round
+        unsigned rel = (unsigned)list_version << 16;
+        if (!inlined) {
+            if (lane == 0 && na > 1) C.h->frames_done = 0;
+            if (ld_vol(&C.h->finished)) {
+                // no block still reads the list copy of an earlier round (bounded)
+                int past = 1;
+                if (lane == 0) past = wait_blocks_past(C.h, gridDim.x * (unsigned)round);
+                if (__shfl_sync(0xffffffffu, past, 0)) rebuild_active_warp(frames, n_frames, C, lane);
+                if (lane == 0) C.h->finished = 0;
+                rel = (unsigned)((list_version + 1) & 0xffff) << 16;
+                if (stop_flags & STOP_ON_FINISH) rel |= REL_STOP;
+            }
+        }
+        if (lane == 0) {
+            if ((stop_flags & STOP_ON_IRQ) && ld_vol(&C.h->irq)) rel |= REL_STOP;
+            uint4 r = make_uint4((unsigned)(round + 1), rel, 0u, 0u);
+            if (inlined) {
+                const FInfo nx = info_of(S);
+                r.y |= rel_pack(nx);
+                r.z = __float_as_uint(nx.alpha);
+                r.w = __float_as_uint(nx.beta);
+            } else {
+                fence_acq_rel();
+            }
+            st_record(&C.h->rel, r);
+        }
+    }
+    if (rt) trace[7 * round + 4] = gtimer();
+    if (inlined) frame_store<SHARED>(S, C.fs + f, lane);
 }
 
 // The active list (n_active = na <= FCACHE) with its prefix sums and each frame's candidate
 // rule, copied into the block's shared memory (whole block).
-__device__ void load_list(Ctl &C, int lb, int na, int *s_cpre, int *s_gpre, int *s_act, FInfo *s_fi) {
+__device__ __forceinline__ void load_list(Ctl &C, int lb, int na, int *s_cpre, int *s_gpre, int *s_act, FRule *s_fi) {
     if (na > FCACHE) return;
     for (int s = threadIdx.x; s <= na; s += NT) {
         s_cpre[s] = __ldcg(C.cp(lb) + s);
@@ -1049,8 +1346,42 @@ __device__ void load_list(Ctl &C, int lb, int na, int *s_cpre, int *s_gpre, int 
     for (int s = threadIdx.x; s < na; s += NT) {
         const int f = checked_index(__ldcg(C.act(lb) + s), C.n, C.h);
         s_act[s] = f;
-        s_fi[s] = frame_info(C.fs + f);
+        s_fi[s] = make_rule(frame_info(C.fs + f));
     }
+}
+
+// The chunk range of warp wid when one frame is active.  Every block takes a contiguous share of the
+// chunks (neighbouring elements share coefficient rows in cache), split evenly over its warps, so that
+// no SM has more chunks than the others (shares dealt out warp by warp left 49 of 152 SMs with all of
+// a 512 x 512 frame, and 80 against 64 chunks per SM at 2048 x 2048).  Blocks whose warps reduce node
+// groups (group gi: warp gi), and the last block, which runs the control step, take LEAD_PIXELS pixels
+// less than the others: a block's pixel work of about 2.5 us, the time of the node work that comes
+// before the wait for a group's chunks.  (Without it a 512 x 512 round takes 13.8 instead of 12.5 us.)
+constexpr int LEAD_PIXELS = 2304;
+__device__ __forceinline__ int2 chunk_share(const d2ic_frame_t &F, int total, int tg, int wid) {
+    const int nb = (int)gridDim.x, b = (int)blockIdx.x, rb = (tg + NWARP - 1) / NWARP, full = nb - rb - 1;
+    int b0, n;
+    if (full > 0) {
+        const int lead = (int)((long long)LEAD_PIXELS * total / max(F.n_pix, 1));   // in chunks
+        const int light = (int)max(((long long)total - (long long)lead * full) / nb, 0ll);
+        const int rest = total - (rb + 1) * light;
+        if (b < rb) {
+            b0 = b * light;
+            n = light;
+        } else if (b == nb - 1) {
+            b0 = total - light;
+            n = light;
+        } else {
+            b0 = rb * light + (int)((long long)rest * (b - rb) / full);
+            n = rb * light + (int)((long long)rest * (b - rb + 1) / full) - b0;
+        }
+    } else {
+        b0 = (int)((long long)total * b / nb);
+        n = (int)((long long)total * (b + 1) / nb) - b0;
+    }
+    const int base = n / NWARP, extra = n - base * NWARP;   // spare chunks to the last warps
+    const int c0 = b0 + wid * base + max(wid - (NWARP - extra), 0);
+    return make_int2(c0, c0 + base + (wid >= NWARP - extra ? 1 : 0));
 }
 
 // ---------------------------------------------------------------------------
@@ -1060,7 +1391,7 @@ __device__ void load_list(Ctl &C, int lb, int na, int *s_cpre, int *s_gpre, int 
 // fixed address, so its fields are loop invariants (loaded once, not per chunk; measured 2-5%
 // faster per round).
 template <int KIND, bool ONE = false>
-__global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_frame_t *__restrict__ frames, int n_frames,
+__global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_frame_t *__restrict__ frames, int n_frames_arg,
                                                    char *ctl_base, int eval_only, const float *u_eval,
                                                    double *J_out, float *grad_out, unsigned long long *trace,
                                                    int trace_rounds, int max_rounds, int stop_flags) {
@@ -1068,12 +1399,18 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
     // per warp and buffer: the nodal candidate inputs of the staged chunk, u of node a at [a], g at
     // [4 + a], the previous direction at [8 + a] (cp.async, completing on the buffer's mbarrier)
     __shared__ __align__(16) float2 s_cand[NWARP][2][CAND_N];
-    __shared__ int s_cpre[FCACHE + 1];               // per-round copies of the active list (na <= FCACHE)
-    __shared__ int s_gpre[FCACHE + 1];
-    __shared__ int s_act[FCACHE];
-    __shared__ FInfo s_fi[FCACHE];
-    __shared__ int s_hdr[6];                         // n_active, total_chunks, total_groups, abort, slice_stop,
-                                                     // list_buf
+    const int n_frames = ONE ? 1 : n_frames_arg;     // ONE: the control block's offsets are constants
+    constexpr int FC = ONE ? 1 : FCACHE;
+    __shared__ int s_cpre[FC + 1];                   // per-round copies of the active list (na <= FCACHE)
+    __shared__ int s_gpre[FC + 1];
+    __shared__ int s_act[FC];
+    __shared__ FRule s_fi[FC];
+    __shared__ __align__(16) unsigned long long s_frame[ONE ? sizeof(d2ic_frame_t) / 8 : 1];   // ONE: the descriptor
+    __shared__ FrameState s_state;                   // ONE: the state in the control step (one warp of the grid)
+    __shared__ int2 s_range[NWARP];                  // each warp's chunk range (one active frame)
+    __shared__ unsigned s_tag[NWARP];                // the current chunk's tag when the list is not cached
+    __shared__ int s_hdr[10];                         // n_active, total_chunks, total_groups, abort, slice stop,
+                                                     // what to refresh, rounds completed, list_buf, list version
     __shared__ DF s_gq[NWARP][D2IC_NPART];           // group partials of this block's supergroup
     __shared__ int s_sgcnt;                          // groups of this block's supergroup reduced this round
     // per warp: two record buffers, then two coefficient-tile buffers (all 128-byte aligned)
@@ -1092,6 +1429,14 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
         if (frames[f].tile_w > 0)
             asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(frames[f].coeff_map) : "memory");
     const bool tiles_ok = (smem_addr(s_dyn) & 127) == 0;   // tile buffers need 128-byte alignment
+    // ONE: the block's copy of the descriptor.  Every round begins with an acquire that empties the L1,
+    // so fields read from global memory cost an L2 round trip at each step of the round.
+    if (ONE)
+        for (int i = threadIdx.x; i < (int)(sizeof(d2ic_frame_t) / 8); i += NT)
+            s_frame[i] = reinterpret_cast<const unsigned long long *>(frames)[i];
+    auto frame = [&](int f) -> const d2ic_frame_t & {
+        return ONE ? *reinterpret_cast<const d2ic_frame_t *>(s_frame) : frames[f];
+    };
     __syncthreads();
     // optional phase trace per round: warp 0 of block 0 stamps [0] round start, [1] end of its pixel
     // work, [2] end of its group work, [5] after the barrier; the warp that runs a frame's control
@@ -1118,12 +1463,15 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
 #pragma unroll
             for (int j = 1; j < 7; ++j) nbuf(F, j)[i] = make_float2(0.f, 0.f);
         }
-        // gradient slots that no chunk owns must read as 0; group counters start at 0
+        // gradient slots that no chunk owns must read as 0 (and never carry a tag); counters start at 0
         float4 *ng = reinterpret_cast<float4 *>(F.node_grad);
         for (size_t i = blockIdx.x * NT + threadIdx.x; i < (size_t)F.node_chunk_k * nn; i += (size_t)gridDim.x * NT)
             ng[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        const int n_cnt = F.n_groups + (F.n_groups + SG - 1) / SG + 1;
-        for (int i = blockIdx.x * NT + threadIdx.x; i < n_cnt; i += gridDim.x * NT) F.group_cnt[i] = 0;
+        const int n_sg = (F.n_groups + SG - 1) / SG;
+        for (int i = blockIdx.x * NT + threadIdx.x; i < n_sg + 1; i += gridDim.x * NT) F.group_cnt[i] = 0;
+        uint4 *sr = sg_records(F);
+        for (int i = blockIdx.x * NT + threadIdx.x; i < n_sg * SG_RECORDS; i += gridDim.x * NT)
+            sr[i] = make_uint4(0u, 0u, 0u, 0u);        // tag 0: evaluations start at 1
         if (F.hist)
             for (int i = blockIdx.x * NT + threadIdx.x; i < 3 * F.max_iter; i += gridDim.x * NT)
                 F.hist[i] = __int_as_float(0x7fc00000);
@@ -1150,17 +1498,22 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
         s_hdr[2] = ld_vol(&C.h->total_groups);
         s_hdr[3] = ld_vol(&C.h->abort);
         s_hdr[4] = 0;
-        s_hdr[5] = ld_vol(&C.h->list_buf);
+        s_hdr[5] = 0;
+        s_hdr[6] = 0;
+        s_hdr[7] = ld_vol(&C.h->list_buf);
+        s_hdr[8] = 0;
     }
     __syncthreads();
-    load_list(C, s_hdr[5], s_hdr[0], s_cpre, s_gpre, s_act, s_fi);
+    load_list(C, s_hdr[7], s_hdr[0], s_cpre, s_gpre, s_act, s_fi);
+    __syncthreads();
+    if (lane == 0 && s_hdr[0] == 1) s_range[wid] = chunk_share(frame(s_act[0]), s_hdr[1], s_hdr[2], wid);
     __syncthreads();
 
     while (round < max_rounds) {                    // a slice: at most max_rounds rounds, state kept in HBM
-        const int na = s_hdr[0];
+        const int na = ONE ? min(s_hdr[0], 1) : s_hdr[0];
         const int total = s_hdr[1];
         const int tg = s_hdr[2];
-        const int lb = s_hdr[5];
+        const int lb = s_hdr[7];
         if (na == 0 || s_hdr[3] || s_hdr[4]) break;
         const bool trr = tr && round < trace_rounds;
         if (trr) trace[7 * round + 0] = gtimer();
@@ -1182,13 +1535,14 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
         pf_st0 = Stage{};
         // ---- P phase: chunks of the active list spread over the warps (see below) ----
         {
-            const bool cached = na <= FCACHE;
+            const bool cached = ONE || na <= FCACHE;
             const int gw = (int)((blockIdx.x * NT + threadIdx.x) >> 5);
             const int nw = (int)((gridDim.x * NT) >> 5);
             int cur = 0;   // active slot of the last located chunk (chunks ascend per warp)
             auto fetch_meta = [&](int g) {
-                int s, f, base;
-                if (cached) {
+                int s = 0, f = 0, base = 0;
+                if (ONE) {
+                } else if (cached) {
                     while (cur + 1 < na && s_cpre[cur + 1] <= g) ++cur;
                     s = cur;
                     f = s_act[s];
@@ -1198,13 +1552,13 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                     f = checked_index(__ldcg(C.act(lb) + s), n_frames, C.h);
                     base = __ldcg(C.cp(lb) + s);
                 }
-                ChunkMeta m = load_meta(frames, f, checked_index(g - base, frames[f].n_chunks, C.h), lane);
+                ChunkMeta m = load_meta(frame(f), f, checked_index(g - base, frame(f).n_chunks, C.h), lane);
                 m.s = s;
                 return m;
             };
             // stage a chunk: TMA bulk copy of its records, 2-D TMA copy of its coefficient tile
             auto issue_tma = [&](const ChunkMeta &m, unsigned i) {
-                const d2ic_frame_t &F = frames[ONE ? 0 : m.f];
+                const d2ic_frame_t &F = frame(m.f);
                 const int n = max(m.pe - m.pb, 0);
                 const unsigned bytes = (unsigned)min(n, D2IC_CHUNK_MAX) * 16u;
                 const uint4 *src = reinterpret_cast<const uint4 *>(F.pix) + m.pb;
@@ -1226,7 +1580,7 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                     mbar_arrive_tx(bar, (st.staged ? bytes : 0u) + tbytes);
                     if (st.staged) bulk_load(wbuf + (i & 1) * CHUNK_BYTES, src, bytes, bar);
                     if (st.tiled)
-                        tensor_load_2d(wbuf + 2 * CHUNK_BYTES + (i & 1) * TILE_BYTES, F.coeff_map, st.tx0 + F.pad,
+                        tensor_load_2d(wbuf + 2 * CHUNK_BYTES + (i & 1) * TILE_BYTES, frames[ONE ? 0 : m.f].coeff_map, st.tx0 + F.pad,
                                        st.ty0 + F.pad, bar);
                 }
                 return st;
@@ -1237,8 +1591,8 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                 const int a = lane & 3, k = lane >> 2;
                 const int nd = __shfl_sync(0xffffffffu, m.nd, a);
                 if (lane < CAND_N) {
-                    const d2ic_frame_t &F = frames[ONE ? 0 : m.f];
-                    const FInfo fi = cached ? s_fi[m.s] : frame_info(C.fs + m.f);
+                    const d2ic_frame_t &F = frame(m.f);
+                    const FInfo fi = cached ? s_fi[m.s].info() : frame_info(C.fs + m.f);
                     const int j = k == 0 ? fi.iu : (k == 1 ? 2 + fi.igc : 5 + fi.idp);
                     cp_async8(&s_cand[wid][i & 1][lane], nbuf(F, j) + nd);
                     cp_async_arrive(&s_bar[wid][i & 1]);
@@ -1247,26 +1601,12 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
             ChunkMeta m0{}, m1{}, m2{};
             Stage st0{}, st1{};
             bool p_ok = true;
-            // One frame: warp gw takes the contiguous chunk range [cb, ce) (neighbouring elements
-            // share coefficient rows in cache; measured faster).  Several frames: chunk g goes to
-            // warp g mod (warps), so that every step of the pass spans few frames (measured faster
-            // for batches of small frames).
-            // With fewer node groups than warps, group gi is reduced by warp gi (below); when the
-            // spare chunks fit on the other warps, those warps take them, so that the group
-            // reducers finish their own pixel work first and wait for none of it.
-            const bool contiguous = na == 1;
-            int cb = gw, ce = total;
-            if (contiguous) {
-                const int base = total / nw, extra = total - base * nw;
-                if (tg < nw && extra <= nw - tg) {
-                    const int k = max(gw - tg, 0);
-                    cb = gw * base + min(k, extra);
-                    ce = cb + base + (gw >= tg && k < extra ? 1 : 0);
-                } else {
-                    cb = (int)(((long long)gw * total) / nw);
-                    ce = (int)(((long long)(gw + 1) * total) / nw);
-                }
-            }
+            // One frame: the warp's contiguous share (chunk_share).  Several frames: chunk g goes to warp
+            // g mod (warps), warps counted across the blocks, so that every step of the pass spans few
+            // frames (measured faster for batches of small frames).
+            const bool contiguous = ONE || na == 1;
+            const int2 range = contiguous ? s_range[wid] : make_int2(wid * (int)gridDim.x + (int)blockIdx.x, total);
+            const int cb = range.x, ce = range.y;
             const int cs = contiguous ? 1 : nw;
             if (cb < ce) {
                 if (pf_use) {
@@ -1299,187 +1639,134 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                 }
                 float2 uc = make_float2(0.f, 0.f);
                 if (lane < 4) {
-                    const FInfo fi = cached ? s_fi[m0.s] : frame_info(C.fs + m0.f);
+                    const FInfo fi = cached ? s_fi[m0.s].info() : frame_info(C.fs + m0.f);
                     const float2 *sc = s_cand[wid][pipe_i & 1];
                     float2 dir;
                     uc = cand_value(sc[lane], sc[4 + lane], sc[8 + lane], fi.alpha, fi.beta, fi.mode, dir);
+                    if (!cached) s_tag[wid] = fi.tag;
                 }
-                chunk_compute<KIND>(frames[ONE ? 0 : m0.f], m0, uc, st0,
+                chunk_compute<KIND>(frame(m0.f), m0, uc, st0,
                                     reinterpret_cast<const uint4 *>(wbuf + (pipe_i & 1) * CHUNK_BYTES),
                                     reinterpret_cast<const float *>(wbuf + 2 * CHUNK_BYTES + (pipe_i & 1) * TILE_BYTES),
-                                    lane);
+                                    lane, cached ? &s_fi[m0.s].tag : &s_tag[wid]);
                 ++pipe_i;
                 m0 = m1;
                 st0 = st1;
                 m1 = m2;
             }
-            // ---- count this warp's chunks into their node groups: one fence for the whole pass
-            // (a fence per chunk would also wait for the pipeline's prefetch loads in flight) ----
-            // Eight chunks per step: lane 4 j + a reads node a of chunk j, so the node loads of
-            // the eight are in flight together.
-            __threadfence();
-            __syncwarp();
-            if (p_ok) {
-                for (int g0 = cb; g0 < ce; g0 += 8 * cs) {
-                    const int g = g0 + (lane >> 2) * cs;
-                    int grp = -1;
-                    int *cnt = nullptr;
-                    if (g < ce) {
-                        int f, base;
-                        if (cached) {
-                            const int sl = na == 1 ? 0 : find_slot_smem(s_cpre, na, g);
-                            f = s_act[sl];
-                            base = s_cpre[sl];
-                        } else {
-                            const int sl = find_slot(C.cp(lb), na, g);
-                            f = checked_index(__ldcg(C.act(lb) + sl), n_frames, C.h);
-                            base = __ldcg(C.cp(lb) + sl);
-                        }
-                        const d2ic_frame_t &F = frames[f];
-                        const int c = checked_index(g - base, F.n_chunks, C.h);
-                        grp = __ldg(F.chunk_nodes + 4 * c + (lane & 3)) / GN;
-                        cnt = F.group_cnt;
-                    }
-                    count_chunk_groups_quad(cnt, grp, lane);
-                }
-            }
             if (trr) trace[7 * round + 1] = gtimer();
             // ---- N work: group gi of the active list goes to global warp gi mod (warps in grid); the
             // warp waits until every chunk with a node in the group has written its slots.  With
             // at most one group per warp, a supergroup is the warps of one block and is reduced
-            // in shared memory; otherwise through the frame's global partials. ----
+            // in shared memory, and frame s's control step runs on warp (warps) - 1 - s, which waits
+            // for the supergroup records themselves; otherwise groups go through the frame's global
+            // partials and the warp that completes the last supergroup runs the control step. ----
             const bool blockred = tg <= nw;
             int gcur = 0;
-            for (int gi = gw; gi < tg; gi += nw) {
-                int s, f, base;
-                if (cached) {
-                    while (gcur + 1 < na && s_gpre[gcur + 1] <= gi) ++gcur;
-                    s = gcur;
-                    f = s_act[s];
-                    base = s_gpre[s];
-                } else {
-                    s = find_slot(C.gp(lb), na, gi);
-                    f = checked_index(__ldcg(C.act(lb) + s), n_frames, C.h);
-                    base = __ldcg(C.gp(lb) + s);
-                }
-                const d2ic_frame_t &F = frames[f];
-                const int g = gi - base;
-                if (g >= F.n_groups) continue;         // padding of the frame's group range
-                if (g < 0) {                           // self-check: the prefix sums are ascending
-                    checked_index(g, 0, C.h);
-                    continue;
-                }
-                const FInfo fi = cached ? s_fi[s] : frame_info(C.fs + f);
-                const NodePre pre = node_pre(F, fi, g * GN + lane);   // independent of the pixel pass
-                int ok = 1;
-                if (lane == 0) {
-                    const int need = __ldg(F.group_need + g);
-                    const unsigned *cnt = reinterpret_cast<const unsigned *>(F.group_cnt + g);
-                    if ((int)ld_acquire_u32(cnt) < need) {
-                        const unsigned long long t0 = gtimer();
-                        while ((int)ld_acquire_u32(cnt) < need) {
-                            if (ld_vol(&C.h->abort)) {
-                                ok = 0;
-                                break;
-                            }
-                            if (gtimer() - t0 > WAIT_NS) {
-                                C.h->err = D2IC_WAIT_TIMEOUT;
-                                atomicExch(&C.h->abort, 1);
-                                ok = 0;
-                                break;
-                            }
-                            __nanosleep(32);
-                        }
+            for (int gi = gw, cslot = nw - 1 - gw;;) {
+                int cf = -1;
+                unsigned ctag = 0;
+                if (gi < tg) {
+                    int s = 0, f = 0, base = 0;
+                    if (ONE) {
+                    } else if (cached) {
+                        while (gcur + 1 < na && s_gpre[gcur + 1] <= gi) ++gcur;
+                        s = gcur;
+                        f = s_act[s];
+                        base = s_gpre[s];
+                    } else {
+                        s = find_slot(C.gp(lb), na, gi);
+                        f = checked_index(__ldcg(C.act(lb) + s), n_frames, C.h);
+                        base = __ldcg(C.gp(lb) + s);
                     }
-                }
-                __syncwarp();                          // the slots seen by lane 0 are seen by the warp
-                if (!__shfl_sync(0xffffffffu, ok, 0)) break;
-                DF q[5];
-                node_post(F, fi, g * GN + lane, pre, q);
-#pragma unroll
-                for (int i = 0; i < 5; ++i) q[i] = df_warp_sum(q[i]);
-                // group -> supergroup (SG groups) -> frame: the warp that completes a level reduces
-                // it; a supergroup's sum is the same lane-ordered warp sum on both paths
-                const int ngr = F.n_groups, nsg = (ngr + SG - 1) / SG, sg = g / SG;
-                const int members = min(SG, ngr - sg * SG);
-                float2 *gp = reinterpret_cast<float2 *>(F.group_part);
-                int last = 0;
-                if (blockred) {                        // members are warps 0 .. members-1 here
-                    if (lane == 0) {
-#pragma unroll
-                        for (int i = 0; i < 5; ++i) s_gq[wid][i] = q[i];
-                        F.group_cnt[g] = 0;            // every chunk of this round has counted
-                        __threadfence_block();
-                        last = atomicAdd(&s_sgcnt, 1) == members - 1;
-                        if (last) {
-                            s_sgcnt = 0;
+                    const d2ic_frame_t &F = frame(f);
+                    const int g = gi - base;
+                    gi += nw;
+                    if (g >= F.n_groups) continue;         // padding of the frame's group range
+                    if (g < 0) {                           // self-check: the prefix sums are ascending
+                        checked_index(g, 0, C.h);
+                        continue;
+                    }
+                    const FInfo fi = cached ? s_fi[s].info() : frame_info(C.fs + f);
+                    const NodePre pre = node_pre(F, fi, g * GN + lane);   // independent of the pixel pass
+                    SlotSums slots;
+                    if (!gather_slots(F, g * GN + lane, __ldg(F.group_need + g), fi.tag, C.h, slots)) break;
+                    DF q[5];
+                    node_post(F, fi, g * GN + lane, pre, slots, q);
+                    DF sum = df_reduce5(q, lane);
+                    const int which = red5_value(lane);
+                    const bool holds = which >= 0 && (lane & 3) == 0;
+                    // group -> supergroup (SG groups) -> frame: the warp that completes a supergroup reduces
+                    // it; a supergroup's sum is the same lane-ordered warp sum on both paths
+                    const int ngr = F.n_groups, nsg = (ngr + SG - 1) / SG, sg = g / SG;
+                    const int members = min(SG, ngr - sg * SG);
+                    float2 *gp = reinterpret_cast<float2 *>(F.group_part);
+                    int last = 0;
+                    __syncwarp();
+                    if (blockred) {                        // members are warps 0 .. members-1 here
+                        if (holds) s_gq[wid][which] = sum;
+                        __syncwarp();
+                        if (lane == 0) {
                             __threadfence_block();
-                        }
-                    }
-                } else if (lane == 0) {
-#pragma unroll
-                    for (int i = 0; i < 5; ++i) gp[(size_t)g * D2IC_NPART + i] = make_float2(q[i].hi, q[i].lo);
-                    F.group_cnt[g] = 0;                // every chunk of this round has counted
-                    last = atom_acq_rel_add(F.group_cnt + ngr + sg, 1) == members - 1;
-                    if (last) F.group_cnt[ngr + sg] = 0;
-                }
-                __syncwarp();
-                if (__shfl_sync(0xffffffffu, last, 0)) {
-                    DF v[5];
-                    const int gg = sg * SG + lane;
-#pragma unroll
-                    for (int i = 0; i < 5; ++i) {
-                        DF t = DF{0.f, 0.f};
-                        if (lane < members) {
-                            if (blockred) {
-                                t = s_gq[lane][i];
-                            } else {
-                                const float2 t2 = __ldcg(gp + (size_t)gg * D2IC_NPART + i);
-                                t = DF{t2.x, t2.y};
+                            last = atomicAdd(&s_sgcnt, 1) == members - 1;
+                            if (last) {
+                                s_sgcnt = 0;
+                                __threadfence_block();
                             }
                         }
-                        v[i] = df_warp_sum(t);
-                    }
-                    int lastf = 0;
-                    if (lane == 0) {
-                        float2 *sp = gp + (size_t)(ngr + sg) * D2IC_NPART;
-#pragma unroll
-                        for (int i = 0; i < 5; ++i) sp[i] = make_float2(v[i].hi, v[i].lo);
-                        lastf = atom_acq_rel_add(F.group_cnt + ngr + nsg, 1) == nsg - 1;
-                        if (lastf) F.group_cnt[ngr + nsg] = 0;
+                    } else {
+                        if (holds) gp[(size_t)g * D2IC_NPART + which] = make_float2(sum.hi, sum.lo);
+                        __syncwarp();
+                        if (lane == 0) {
+                            last = atom_acq_rel_add(F.group_cnt + sg, 1) == members - 1;
+                            if (last) F.group_cnt[sg] = 0;
+                        }
                     }
                     __syncwarp();
-                    if (__shfl_sync(0xffffffffu, lastf, 0)) {   // the frame's last supergroup
-                        const bool rt = trace != nullptr && lane == 0 && round < trace_rounds;
-                        if (rt) trace[7 * round + 3] = gtimer();
-                        frame_r(F, f, C, eval_only, lane);
-                        int last_frame = 0;
-                        if (lane == 0) last_frame = na == 1 || atom_acq_rel_add(&C.h->frames_done, 1) == na - 1;
-                        __syncwarp();
-                        if (__shfl_sync(0xffffffffu, last_frame, 0)) {
-                            // every frame of the round has run its control step, so every block's
-                            // work of the round is done: rebuild the active list and release the round
-                            if (lane == 0) C.h->frames_done = 0;
-                            int stop = 0;
-                            if (ld_vol(&C.h->finished)) {
-                                // no block still reads the list copy of an earlier round (bounded)
-                                int past = 1;
-                                if (lane == 0) past = wait_blocks_past(C.h, gridDim.x * (unsigned)round);
-                                if (__shfl_sync(0xffffffffu, past, 0))
-                                    rebuild_active_warp(frames, n_frames, C, lane);
-                                if (lane == 0) C.h->finished = 0;
-                                stop = stop_flags & STOP_ON_FINISH;
-                            }
-                            if (lane == 0 && (stop || ((stop_flags & STOP_ON_IRQ) && ld_vol(&C.h->irq))))
-                                C.h->slice_stop = 1;   // published by the release below
-                            __syncwarp();
-                            if (lane == 0) {
-                                __threadfence();
-                                atomicExch(&C.h->rounds_done, (unsigned)(round + 1));
+                    if (__shfl_sync(0xffffffffu, last, 0)) {
+                        const int gg = sg * SG + lane;
+#pragma unroll
+                        for (int i = 0; i < 5; ++i) {
+                            q[i] = DF{0.f, 0.f};
+                            if (lane < members) {
+                                if (blockred) {
+                                    q[i] = s_gq[lane][i];
+                                } else {
+                                    const float2 t2 = __ldcg(gp + (size_t)gg * D2IC_NPART + i);
+                                    q[i] = DF{t2.x, t2.y};
+                                }
                             }
                         }
-                        if (rt) trace[7 * round + 4] = gtimer();
+                        sum = df_reduce5(q, lane);
+                        fence_acq_rel();                   // the supergroup's node data before its records
+                        if (holds)
+                            st_record(sg_records(F) + (size_t)sg * SG_RECORDS + which,
+                                      make_uint4(__float_as_uint(sum.hi), __float_as_uint(sum.lo), fi.tag, 0u));
+                        if (!blockred) {
+                            int lastf = 0;
+                            __syncwarp();
+                            if (lane == 0) {
+                                lastf = atom_acq_rel_add(F.group_cnt + nsg, 1) == nsg - 1;
+                                if (lastf) F.group_cnt[nsg] = 0;
+                            }
+                            __syncwarp();
+                            if (__shfl_sync(0xffffffffu, lastf, 0)) {   // the frame's last supergroup
+                                cf = f;
+                                ctag = fi.tag;
+                            }
+                        }
                     }
+                } else if (blockred && cslot < na) {
+                    cf = ONE ? 0 : cached ? s_act[cslot] : checked_index(__ldcg(C.act(lb) + cslot), n_frames, C.h);
+                    ctag = cached ? s_fi[cslot].tag : frame_info(C.fs + cf).tag;
+                    cslot += nw;
+                } else {
+                    break;
+                }
+                if (cf >= 0) {
+                    FrameState local;
+                    control_step<ONE>(frames, frame(cf), n_frames, C, cf, ctag, ONE ? 1 : na, blockred, round, s_hdr[8],
+                                      eval_only, stop_flags, trace, trace_rounds, lane, ONE ? s_state : local);
                 }
             }
             if (trr) trace[7 * round + 2] = gtimer();
@@ -1495,46 +1782,75 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                 pf_total = total;
             }
         }
-        // ---- end of round: wait until the warp that ran the round's last frame step releases it
-        // (rounds_done is monotonic, so a block that arrives after the release passes at once) ----
+        // ---- end of round: one thread per block polls the release record.  Records only move
+        // forward; a block that had no work in a round may find a later one. ----
         __syncthreads();
         if (threadIdx.x == 0) {
             atomicAdd(&C.h->blocks_past, 1u);           // this block's list reads of the round are done
             const unsigned target = (unsigned)(round + 1);
-            if (ld_acquire_u32(&C.h->rounds_done) < target) {
-                const unsigned long long t0 = gtimer();
-                while (ld_acquire_u32(&C.h->rounds_done) < target) {
-                    if (ld_vol(&C.h->abort)) break;
-                    if (gtimer() - t0 > WAIT_NS) {
+            uint4 r = ld_record(&C.h->rel);
+            unsigned long long t0 = 0;
+            int dead = 0;
+            for (unsigned it = 0; r.x < target; ++it) {
+                if ((it & 63) == 63) {
+                    const unsigned long long now = gtimer();
+                    if (t0 == 0) t0 = now;
+                    if (ld_vol(&C.h->abort)) dead = 1;
+                    else if (now - t0 > WAIT_NS) {
                         C.h->err = D2IC_WAIT_TIMEOUT;
                         atomicExch(&C.h->abort, 1);
-                        break;
+                        dead = 1;
                     }
-                    __nanosleep(32);
+                    if (dead) break;
+                }
+                r = ld_record(&C.h->rel);
+            }
+            fence_acq_rel();
+            s_hdr[3] = dead;
+            if (!dead) {
+                s_hdr[4] = (int)(r.y & REL_STOP);
+                s_hdr[6] = (int)r.x;
+                if (r.y & REL_INLINE) {                 // na == 1 and the list unchanged
+                    s_fi[0] = FRule{__uint_as_float(r.z), __uint_as_float(r.w), r.y,
+                                    (s_fi[0].tag + (r.x - (unsigned)round)) & TAG_MASK};
+                    s_hdr[5] = REFRESH_NONE;
+                } else {
+                    if ((int)(r.y >> 16) != s_hdr[8]) {   // the list changed: the header of the round released last
+                        for (int t = 0; t < 64; ++t) {
+                            s_hdr[0] = ld_vol(&C.h->n_active);
+                            s_hdr[1] = ld_vol(&C.h->total_chunks);
+                            s_hdr[2] = ld_vol(&C.h->total_groups);
+                            s_hdr[7] = ld_vol(&C.h->list_buf);
+                            fence_acq_rel();
+                            const uint4 r2 = ld_record(&C.h->rel);
+                            if (r2.x == r.x) break;
+                            r = r2;
+                        }
+                        s_hdr[4] = (int)(r.y & REL_STOP);
+                        s_hdr[6] = (int)r.x;
+                        s_hdr[8] = (int)(r.y >> 16);
+                        s_hdr[5] = REFRESH_LIST;
+                    } else {
+                        s_hdr[5] = REFRESH_RULES;
+                    }
                 }
             }
-            __threadfence();
         }
         __syncthreads();
-        // one round trip for the next round's state: the header (thread 0) and, for the list as it
-        // was, each frame's candidate rule; a changed list (a frame finished) is reloaded
-        if (threadIdx.x == 0) {
-            s_hdr[0] = ld_vol(&C.h->n_active);
-            s_hdr[1] = ld_vol(&C.h->total_chunks);
-            s_hdr[2] = ld_vol(&C.h->total_groups);
-            s_hdr[3] = ld_vol(&C.h->abort);
-            s_hdr[4] = ld_vol(&C.h->slice_stop);
-            s_hdr[5] = ld_vol(&C.h->list_buf);
-        }
-        if (na <= FCACHE)
-            for (int s = threadIdx.x; s < na; s += NT) s_fi[s] = frame_info(C.fs + s_act[s]);
-        __syncthreads();
-        if (s_hdr[0] != na && s_hdr[0] > 0 && !s_hdr[3]) {
-            load_list(C, s_hdr[5], s_hdr[0], s_cpre, s_gpre, s_act, s_fi);
+        if (s_hdr[5] != REFRESH_NONE && !s_hdr[3]) {    // rules from the frame states; a changed list is reloaded
+            if (s_hdr[5] == REFRESH_RULES) {
+                if (na <= FCACHE)
+                    for (int s = threadIdx.x; s < na; s += NT) s_fi[s] = make_rule(frame_info(C.fs + s_act[s]));
+            } else if (s_hdr[0] > 0) {
+                load_list(C, s_hdr[7], s_hdr[0], s_cpre, s_gpre, s_act, s_fi);
+                __syncthreads();
+                if (lane == 0 && s_hdr[0] == 1) s_range[wid] = chunk_share(frame(s_act[0]), s_hdr[1], s_hdr[2], wid);
+            }
             __syncthreads();
         }
+        const int next_round = s_hdr[3] ? round + 1 : s_hdr[6];
         if (trr) trace[7 * round + 5] = gtimer();
-        ++round;
+        round = next_round;
     }
 
     if (pf) {                                       // no copy in flight at exit (bounded wait)
@@ -1678,10 +1994,10 @@ extern "C" size_t d2ic_cg_control_bytes(int n_frames) {
 }
 
 // Workspace of one frame: 7 node buffers (u x2, g x3, dir x2), the K gradient
-// slots per node (16 bytes: gx, gy and the chunk's r^2 sum as a double-float),
-// the partials (D2IC_NPART double-float pairs) of every group and then of every
-// supergroup of SG groups, the completion counters (groups, supergroups, the
-// frame's count of supergroups), and the tile origins (4 bytes per chunk).
+// slots per node (tagged 16-byte records: gx, gy, a word of the chunk's r^2 sum, the tag),
+// the partials (D2IC_NPART double-float pairs) of every group and the tagged
+// records of every supergroup of SG groups, the completion counters (supergroups
+// and the frame's count of them), and the tile origins (4 bytes per chunk).
 static size_t ws_layout(int n_nodes, int n_chunks, int node_chunk_k, size_t off[5]) {
     const size_t ng = (size_t)(n_nodes + GN - 1) / GN;
     size_t o = 0;
@@ -1691,7 +2007,7 @@ static size_t ws_layout(int n_nodes, int n_chunks, int node_chunk_k, size_t off[
     o += align256(sizeof(float) * 4 * (size_t)node_chunk_k * n_nodes);
     off[2] = o;                                               // group_part
     const size_t ns = (ng + SG - 1) / SG;                     // supergroups of SG groups
-    o += align256(sizeof(float) * 2 * D2IC_NPART * (ng + ns));
+    o += align256(sg_record_offset((int)ng) + sizeof(uint4) * SG_RECORDS * ns);
     off[3] = o;                                               // group_cnt
     o += align256(sizeof(int) * (ng + ns + 1));
     off[4] = o;                                               // chunk_tile

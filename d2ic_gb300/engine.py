@@ -255,7 +255,7 @@ class FrameLayout:
         chunk_slot = (r4[:, 0] | (r4[:, 1] << 8) | (r4[:, 2] << 16) | (r4[:, 3] << 24)).astype(np.uint32).view(np.int32)
         self.node_chunk_k = K
         # chunks with a node in each group of NODE_GROUP consecutive nodes (the group's reducer
-        # waits for that many completion counts per pass)
+        # waits for the records of that many chunks per pass)
         ng = (self.n_nodes + _lib.NODE_GROUP - 1) // _lib.NODE_GROUP
         cg = np.sort(chunk_nodes.astype(np.int64).reshape(-1, 4) // _lib.NODE_GROUP, axis=1)
         first = np.ones(cg.shape, dtype=bool)

@@ -95,14 +95,16 @@ typedef struct d2ic_frame {
     /* workspace */
     float       *node_ws;          /* 14 * n_nodes floats                               */
     float       *node_grad;        /* 4 * node_chunk_k * n_nodes: per-node slots of the
-                                      chunks' partials (gx, gy, and for the chunk's node 0
-                                      its sum of r^2 as a double-float hi, lo), column-major
-                                      (slot k of node n at k * n_nodes + n), unused slots 0 */
-    float       *group_part;       /* 2 * D2IC_NPART * (n_groups + n_super) double-float
-                                      partials of the groups, then of the supergroups of
-                                      16 groups (n_super = ceil(n_groups / 16))          */
-    int         *group_cnt;        /* n_groups + n_super + 1 completion counters (all 0
-                                      between rounds)                                   */
+                                      chunks' partials, 16-byte records (gx, gy, for the
+                                      chunk's nodes 0 and 1 the hi and lo word of its sum of
+                                      r^2 as a double-float, the evaluation's tag), column-
+                                      major (slot k of node n at k * n_nodes + n), unused 0 */
+    float       *group_part;       /* 2 * D2IC_NPART * n_groups: double-float partials of the
+                                      groups, then (16-byte aligned) D2IC_NPART tagged 16-byte
+                                      records for each of the n_super = ceil(n_groups / 16)
+                                      supergroups                                       */
+    int         *group_cnt;        /* n_super + 1 completion counters (all 0 between rounds;
+                                      room for n_groups + n_super + 1)                  */
     int         *chunk_tile;       /* n_chunks: origin (col | row << 16, int16 each) of the
                                       chunk's coefficient tile for the next pass        */
     double       tol;

@@ -1,0 +1,80 @@
+"""Rounds of the CG engine at the edges of its work split (GPU).
+
+The split of a round over the grid -- a supergroup reduced in one block or through global partials,
+blocks with and without a lighter share of the chunks, a control step on a warp of its own or on the
+one that completes the frame -- depends on the number of node groups and chunks against the warps of
+the grid.  Every partial has its own slot and every sum a fixed order, so a solve gives the same bits
+on every grid; one evaluation is compared with the FP64 oracle.
+"""
+from __future__ import annotations
+
+from dataclasses import replace
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("side,element,interp", [
+    (40, 16, "cubic"),        # 9 nodes: one group
+    (354, 16, "cubic"),       # 23 x 23 nodes: 17 groups, the second supergroup has one
+    (250, 8, "cubic"),        # 32 x 32 nodes: 32 groups, two full supergroups; 64-pixel chunks
+    (257, 11, "linear"),      # odd image and element sizes
+    (300, 32, "cubic"),       # several chunks per element: 16 slots per node
+])
+def test_grids_give_the_same_bits(cuda, side, element, interp):
+    import d2ic_gb300 as d2
+    from d2ic_gb300.engine import Engine, FrameLayout, FrameSlot, descriptors_to_device
+    from d2ic_gb300.synthetic import Affine, rect_mask, speckle_sequence
+    from oracle import objective, pixels
+    ref, frames = speckle_sequence(side, side, [Affine([[0.004, 0.001], [0, -0.003]], [0.4, -0.3], [side / 2] * 2)],
+                                   seed=81, noise_seeds=[81, 82])
+    mesh, assets = d2.mask_to_mesh_assets(rect_mask(side, side, side - 12, side - 12), element)
+    pix = d2.build_pixel_assets(mesh, ref, 1.0, assets.roi_mask)
+    n_nodes = mesh.nodes_xy.shape[0]
+    layout = FrameLayout(pix, n_nodes, ref, interp, cuda)
+    slot = FrameSlot(layout, 12)
+    slot.set_params(1e-6, 0.1)
+    slot.load_image(frames[0])
+    slot.set_u0(None)
+    engine, desc = Engine(cuda, 1), descriptors_to_device([slot.desc], cuda)
+    results = []
+    for grid in (0, 1, 2, 7, 40):
+        engine.solve(desc, 1, layout.kind, grid)
+        torch.cuda.synchronize()
+        results.append((slot.u_out.clone(), slot.hist.clone(), slot.info.clone()))
+    for u, hist, info in results[1:]:
+        assert torch.equal(u, results[0][0]) and torch.equal(info, results[0][2])
+        assert torch.equal(hist.nan_to_num(7.0), results[0][1].nan_to_num(7.0))
+    # one evaluation against the FP64 oracle, at the tolerance of the other gradient tests
+    u = torch.as_tensor(np.random.default_rng(3).normal(0.0, 0.3, (n_nodes, 2)), dtype=torch.float32, device=cuda)
+    J, g = engine.eval_objective(desc, u, layout.kind)
+    oa = pixels.build_pixel_assets(np.asarray(mesh.nodes_xy), np.asarray(mesh.elements), side, side, assets.roi_mask)
+    pb = objective.Problem.build(ref, frames[0], oa, interp)
+    J64, g64 = objective.J_total_and_grad(u.cpu().numpy().astype(np.float64), pb, 0.1)
+    assert abs(float(J) - J64) <= 1e-5 * J64
+    assert np.abs(g.cpu().numpy() - g64).max() <= 1e-5 * np.abs(g64).max()
+
+
+@pytest.mark.parametrize("slots", [2, 5])
+def test_uneven_frames_finish_in_different_rounds(cuda, slots):
+    """Several frames in one launch: the control steps of all frames, the rebuilt list, the last frame alone."""
+    import d2ic_gb300 as d2
+    from d2ic_gb300.engine import FrameLayout
+    from d2ic_gb300.serving import solve_batch
+    from d2ic_gb300.synthetic import Translation, rect_mask, speckle_sequence
+    work = []
+    for i in range(slots):
+        side = 72 + 40 * i
+        ref, frames = speckle_sequence(side, side, [Translation(0.3, -0.2)], seed=90 + i, noise_seeds=[i, i + 50])
+        mesh, assets = d2.mask_to_mesh_assets(rect_mask(side, side, side - 12, side - 12), 12)
+        pix = d2.build_pixel_assets(mesh, ref, 1.0, assets.roi_mask)
+        layout = FrameLayout(pix, mesh.nodes_xy.shape[0], ref, "cubic", cuda)
+        work.append((layout, frames[0], None, d2.MeshDICConfig(max_iters=5 + 9 * i, tol=1e-6, reg_strength=0.1)))
+    together = solve_batch(work)
+    for w, got in zip(work, together):
+        alone = solve_batch([w])[0]
+        assert got[1] == alone[1] and np.array_equal(got[0], alone[0])
+        assert np.array_equal(got[3], alone[3], equal_nan=True)
