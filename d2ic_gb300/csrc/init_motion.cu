@@ -3,15 +3,323 @@
 //
 // ZNCC (d2ic/solver_translation_zncc.py:89-168): one block per centre; the
 // template (win x win) and the search patch ((win + 2 s)^2) are staged in
-// shared memory; each thread scores one (up to 1024 offsets) or several of the (2 s + 1)^2 offsets with a
-// two-pass (mean, then centred sums) window normalisation; the block keeps the
-// first maximum in row-major (ky, kx) order.  FP32 arithmetic on the CUDA
-// cores: nothing here is a dense contraction.
+// shared memory.  The score of an offset is the mean product of the normalised
+// template t and the normalised window, first maximum in row-major (ky, kx)
+// order.
+//
+// With the patch centred once (d = patch - c), an offset needs sum d t over its
+// window, and sum d and sum d^2 for its mean and variance:
+//   * the products are a register-blocked correlation: a thread makes
+//     2 x R offsets (two rows of R), and per template value reads two patch
+//     values and one template value from shared memory for 2 R multiply-adds;
+//   * the two sums come from separable running sums in double-float, so that
+//     v = sum d^2 - (sum d)^2 / n is exact to FP32 (rows are rounded to FP32
+//     once, 6e-8 relative).
+// A window whose mean lies more than 8 standard deviations from c would lose
+// digits in v; it is scored by the two-pass form (mean first, then centred
+// sums), as is every window of a patch with values that are not finite or
+// beyond 1e15.
+//
+// Bound by FP32 issue and shared-memory reads.  9,216 centres at win 41,
+// search 24 (2401 offsets x 1681 pixels): 14.2 ms with one offset per thread in
+// the two-pass form (5 instructions and 3 shared-memory reads per pixel and
+// offset), 2.39 ms blocked with scalar multiply-adds, 2.07 ms with two offsets
+// per instruction (fma.rn.f32x2).  16,384 centres at win 17, search 8: 743 ->
+// 365 us; staging and running sums weigh more there.
 #include "common.cuh"
 
 namespace d2ic {
 
-__global__ void __launch_bounds__(1024) zncc_kernel(const float *__restrict__ ref, int Hr, int Wr, const float *__restrict__ def, int Hd,
+// the two-pass score of one offset: window mean, then centred sums
+__device__ __forceinline__ float zncc_two_pass(const float *w0, int ps, const float *tpl, int win) {
+    const float n = (float)(win * win);
+    float s = 0.f;
+    for (int i = 0; i < win; ++i)
+        for (int j = 0; j < win; ++j) s += w0[i * ps + j];
+    const float mw = s / n;
+    float v = 0.f, cr = 0.f;
+    for (int i = 0; i < win; ++i)
+        for (int j = 0; j < win; ++j) {
+            const float d = w0[i * ps + j] - mw;
+            v += d * d;
+            cr += d * tpl[i * win + j];
+        }
+    return cr / (sqrtf(v / n) + 1e-12f) / n;
+}
+
+// a float added to a double-float whose low word collects the rounding errors
+__device__ __forceinline__ void df_acc(DF &a, float x) {
+    const DF s = df_two_sum(a.hi, x);
+    a.hi = s.hi;
+    a.lo += s.lo;
+}
+
+// Running sums along one line: out[k] = sum_{i < win} f(k + i) for k in [k0, k1), f(i) a double-float
+// (or, with an exact low word of 0, a float).
+template <class F, class O>
+__device__ __forceinline__ void running_sums(int k0, int k1, int win, F &&f, O &&out) {
+    DF a = {0.f, 0.f};
+    for (int i = 0; i < win; ++i) f(k0 + i, [&](float x) { df_acc(a, x); });
+    for (int k = k0;;) {
+        out(k, a);
+        if (++k >= k1) break;
+        f(k - 1, [&](float x) { df_acc(a, -x); });
+        f(k + win - 1, [&](float x) { df_acc(a, x); });
+    }
+}
+
+constexpr int ZNCC_SEG = 7;   // outputs per thread of a running sum
+constexpr int ZNCC_MAX_THREADS = 384, ZNCC_TPT = 2;   // column tasks per thread
+
+// Two FP32 values in a 64-bit register pair and their fused multiply-add (fma.rn.f32x2: one instruction
+// for two IEEE multiply-adds).
+typedef unsigned long long Pair;
+__device__ __forceinline__ Pair pair(float lo, float hi) {
+    Pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float pair_lo(Pair p) { return __uint_as_float((unsigned)p); }
+__device__ __forceinline__ float pair_hi(Pair p) { return __uint_as_float((unsigned)(p >> 32)); }
+__device__ __forceinline__ Pair pair_fma(Pair a, Pair b, Pair c) {
+    Pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+template <int R>
+__global__ void __launch_bounds__(ZNCC_MAX_THREADS) zncc_kernel(const float *__restrict__ ref, int Hr, int Wr,
+                                                                const float *__restrict__ def, int Hd, int Wd,
+                                                                const float2 *__restrict__ centers, int win,
+                                                                int search, float2 *__restrict__ u_out,
+                                                                float *__restrict__ score_out) {
+    extern __shared__ float sm[];
+    const int ps = win + 2 * search, npa = 2 * search + 1;
+    const int n = win * win, np2 = npa * npa;
+    float *tpl = sm;                 // win * win, normalised template
+    float *pat = sm + n;             // ps * ps, centred patch (one spare row of R values for the last block's reads)
+    float *row1 = pat + ps * ps + R, *row2 = row1 + ps * npa;   // row sums of d and d^2: ps x npa
+    float *mean = row1, *var = row1 + np2;                      // over them: window mean and n * variance
+    __shared__ float s_red[32];
+    __shared__ int s_idx[32];
+    const int c = blockIdx.x;
+    const float2 ctr = centers[c];
+    // half to even, as jnp.rint; non-finite or far-away centres fail the bounds test below
+    const bool finite = fabsf(ctr.x) < 1e7f && fabsf(ctr.y) < 1e7f;
+    const int x = finite ? (int)rintf(ctr.x) : -(1 << 28), y = finite ? (int)rintf(ctr.y) : -(1 << 28);
+    const int r = win / 2;
+    const bool tpl_ok = (y - r >= 0) && (y + r < Hr) && (x - r >= 0) && (x + r < Wr);
+    const int xs = x - search, ys = y - search, xe = x + search, ye = y + search;
+    const bool patch_ok = (ys - r >= 0) && (ye + r < Hd) && (xs - r >= 0) && (xe + r < Wd);
+    if (!(tpl_ok && patch_ok)) {
+        if (threadIdx.x == 0) {
+            u_out[c] = make_float2(0.f, 0.f);
+            score_out[c] = __int_as_float(0x7fc00000);
+        }
+        return;
+    }
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    auto block_sum = [&](float a) {
+        a = warp_sum_f(a);
+        __syncthreads();
+        if (lane == 0) s_red[wid] = a;
+        __syncthreads();
+        float t = 0.f;
+        for (int w = 0; w < nw; ++w) t += s_red[w];
+        return t;
+    };
+    float a = 0.f, pa = 0.f;
+    bool odd = false;                // a value that the running sums cannot take
+    for (int i = wid; i < win; i += nw)
+        for (int j = lane; j < win; j += 32) {
+            const float t = __ldg(ref + (size_t)(y - r + i) * Wr + (x - r + j));
+            tpl[i * win + j] = t;
+            odd |= !(fabsf(t) < 1e15f);
+            a += t;
+        }
+    for (int i = wid; i < ps; i += nw)
+        for (int j = lane; j < ps; j += 32) {
+            const float t = __ldg(def + (size_t)(ys - r + i) * Wd + (xs - r + j));
+            pat[i * ps + j] = t;
+            odd |= !(fabsf(t) < 1e15f);
+            pa += t;
+        }
+    odd = __syncthreads_or(odd);
+    // template mean and population std (two passes)
+    const float mu = block_sum(a) / (float)n;
+    a = 0.f;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const float d = tpl[i] - mu;
+        a += d * d;
+    }
+    const float inv = 1.0f / (sqrtf(block_sum(a) / (float)n) + 1e-12f);
+    float t1 = 0.f;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const float t = (tpl[i] - mu) * inv;
+        tpl[i] = t;
+        t1 += t;
+    }
+    t1 = block_sum(t1);              // zero but for rounding
+    float best = -INFINITY;
+    int bidx = 0x7fffffff;
+    auto take = [&](float sc, int o) {
+        if (sc > best || (sc != sc && best == best)) {   // NaN wins, as argmax
+            best = sc;
+            bidx = o;
+        }
+    };
+    if (odd) {
+        __syncthreads();
+        for (int o = threadIdx.x; o < np2; o += blockDim.x)
+            take(zncc_two_pass(pat + (o / npa) * ps + o % npa, ps, tpl, win), o);
+    } else {
+        const float pc = block_sum(pa) / (float)(ps * ps);
+        for (int i = threadIdx.x; i < ps * ps; i += blockDim.x) pat[i] -= pc;
+        if ((int)threadIdx.x < R) pat[ps * ps + threadIdx.x] = 0.f;
+        __syncthreads();
+        const int segs = (npa + ZNCC_SEG - 1) / ZNCC_SEG;
+        // rows: sums over win columns (a thread: one row, ZNCC_SEG columns; neighbouring threads take
+        // neighbouring rows)
+        for (int t = threadIdx.x; t < 2 * ps * segs; t += blockDim.x) {
+            const bool sq = t >= ps * segs;
+            const int q = sq ? t - ps * segs : t, row = q % ps, k0 = (q / ps) * ZNCC_SEG;
+            const float *src = pat + row * ps;
+            float *dst = (sq ? row2 : row1) + row * npa;
+            if (sq)
+                running_sums(k0, min(k0 + ZNCC_SEG, npa), win,
+                             [&](int i, auto &&add) {
+                                 const DF p = df_prod(src[i], src[i]);
+                                 add(p.hi);
+                                 add(p.lo);
+                             },
+                             [&](int k, const DF &v) { dst[k] = v.hi + v.lo; });
+            else
+                running_sums(k0, min(k0 + ZNCC_SEG, npa), win, [&](int i, auto &&add) { add(src[i]); },
+                             [&](int k, const DF &v) { dst[k] = v.hi + v.lo; });
+        }
+        __syncthreads();
+        // columns: the window sums, kept in registers until every thread has read its rows (mean and var
+        // lie over the rows).  A task is one column, ZNCC_SEG rows; at most ZNCC_TPT per thread.
+        float wm[ZNCC_TPT][ZNCC_SEG], wv[ZNCC_TPT][ZNCC_SEG];
+#pragma unroll
+        for (int h = 0; h < ZNCC_TPT; ++h) {
+            const int task = threadIdx.x + h * blockDim.x, kx = task % npa, ky0 = (task / npa) * ZNCC_SEG;
+            if (task < npa * segs) {
+                DF s1 = {0.f, 0.f}, s2 = {0.f, 0.f};
+                for (int i = 0; i < win; ++i) {
+                    df_acc(s1, row1[(ky0 + i) * npa + kx]);
+                    df_acc(s2, row2[(ky0 + i) * npa + kx]);
+                }
+#pragma unroll
+                for (int q = 0; q < ZNCC_SEG; ++q) {
+                    // n * variance = sum d^2 - (sum d)^2 / n, negative where the window needs the two-pass form
+                    const float hi = s1.hi + s1.lo, lo = s1.lo - (hi - s1.hi), m = hi / (float)n;
+                    const float rest = __fmaf_rn(-m, (float)n, hi) + lo;        // sum d - n m
+                    const DF sq = df_prod(m, hi);
+                    const DF d = df_add(s2, DF{-sq.hi, -(sq.lo + m * (lo + rest))});
+                    const float v = d.hi + d.lo;
+                    wm[h][q] = m;
+                    wv[h][q] = v * 65.f >= s2.hi + s2.lo ? fmaxf(v, 0.f) : -1.f;
+                    if (ky0 + q + 1 < npa && q + 1 < ZNCC_SEG) {
+                        df_acc(s1, -row1[(ky0 + q) * npa + kx]);
+                        df_acc(s1, row1[(ky0 + q + win) * npa + kx]);
+                        df_acc(s2, -row2[(ky0 + q) * npa + kx]);
+                        df_acc(s2, row2[(ky0 + q + win) * npa + kx]);
+                    }
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int h = 0; h < ZNCC_TPT; ++h) {
+            const int task = threadIdx.x + h * blockDim.x, kx = task % npa, ky0 = (task / npa) * ZNCC_SEG;
+            if (task < npa * segs)
+#pragma unroll
+                for (int q = 0; q < ZNCC_SEG; ++q)
+                    if (ky0 + q < npa) {
+                        mean[(ky0 + q) * npa + kx] = wm[h][q];
+                        var[(ky0 + q) * npa + kx] = wv[h][q];
+                    }
+        }
+        __syncthreads();
+        // the correlation: 2 rows x R columns of offsets per thread
+        const int nbx = (npa + R - 1) / R, nby = (npa + 1) / 2;
+        for (int t = threadIdx.x; t < nbx * nby; t += blockDim.x) {
+            // rows ky and ky + nby: neighbouring threads read neighbouring rows, an odd number of words apart
+            const int ky = t % nby, kx0 = (t / nby) * R;
+            const bool two = ky + nby < npa;
+            const float *p0 = pat + ky * ps + kx0, *p1 = two ? p0 + nby * ps : p0;
+            Pair acc[R];
+#pragma unroll
+            for (int q = 0; q < R; ++q) acc[q] = pair(0.f, 0.f);
+            for (int i = 0; i < win; ++i, p0 += ps, p1 += ps) {
+                const float *ti = tpl + i * win;
+                Pair w[R];                                 // sliding window: column j + q at (j + q) % R
+#pragma unroll
+                for (int q = 0; q < R - 1; ++q) w[q] = pair(p0[q], p1[q]);
+                auto column = [&](int j, int q) {          // q = j mod R, known at compile time
+                    const Pair tv = pair(ti[j], ti[j]);
+                    w[(q + R - 1) % R] = pair(p0[j + R - 1], p1[j + R - 1]);
+#pragma unroll
+                    for (int o = 0; o < R; ++o) acc[o] = pair_fma(w[(q + o) % R], tv, acc[o]);
+                };
+                int j = 0;
+                for (; j + R <= win; j += R)
+#pragma unroll
+                    for (int q = 0; q < R; ++q) column(j + q, q);
+#pragma unroll
+                for (int q = 0; q < R - 1; ++q)             // the last win % R columns
+                    if (j + q < win) column(j + q, q);
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (h == 0 || two)
+#pragma unroll
+                    for (int q = 0; q < R; ++q)
+                        if (kx0 + q < npa) {
+                            const int o = (ky + h * nby) * npa + kx0 + q;
+                            const float v = var[o], cr = (h == 0 ? pair_lo(acc[q]) : pair_hi(acc[q])) - mean[o] * t1;
+                            float sc = cr / (sqrtf(v / (float)n) + 1e-12f) / (float)n;
+                            if (v < 0.f) sc = zncc_two_pass(pat + (ky + h * nby) * ps + kx0 + q, ps, tpl, win);
+                            if (sc > best || (sc == best && o < bidx)) {   // offsets are not visited in order
+                                best = sc;
+                                bidx = o;
+                            }
+                        }
+        }
+    }
+    // block argmax: larger score, then smaller index
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const float ob = __shfl_xor_sync(0xffffffffu, best, off);
+        const int oi = __shfl_xor_sync(0xffffffffu, bidx, off);
+        if (ob > best || (ob == best && oi < bidx)) {
+            best = ob;
+            bidx = oi;
+        }
+    }
+    __syncthreads();
+    if (lane == 0) {
+        s_red[wid] = best;
+        s_idx[wid] = bidx;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float b = s_red[0];
+        int bi = s_idx[0];
+        for (int w = 1; w < nw; ++w)
+            if (s_red[w] > b || (s_red[w] == b && s_idx[w] < bi)) {
+                b = s_red[w];
+                bi = s_idx[w];
+            }
+        const int ky = bi / npa, kx = bi % npa;
+        u_out[c] = make_float2((float)(xs + kx - x), (float)(ys + ky - y));
+        score_out[c] = b;
+    }
+}
+
+// Windows and search ranges beyond what zncc_kernel's row sums and tasks hold: one offset per thread.
+__global__ void __launch_bounds__(1024) zncc_wide_kernel(const float *__restrict__ ref, int Hr, int Wr, const float *__restrict__ def, int Hd,
                             int Wd, const float2 *__restrict__ centers, int win, int search, float2 *__restrict__ u_out,
                             float *__restrict__ score_out) {
     extern __shared__ float sm[];
@@ -217,20 +525,44 @@ extern "C" int d2ic_zncc_match(const float *ref, int Hr, int Wr, const float *de
     D2IC_REQUIRE(ref && def && u_out && score_out && (centers || n_centers == 0), "d2ic_zncc_match: null pointer");
     D2IC_REQUIRE(win > 0 && (win % 2) == 1, "d2ic_zncc_match: win must be odd and positive (got %d)", win);
     D2IC_REQUIRE(search >= 0 && n_centers >= 0 && Hr > 0 && Wr > 0 && Hd > 0 && Wd > 0, "d2ic_zncc_match: bad sizes");
-    const size_t smem = sizeof(float) * ((size_t)win * win + (size_t)(win + 2 * search) * (win + 2 * search));
-    D2IC_REQUIRE(smem <= 200 * 1024, "d2ic_zncc_match: win/search too large for shared memory (%zu bytes)", smem);
+    const size_t base = (size_t)win * win + (size_t)(win + 2 * search) * (win + 2 * search);
+    D2IC_REQUIRE(sizeof(float) * base <= 200 * 1024, "d2ic_zncc_match: win/search too large for shared memory (%zu bytes)",
+                 sizeof(float) * base);
     if (n_centers == 0) return D2IC_OK;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(zncc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // R columns of offsets per thread: the fewest multiply-adds on columns beyond the search range
+    const int npa = 2 * search + 1, ps = win + 2 * search;
+    auto blocks = [&](int R) { return (npa + R - 1) / R; };
+    int R = 7;
+    for (int q = 6; q >= 5; --q)
+        if (blocks(q) * q < blocks(R) * R) R = q;
+    const int tasks = blocks(R) * ((npa + 1) / 2);
+    int threads = ((tasks + 31) / 32) * 32;
+    threads = threads < 64 ? 64 : (threads > ZNCC_MAX_THREADS ? ZNCC_MAX_THREADS : threads);
+    const size_t smem = sizeof(float) * (base + R + 2 * (size_t)ps * npa);
+    // the register-blocked form where its row sums fit in shared memory and its column tasks in the block
+    // (search <= 34 at win 41); the wide form, one offset per thread, beyond
+    if (smem <= 200 * 1024 && npa * ((npa + ZNCC_SEG - 1) / ZNCC_SEG) <= ZNCC_TPT * threads) {
+        auto launch = [&](auto kernel) {
+            if (smem > 48 * 1024) {
+                cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                if (e != cudaSuccess) return cuda_status(e, "zncc smem attribute");
+            }
+            kernel<<<n_centers, threads, smem, (cudaStream_t)stream>>>(ref, Hr, Wr, def, Hd, Wd, (const float2 *)centers,
+                                                                      win, search, (float2 *)u_out, score_out);
+            D2IC_CHECK_LAUNCH("zncc_kernel");
+            return (int)D2IC_OK;
+        };
+        return R == 7 ? launch(zncc_kernel<7>) : (R == 6 ? launch(zncc_kernel<6>) : launch(zncc_kernel<5>));
+    }
+    const size_t wide = sizeof(float) * base;
+    if (wide > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(zncc_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wide);
         if (e != cudaSuccess) return cuda_status(e, "zncc smem attribute");
     }
-    // one thread per offset where they fit in a block (289 offsets at search 8: 320 threads), so that
-    // no thread scores a second offset while the others wait
-    const int npa = 2 * search + 1;
-    const int threads = npa * npa >= 1024 ? 1024 : ((npa * npa + 31) / 32) * 32;
-    zncc_kernel<<<n_centers, threads < 64 ? 64 : threads, smem, (cudaStream_t)stream>>>(
+    const int wide_threads = npa * npa >= 1024 ? 1024 : ((npa * npa + 31) / 32) * 32;
+    zncc_wide_kernel<<<n_centers, wide_threads < 64 ? 64 : wide_threads, wide, (cudaStream_t)stream>>>(
         ref, Hr, Wr, def, Hd, Wd, (const float2 *)centers, win, search, (float2 *)u_out, score_out);
-    D2IC_CHECK_LAUNCH("zncc_kernel");
+    D2IC_CHECK_LAUNCH("zncc_wide_kernel");
     return D2IC_OK;
 }
 
