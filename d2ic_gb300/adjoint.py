@@ -14,7 +14,8 @@ right-hand sides runs on those blocks (chunk -> slot -> node, no atomics), the
 mixed term is a pixel pass over an image direction's B-spline coefficients and
 its adjoint is the backward of the bicubic sampling (scatter + transposed
 prefilter).  The right-hand sides of all noise realisations are solved
-together by a block-Jacobi preconditioned CG (FP64 vectors, FP32 matvec).
+together by a block-Jacobi preconditioned CG (double-float vectors on the chip,
+FP32 matvec).
 """
 from __future__ import annotations
 
@@ -115,8 +116,8 @@ class ImplicitAdjoint:
         return Y.to(torch.float64)
 
     def solve(self, B: torch.Tensor, rtol: float = 1e-7, max_iter: int = 2000):
-        """X = H^-1 B column by column: block-Jacobi PCG, all columns in lock step, run by
-        ``d2ic_pcg_solve`` (FP64 vectors, FP32 Hessian matvec, deterministic reductions)."""
+        """X = H^-1 B column by column: block-Jacobi PCG, up to 64 columns in lock step, run by
+        ``d2ic_pcg_solve`` (double-float vectors, FP32 Hessian matvec, deterministic reductions)."""
         import ctypes
         L = self.L
         B = B.to(device=self.dev, dtype=torch.float64).contiguous()

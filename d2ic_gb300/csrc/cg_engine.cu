@@ -165,12 +165,6 @@ __device__ inline Ctl make_ctl(char *base, int n) {
     return c;
 }
 
-__device__ __forceinline__ unsigned long long gtimer() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -178,10 +172,6 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
 }
 
 __device__ __forceinline__ int ld_vol(const int *p) { return *(volatile const int *)p; }
-
-// Orders this thread's earlier accesses (and those it has observed) before its later ones for the GPU:
-// the acquire/release fence, lighter than __threadfence(), which is sequentially consistent.
-__device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
 // Warp sums of five double-floats by a reduce-scatter butterfly: at the exchange distances 16, 8 and 4
 // a lane keeps half of its values and adds its partner's copy of that half, so the five sums take 8
@@ -207,27 +197,6 @@ __device__ __forceinline__ DF df_reduce5(const DF q[5], int lane) {
     DF v = df_add(b2 ? c1 : c0, df_shfl_xor(b2 ? c0 : c1, 4));
     v = df_add(v, df_shfl_xor(v, 2));
     return df_add(v, df_shfl_xor(v, 1));
-}
-
-// 16-byte records that carry their own round tag: one 128-bit access is a single memory operation
-// (ld/st.b128 of the PTX memory model), so a reader that finds the tag has the data of the same
-// write.  A producer therefore needs no fence and no counter to hand over a record, and the
-// consumer polls the record itself: one L2 round trip from the store to the value, instead of
-// store, fence, atomic, polled counter, load.
-__device__ __forceinline__ uint4 ld_record(const void *p) {
-    unsigned long long lo, hi;
-    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
-                 : "=l"(lo), "=l"(hi)
-                 : "l"(p)
-                 : "memory");
-    return make_uint4((unsigned)lo, (unsigned)(lo >> 32), (unsigned)hi, (unsigned)(hi >> 32));
-}
-__device__ __forceinline__ void st_record(void *p, uint4 v) {
-    const unsigned long long lo = (unsigned long long)v.x | ((unsigned long long)v.y << 32);
-    const unsigned long long hi = (unsigned long long)v.z | ((unsigned long long)v.w << 32);
-    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
-                 "l"(lo), "l"(hi)
-                 : "memory");
 }
 
 // Control data is rewritten by other blocks during the launch: read it through

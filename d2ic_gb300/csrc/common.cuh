@@ -182,6 +182,37 @@ __device__ __forceinline__ DF df_warp_sum(DF v) {
 }
 __device__ __forceinline__ double df_to_double(DF v) { return (double)v.hi + (double)v.lo; }
 
+__device__ __forceinline__ unsigned long long gtimer() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// Orders this thread's earlier accesses (and those it has observed) before its later ones for the GPU:
+// the acquire/release fence, lighter than __threadfence(), which is sequentially consistent.
+__device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
+// 16-byte records that carry their own round tag: one 128-bit access is a single memory operation
+// (ld/st.b128 of the PTX memory model), so a reader that finds the tag has the data of the same
+// write.  A producer therefore needs no fence and no counter to hand over a record, and the
+// consumer polls the record itself: one L2 round trip from the store to the value, instead of
+// store, fence, atomic, polled counter, load.
+__device__ __forceinline__ uint4 ld_record(const void *p) {
+    unsigned long long lo, hi;
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(lo), "=l"(hi)
+                 : "l"(p)
+                 : "memory");
+    return make_uint4((unsigned)lo, (unsigned)(lo >> 32), (unsigned)hi, (unsigned)(hi >> 32));
+}
+__device__ __forceinline__ void st_record(void *p, uint4 v) {
+    const unsigned long long lo = (unsigned long long)v.x | ((unsigned long long)v.y << 32);
+    const unsigned long long hi = (unsigned long long)v.z | ((unsigned long long)v.w << 32);
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+                 "l"(lo), "l"(hi)
+                 : "memory");
+}
+
 __device__ __forceinline__ double warp_sum_d(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -14,13 +14,13 @@
 // columns.  This replaces the chunk -> node-slot -> node pass per product (one
 // write and one read of node_chunk_k * Nn * 2 * K floats per product).
 //
-// PCG: per iteration AP = H P with the block partials of P.AP, their column sums,
-// the update of X, R, Z with the partials of R.R and R.Z, their column sums (one
-// warp per column, blocks summed in a fixed order: deterministic) and the new
-// direction.  The last block of the second column sum decides convergence
-// (||R|| <= rtol ||B|| for every column) into a device flag that makes the later
-// kernels return at once, so the host launches iterations in batches and reads
-// the flag once per batch instead of synchronising every iteration.
+// PCG: one cooperative launch runs all iterations of up to 64 columns with the vectors in shared memory
+// (pcg_resident).  Meshes whose vectors do not fit on the chip keep them in memory and run five kernels
+// per iteration: AP = H P with the block partials of P.AP, their column sums, the update of X, R, Z with
+// the partials of R.R and R.Z, their column sums (one warp per column, blocks summed in a fixed order:
+// deterministic) and the new direction; the last block of the second column sum decides convergence
+// (||R|| <= rtol ||B|| for every column) into a device flag that makes the later kernels return at once,
+// so the host launches iterations in batches and reads the flag once per batch.
 #include <stdlib.h>
 #include <string.h>
 
@@ -504,6 +504,494 @@ __global__ void __launch_bounds__(PT) pcg_dir(int n_nodes, int K, const double *
     }
 }
 
+// ---------------------------------------------------------------------------
+// PCG with the vectors on the chip
+// ---------------------------------------------------------------------------
+// One launch runs all iterations of up to PR_COLS columns: block b owns a range of nodes and keeps X, R,
+// P and H P of its (node, column) pairs in shared memory; only P in FP32, which neighbours need, goes
+// through global memory.  Per iteration: H P and P.HP; the step with R.R and R.Z; the new direction.  A
+// sum over the grid is two hops of tagged records (the block's partial to the warp that owns the sum,
+// the sum to every block), the exchange of P one grid barrier; a system that fits one block needs only
+// block barriers.
+//
+// The vectors and the sums are double-floats (48 bits) instead of FP64: GB300 issues an FP64
+// instruction per SM every 16 cycles, so the 12 FP64 operations per vector entry and iteration cost 20 us
+// at 7,396 nodes x 64 columns, the same in double-float 3 us; the product with H is FP32 either way.
+// Columns are scaled by a power of two to a largest entry in [1, 2), so that FP32's exponent range
+// suffices.  Errors against an FP64 solve are those of the FP32 operator, 1.8e-6, as before.
+//
+// Bound by the hops at few columns (two sums and a barrier, about 6 us) and by the double-float
+// arithmetic and the latency of the neighbours' values at many.  Per iteration, five kernels before ->
+// now: 7,569 nodes x 64 columns 66 -> 26 us, 4,331 x 6 55 -> 12 us, 1,089 x 1 (one block) 27 -> 12 us.
+constexpr int PR_T = 512;                  // threads per block
+constexpr int PR_PAIR_BYTES = 7 * 8;       // x, r, p (two components, double-float) and two floats of H P
+constexpr int PR_NODE_BYTES = 4 * HOP + 32;   // the operator's column nodes and the preconditioner block
+constexpr int PR_BLOCK_BYTES = 16 * HOP;       // the operator's blocks of a node
+constexpr int PR_BYTES = 212 * 1024;       // dynamic shared memory per block at most
+constexpr int PR_COLS = 64;                // columns per launch
+constexpr int PR_POLL = 5;                 // records a lane polls at a time: 160 blocks in one round trip
+constexpr int PR_ONE_BLOCK = 2048;         // systems of at most this many pairs run in one block
+constexpr unsigned long long PR_WAIT_NS = 5ull * 1000ull * 1000ull * 1000ull;
+
+struct PrArgs {
+    const int *idx;                        // the operator
+    const float4 *blk;
+    const int *overflow;                   // the assembly's error flag
+    const float2 *M;                       // inverse diagonal blocks, 4 double-floats per node
+    const unsigned char *act;
+    const double *B;
+    double *X;
+    float *P;                              // exchanged direction: (node, component, column of the launch)
+    uint4 *part, *tot;                     // records: partials (sum, block), totals
+    unsigned *bar;                         // barrier arrivals
+    int *out;                              // iterations (max over launches), status
+    int n_nodes, K, k0, Kb, max_iter;      // columns k0 .. k0 + Kb of K
+    int staged;                            // operator indices and preconditioner in shared memory
+    double rtol;
+};
+
+__device__ __forceinline__ DF df_mul(DF a, DF b) {
+    const DF p = df_prod(a.hi, b.hi);
+    const float lo = p.lo + __fmaf_rn(a.hi, b.lo, a.lo * b.hi);
+    const float h = p.hi + lo;
+    return {h, lo - (h - p.hi)};
+}
+__device__ __forceinline__ DF df_mul_f(DF a, float b) {
+    const DF p = df_prod(a.hi, b);
+    const float lo = __fmaf_rn(a.lo, b, p.lo), h = p.hi + lo;
+    return {h, lo - (h - p.hi)};
+}
+__device__ __forceinline__ DF df_neg(DF a) { return {-a.hi, -a.lo}; }
+__device__ __forceinline__ DF df_div(DF a, DF b) {   // two quotient digits
+    const float q1 = a.hi / b.hi;
+    const DF r = df_add(a, df_neg(df_mul_f(b, q1)));
+    return df_two_sum(q1, r.hi / b.hi);
+}
+__device__ __forceinline__ DF df_from(double x) {
+    const float hi = (float)x;
+    return {hi, (float)(x - (double)hi)};
+}
+
+// the block's shared state
+struct PrShared {
+    DF red[2][PR_T];
+    DF tot[2 * PR_COLS];
+    DF a[PR_COLS], rz[PR_COLS];
+    double thr[PR_COLS];
+    int scale[PR_COLS];                    // biased FP64 exponent of the column's largest entry
+    int stop;                              // a wait ran out somewhere
+};
+extern __shared__ __align__(16) unsigned char pr_dyn[];
+
+struct PrSum {
+    __device__ static DF op(DF a, DF b) { return df_add(a, b); }
+};
+struct PrMax {                             // non-negative integers in the first word
+    __device__ static DF op(DF a, DF b) { return __float_as_int(a.hi) >= __float_as_int(b.hi) ? a : b; }
+};
+
+// whole warp: polls the records rec[lane], rec[lane + 32], ... below n, N at most per lane, until all
+// carry the tag; false after an abort
+template <int N>
+__device__ __forceinline__ bool pr_poll(const uint4 *rec, int n, unsigned tag, uint4 (&r)[N], int *out, int lane) {
+    unsigned long long t0 = 0;
+    for (unsigned it = 0;; ++it) {
+        bool all = true;
+#pragma unroll
+        for (int i = 0; i < N; ++i) r[i] = lane + 32 * i < n ? ld_record(rec + lane + 32 * i) : make_uint4(0u, 0u, tag, 0u);
+#pragma unroll
+        for (int i = 0; i < N; ++i) all = all && r[i].z == tag;
+        if (__all_sync(0xffffffffu, all)) return true;
+        if ((it & 63) == 63) {
+            int go = 1;
+            if (lane == 0) {
+                const unsigned long long now = gtimer();
+                if (t0 == 0) t0 = now;
+                if (*(volatile int *)(out + 1) != 0) go = 0;
+                else if (now - t0 > PR_WAIT_NS) {
+                    atomicExch(out + 1, D2IC_WAIT_TIMEOUT);
+                    go = 0;
+                }
+            }
+            if (!__shfl_sync(0xffffffffu, go, 0)) return false;
+        }
+    }
+}
+
+// Reduces NV values per thread (thread t: column t % Kb) over the grid into S.tot[v * Kb + k], in a fixed
+// order; false after an abort.  tag: unique per call.
+template <int NV, class OP>
+__device__ bool pr_reduce(const DF *v, const PrArgs &A, PrShared &S, int T, int rows, unsigned tag) {
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, Kb = A.Kb, row = tid / Kb, k = tid % Kb;
+    const int G = gridDim.x;
+    DF w[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) w[i] = v[i];
+    int h = rows, r = row;                 // rows of Kb values left, this thread's row
+    bool mine = tid < T;
+    if (32 % Kb == 0) {                    // the warp's rows first, without barriers
+#pragma unroll 1
+        for (int o = 16; o >= Kb; o >>= 1)
+#pragma unroll
+            for (int i = 0; i < NV; ++i)
+                w[i] = OP::op(w[i], DF{__shfl_xor_sync(0xffffffffu, w[i].hi, o), __shfl_xor_sync(0xffffffffu, w[i].lo, o)});
+        h = PR_T / 32;
+        r = wid;
+        mine = lane < Kb;
+    }
+    const int at = r * Kb + k;
+    __syncthreads();                       // the previous totals have been read
+    if (mine)
+#pragma unroll
+        for (int i = 0; i < NV; ++i) S.red[i][at] = w[i];
+    while (h > 1) {
+        const int half = (h + 1) >> 1;
+        __syncthreads();
+        if (mine && r < h - half)
+#pragma unroll
+            for (int i = 0; i < NV; ++i) S.red[i][at] = OP::op(S.red[i][at], S.red[i][at + half * Kb]);
+        h = half;
+    }
+    if (G == 1) {
+        if (tid < Kb)
+#pragma unroll
+            for (int i = 0; i < NV; ++i) S.tot[i * Kb + tid] = S.red[i][tid];
+        __syncthreads();
+        return true;
+    }
+    const int items = NV * Kb;
+    if (tid < Kb)
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+            st_record(A.part + (size_t)(i * Kb + tid) * G + blockIdx.x,
+                      make_uint4(__float_as_uint(S.red[i][tid].hi), __float_as_uint(S.red[i][tid].lo), tag, 0u));
+    bool ok = true;
+    for (int m = blockIdx.x + G * wid; m < items && ok; m += G * (PR_T / 32)) {   // sums this block owns
+        DF t = {0.f, 0.f};
+        for (int g0 = 0; g0 < G && ok; g0 += 32 * PR_POLL) {
+            uint4 r[PR_POLL];
+            ok = pr_poll<PR_POLL>(A.part + (size_t)m * G + g0, G - g0, tag, r, A.out, lane);
+#pragma unroll
+            for (int i = 0; i < PR_POLL; ++i)
+                if (g0 + lane + 32 * i < G) {
+                    const DF x = {__uint_as_float(r[i].x), __uint_as_float(r[i].y)};
+                    t = g0 + i == 0 ? x : OP::op(t, x);
+                }
+        }
+#pragma unroll 1
+        for (int o = 16; o > 0; o >>= 1)
+            t = OP::op(t, DF{__shfl_xor_sync(0xffffffffu, t.hi, o), __shfl_xor_sync(0xffffffffu, t.lo, o)});
+        if (lane == 0 && ok)
+            st_record(A.tot + m, make_uint4(__float_as_uint(t.hi), __float_as_uint(t.lo), tag, 0u));
+    }
+    for (int m0 = wid * 32; m0 < items && ok; m0 += PR_T) {
+        uint4 r[1];
+        ok = pr_poll<1>(A.tot + m0, items - m0, tag, r, A.out, lane);
+        if (ok && m0 + lane < items) S.tot[m0 + lane] = DF{__uint_as_float(r[0].x), __uint_as_float(r[0].y)};
+    }
+    if (!ok && lane == 0) S.stop = 1;
+    __syncthreads();
+    return S.stop == 0;
+}
+
+// every block's writes before it are seen by every block after it; false after an abort
+__device__ bool pr_barrier(const PrArgs &A, PrShared &S, unsigned phase) {
+    __syncthreads();
+    if (gridDim.x == 1) return true;
+    if (threadIdx.x == 0) {
+        fence_acq_rel();
+        atomicAdd(A.bar, 1u);
+        const unsigned target = phase * gridDim.x;
+        unsigned long long t0 = 0;
+        for (unsigned it = 0; *(volatile unsigned *)A.bar < target; ++it)
+            if ((it & 63) == 63) {
+                const unsigned long long now = gtimer();
+                if (t0 == 0) t0 = now;
+                if (*(volatile int *)(A.out + 1) != 0) {
+                    S.stop = 1;
+                    break;
+                }
+                if (now - t0 > PR_WAIT_NS) {
+                    atomicExch(A.out + 1, D2IC_WAIT_TIMEOUT);
+                    S.stop = 1;
+                    break;
+                }
+            }
+        fence_acq_rel();
+    }
+    __syncthreads();
+    return S.stop == 0;
+}
+
+__global__ void __launch_bounds__(PR_T, 1) pcg_resident(const PrArgs A) {
+    __shared__ PrShared S;
+    const int Kb = A.Kb, tid = threadIdx.x;
+    const int per = (A.n_nodes + gridDim.x - 1) / gridDim.x;
+    const int n0 = min((int)blockIdx.x * per, A.n_nodes), nn = min(per, A.n_nodes - n0);
+    // thread t < T has column t % Kb and the block's nodes row, row + rows, ...
+    const int rows = PR_T / Kb, T = rows * Kb, k = tid % Kb, row = tid / Kb;
+    const int cap = per * Kb;                            // pairs of a full block
+    float2 *x = reinterpret_cast<float2 *>(pr_dyn), *r = x + 2 * cap, *p = r + 2 * cap;   // component c at c * cap
+    float *ap = reinterpret_cast<float *>(p + 2 * cap);
+    // with A.staged, the block's nodes' column indices (none for an inactive node) and preconditioner
+    // blocks: every grid barrier empties the L1, so from global memory they cost an L2 round trip per node
+    float4 *sM = reinterpret_cast<float4 *>(pr_dyn + (((size_t)cap * PR_PAIR_BYTES + 15) & ~(size_t)15));
+    int *sidx = reinterpret_cast<int *>(sM + 2 * per);
+    // with A.staged 2 also the operator's blocks
+    float4 *sblk = reinterpret_cast<float4 *>(sidx + HOP * per);
+    if (A.staged == 2)
+        for (int i = tid; i < nn * HOP; i += PR_T) sblk[i] = __ldg(A.blk + (size_t)n0 * HOP + i);
+    if (A.staged) {
+        for (int i = tid; i < nn * 2; i += PR_T) sM[i] = __ldg(reinterpret_cast<const float4 *>(A.M) + 2 * (size_t)n0 + i);
+        for (int i = tid; i < nn * HOP; i += PR_T) sidx[i] = A.act[n0 + i / HOP] ? __ldg(A.idx + (size_t)n0 * HOP + i) : -1;
+    }
+    if (tid == 0) S.stop = 0;
+    if (*A.overflow) return;                             // every block: the host reports it
+    unsigned tag = 0, phase = 0;
+    auto pairs = [&](auto &&f) {
+        if (tid < T)
+            for (int i = row; i < nn; i += rows) f(n0 + i, i * Kb + k);
+    };
+    auto ld = [](float2 v) { return DF{v.x, v.y}; };
+    auto st = [](DF v) { return make_float2(v.hi, v.lo); };
+    auto precond = [&](int n, DF r0, DF r1, DF &z0, DF &z1) {
+        const float4 m0 = A.staged ? sM[2 * (n - n0)] : __ldg(reinterpret_cast<const float4 *>(A.M) + 2 * (size_t)n);
+        const float4 m1 = A.staged ? sM[2 * (n - n0) + 1] : __ldg(reinterpret_cast<const float4 *>(A.M) + 2 * (size_t)n + 1);
+        z0 = df_add(df_mul(DF{m0.x, m0.y}, r0), df_mul(DF{m0.z, m0.w}, r1));
+        z1 = df_add(df_mul(DF{m1.x, m1.y}, r0), df_mul(DF{m1.z, m1.w}, r1));
+    };
+    auto put_p = [&](int n, DF p0, DF p1) {
+        float *o = A.P + (size_t)n * 2 * Kb + k;
+        o[0] = p0.hi;
+        o[Kb] = p1.hi;
+    };
+    // the columns' scales
+    int e = 0;
+    pairs([&](int n, int) {
+        const size_t i0 = (size_t)n * 2 * A.K + A.k0 + k;
+        if (A.act[n]) {
+            e = max(e, (__double2hiint(A.B[i0]) >> 20) & 0x7ff);
+            e = max(e, (__double2hiint(A.B[i0 + A.K]) >> 20) & 0x7ff);
+        }
+    });
+    DF v[2] = {DF{__int_as_float(e), 0.f}, DF{0.f, 0.f}};
+    if (!pr_reduce<1, PrMax>(v, A, S, T, rows, ++tag)) return;
+    if (tid < Kb) {
+        const int m = __float_as_int(S.tot[tid].hi);
+        S.scale[tid] = m == 0 || m == 0x7ff ? 1023 : min(m, 2045);
+    }
+    __syncthreads();
+    const double up = __hiloint2double(min(max(2046 - S.scale[k], 1), 2046) << 20, 0);   // 2^(1023 - scale)
+    // X = 0, R = B, Z = M R, P = Z
+    v[0] = v[1] = DF{0.f, 0.f};
+    pairs([&](int n, int i) {
+        const size_t i0 = (size_t)n * 2 * A.K + A.k0 + k;
+        const bool on = A.act[n] != 0;
+        const DF r0 = on ? df_from(A.B[i0] * up) : DF{0.f, 0.f}, r1 = on ? df_from(A.B[i0 + A.K] * up) : DF{0.f, 0.f};
+        DF z0, z1;
+        precond(n, r0, r1, z0, z1);
+        x[i] = x[cap + i] = make_float2(0.f, 0.f);
+        r[i] = st(r0);
+        r[cap + i] = st(r1);
+        p[i] = st(z0);
+        p[cap + i] = st(z1);
+        put_p(n, z0, z1);
+        v[0] = df_add(v[0], df_add(df_mul(r0, z0), df_mul(r1, z1)));
+        v[1] = df_add(v[1], df_add(df_mul(r0, r0), df_mul(r1, r1)));
+    });
+    if (!pr_reduce<2, PrSum>(v, A, S, T, rows, ++tag)) return;
+    if (tid < Kb) {
+        S.rz[tid] = S.tot[tid];
+        const double bn = A.rtol * fmax(sqrt(df_to_double(S.tot[Kb + tid])), 1e-300);
+        S.thr[tid] = bn * bn;
+    }
+    if (!pr_barrier(A, S, ++phase)) return;
+    int it = 0;
+    while (it < A.max_iter) {
+        // AP = H P and P.AP
+        v[0] = DF{0.f, 0.f};
+        pairs([&](int n, int i) {
+            float y0 = 0.f, y1 = 0.f;
+            const float *P = A.P + k;
+            if (A.staged == 2) {
+                // a node couples to nine nodes on a regular grid: their values are all in flight together
+                const int4 *ix = reinterpret_cast<const int4 *>(sidx + (n - n0) * HOP);
+                const float4 *bl = sblk + (n - n0) * HOP;
+                constexpr int Q = 12;
+                for (int q0 = 0; q0 < HOP && ix[q0 / 4].x >= 0; q0 += Q) {
+                    float vx[Q], vy[Q];
+#pragma unroll
+                    for (int q = 0; q < Q; q += 4) {
+                        const int4 j4 = q0 + q < HOP ? ix[(q0 + q) / 4] : make_int4(-1, -1, -1, -1);
+                        const int jj[4] = {j4.x, j4.y, j4.z, j4.w};
+#pragma unroll
+                        for (int t = 0; t < 4; ++t) {
+                            vx[q + t] = jj[t] >= 0 ? P[(size_t)jj[t] * 2 * Kb] : 0.f;
+                            vy[q + t] = jj[t] >= 0 ? P[(size_t)jj[t] * 2 * Kb + Kb] : 0.f;
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < Q; ++q)
+                        if (q0 + q < HOP) {                // blocks beyond the last entry are zero
+                            const float4 b = bl[q0 + q];
+                            y0 = __fmaf_rn(b.x, vx[q], __fmaf_rn(b.y, vy[q], y0));
+                            y1 = __fmaf_rn(b.y, vx[q], __fmaf_rn(b.z, vy[q], y1));
+                        }
+                }
+            } else {
+                const float4 *bl = A.blk + (size_t)n * HOP;
+                const bool on = A.staged || A.act[n];
+                constexpr int Q = 4;                           // entries in flight together, nine on a regular grid
+                int4 j4 = make_int4(-1, -1, -1, -1);
+                if (on) j4 = A.staged ? *reinterpret_cast<const int4 *>(sidx + (n - n0) * HOP)
+                                      : __ldg(reinterpret_cast<const int4 *>(A.idx + (size_t)n * HOP));
+                for (int q0 = 0; q0 < HOP && j4.x >= 0; q0 += Q) {
+                    const int jj[Q] = {j4.x, j4.y, j4.z, j4.w};
+                    float4 b[Q];
+                    float vx[Q], vy[Q];
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) {
+                        const bool has = jj[q] >= 0;
+                        const float *src = P + (size_t)(has ? jj[q] : 0) * 2 * Kb;
+                        b[q] = has ? __ldg(bl + q0 + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        vx[q] = src[0];
+                        vy[q] = src[Kb];
+                    }
+                    j4 = make_int4(-1, -1, -1, -1);
+                    if (q0 + Q < HOP)
+                        j4 = A.staged ? *reinterpret_cast<const int4 *>(sidx + (n - n0) * HOP + q0 + Q)
+                                      : __ldg(reinterpret_cast<const int4 *>(A.idx + (size_t)n * HOP + q0 + Q));
+#pragma unroll
+                    for (int q = 0; q < Q; ++q)
+                        if (jj[q] >= 0) {
+                            y0 = __fmaf_rn(b[q].x, vx[q], __fmaf_rn(b[q].y, vy[q], y0));
+                            y1 = __fmaf_rn(b[q].y, vx[q], __fmaf_rn(b[q].z, vy[q], y1));
+                        }
+                }
+            }
+            ap[i] = y0;
+            ap[cap + i] = y1;
+            v[0] = df_add(v[0], df_add(df_mul_f(ld(p[i]), y0), df_mul_f(ld(p[cap + i]), y1)));
+        });
+        if (!pr_reduce<1, PrSum>(v, A, S, T, rows, ++tag)) return;
+        if (tid < Kb) S.a[tid] = S.tot[tid].hi > 0.f ? df_div(S.rz[tid], S.tot[tid]) : DF{0.f, 0.f};
+        __syncthreads();
+        // X += a P, R -= a AP, R.R and R.Z
+        const DF a = S.a[k];
+        v[0] = v[1] = DF{0.f, 0.f};
+        pairs([&](int n, int i) {
+            x[i] = st(df_add(ld(x[i]), df_mul(a, ld(p[i]))));
+            x[cap + i] = st(df_add(ld(x[cap + i]), df_mul(a, ld(p[cap + i]))));
+            const DF r0 = df_add(ld(r[i]), df_neg(df_mul_f(a, ap[i])));
+            const DF r1 = df_add(ld(r[cap + i]), df_neg(df_mul_f(a, ap[cap + i])));
+            r[i] = st(r0);
+            r[cap + i] = st(r1);
+            DF z0, z1;
+            precond(n, r0, r1, z0, z1);
+            v[0] = df_add(v[0], df_add(df_mul(r0, r0), df_mul(r1, r1)));
+            v[1] = df_add(v[1], df_add(df_mul(r0, z0), df_mul(r1, z1)));
+        });
+        if (!pr_reduce<2, PrSum>(v, A, S, T, rows, ++tag)) return;
+        ++it;
+        const int open = tid < Kb && !(df_to_double(S.tot[tid]) <= S.thr[tid]);
+        if (!__syncthreads_or(open)) break;
+        if (it == A.max_iter) break;
+        if (tid < Kb) {
+            const DF old = S.rz[tid], now = S.tot[Kb + tid];
+            S.a[tid] = old.hi > 0.f ? df_div(now, old) : DF{0.f, 0.f};
+            S.rz[tid] = now;
+        }
+        __syncthreads();
+        // P = Z + beta P
+        const DF beta = S.a[k];
+        pairs([&](int n, int i) {
+            DF z0, z1;
+            precond(n, ld(r[i]), ld(r[cap + i]), z0, z1);
+            const DF p0 = df_add(z0, df_mul(beta, ld(p[i]))), p1 = df_add(z1, df_mul(beta, ld(p[cap + i])));
+            p[i] = st(p0);
+            p[cap + i] = st(p1);
+            put_p(n, p0, p1);
+        });
+        if (!pr_barrier(A, S, ++phase)) return;
+    }
+    const double down = __hiloint2double(S.scale[k] << 20, 0);   // 2^(scale - 1023)
+    pairs([&](int n, int i) {
+        const size_t i0 = (size_t)n * 2 * A.K + A.k0 + k;
+        A.X[i0] = df_to_double(ld(x[i])) * down;
+        A.X[i0 + A.K] = df_to_double(ld(x[cap + i])) * down;
+    });
+    if (blockIdx.x == 0 && tid == 0) atomicMax(A.out, it);
+}
+
+// the inverse diagonal blocks as double-floats
+__global__ void pcg_blocks_df(const double *__restrict__ Minv, int n, float2 *__restrict__ M) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const DF v = df_from(Minv[i]);
+    M[i] = make_float2(v.hi, v.lo);
+}
+
+// Columns per launch and blocks of pcg_resident; 0 columns: the vectors do not fit on the chip.
+struct PrPlan {
+    int cols, blocks, staged;
+    size_t smem;
+};
+static PrPlan pr_plan(int n_nodes, int K, int sms) {
+    PrPlan p = {0, 0, 0, 0};
+    if (sms < 1) return p;
+    const long long pairs_max = PR_BYTES / PR_PAIR_BYTES - 1;
+    int cols = K < PR_COLS ? K : PR_COLS;
+    const long long per_all = (n_nodes + sms - 1) / sms;      // nodes per block on the whole chip
+    if (per_all * cols > pairs_max) cols = (int)(pairs_max / per_all);
+    if (cols < 1) return p;
+    const long long pairs = (long long)n_nodes * cols;
+    // one block where it fits (no grid hops); else blocks of at least a pair per thread
+    long long blocks = pairs <= PR_ONE_BLOCK ? 1 : (pairs + PR_T - 1) / PR_T;
+    if (blocks > sms) blocks = sms;
+    while (blocks < sms && ((n_nodes + blocks - 1) / blocks) * cols > pairs_max) ++blocks;
+    const long long per = (n_nodes + blocks - 1) / blocks;
+    p.cols = cols;
+    p.blocks = (int)blocks;
+    p.smem = (size_t)((per * cols * PR_PAIR_BYTES + 15) & ~15ll);
+    p.staged = p.smem + (size_t)per * PR_NODE_BYTES <= (size_t)PR_BYTES;
+    if (p.staged) p.smem += (size_t)per * PR_NODE_BYTES;
+    if (p.staged && p.smem + (size_t)per * PR_BLOCK_BYTES <= (size_t)PR_BYTES) {
+        p.staged = 2;
+        p.smem += (size_t)per * PR_BLOCK_BYTES;
+    }
+    return p;
+}
+
+struct PrWork {
+    float *P;
+    float2 *M;
+    uint4 *part, *tot;
+    unsigned *bar;
+    int *out;
+    char *op;
+    size_t zero;                            // bytes from part on to clear before a launch
+};
+static size_t pr_carve(int n_nodes, int K, int node_chunk_k, char *base, PrWork *w) {
+    const int cols = K < PR_COLS ? K : PR_COLS;
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        char *p = base ? base + off : nullptr;
+        off += al256(bytes);
+        return p;
+    };
+    w->P = (float *)take(sizeof(float) * (size_t)n_nodes * 2 * cols);
+    w->M = (float2 *)take(sizeof(float2) * 4 * (size_t)n_nodes);
+    w->out = (int *)take(2 * sizeof(int));
+    const size_t z0 = off;
+    w->part = (uint4 *)take(sizeof(uint4) * 2 * (size_t)cols * 1024);   // up to 1024 blocks
+    w->tot = (uint4 *)take(sizeof(uint4) * 2 * (size_t)cols);
+    w->bar = (unsigned *)take(sizeof(unsigned));
+    w->zero = off - z0;
+    HopView hv;
+    w->op = take(hop_layout(n_nodes, node_chunk_k, nullptr, &hv));
+    return off;
+}
+
 struct PcgWork {
     double *R, *Z, *P, *part_a, *part_b, *rz, *rz2, *pap, *rr, *bb;
     float *Pf, *AP;
@@ -615,10 +1103,12 @@ extern "C" int d2ic_hessian_apply(const void *op, int n_nodes, int node_chunk_k,
 
 extern "C" size_t d2ic_pcg_work_bytes(int n_nodes, int K, int node_chunk_k) {
     PcgWork w;
+    PrWork r;
     if (n_nodes < 1) n_nodes = 1;
     if (K < 1) K = 1;
     if (node_chunk_k < 1) node_chunk_k = 1;
-    return carve(n_nodes, K, node_chunk_k, nullptr, &w);
+    const size_t a = carve(n_nodes, K, node_chunk_k, nullptr, &w), b = pr_carve(n_nodes, K, node_chunk_k, nullptr, &r);
+    return a > b ? a : b;
 }
 
 extern "C" int d2ic_pcg_solve(const d2ic_frame_t *frame_dev, int n_chunks, int n_nodes, int node_chunk_k,
@@ -629,11 +1119,80 @@ extern "C" int d2ic_pcg_solve(const d2ic_frame_t *frame_dev, int n_chunks, int n
                      node_chunk_k >= 1 && max_iter >= 0,
                  "d2ic_pcg_solve: bad arguments");
     D2IC_REQUIRE(((uintptr_t)work & 255) == 0, "d2ic_pcg_solve: work must be 256-byte aligned");
-    PcgWork w;
-    const size_t need = carve(n_nodes, K, node_chunk_k, (char *)work, &w);
+    const size_t need = d2ic_pcg_work_bytes(n_nodes, K, node_chunk_k);
     D2IC_REQUIRE(work_bytes >= need, "d2ic_pcg_solve: work %zu bytes < %zu needed", work_bytes, need);
     cudaStream_t s = (cudaStream_t)stream;
     HopView hv;
+    int dev = 0, sms = 0, smem = 0, coop = 0;
+    cudaError_t de = cudaGetDevice(&dev);
+    if (de == cudaSuccess) de = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (de == cudaSuccess) de = cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (de == cudaSuccess) de = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    if (de != cudaSuccess) return cuda_status(de, "d2ic_pcg_solve: device attributes");
+    const PrPlan plan = pr_plan(n_nodes, K, sms < 1024 ? sms : 1024);
+    // the vectors on the chip wherever a column of them fits (547,000 nodes on 152 SMs), else in memory
+    if (plan.cols > 0 && coop && (size_t)PR_BYTES + sizeof(PrShared) <= (size_t)smem) {
+        PrWork r;
+        pr_carve(n_nodes, K, node_chunk_k, (char *)work, &r);
+        int st = assemble(frame_dev, n_chunks, n_nodes, node_chunk_k, chunk_hess, inv_np, alpha_reg, r.op, s, &hv);
+        if (st) return st;
+        pcg_blocks_df<<<(unsigned)((4 * (size_t)n_nodes + 255) / 256), 256, 0, s>>>(Minv, 4 * n_nodes, r.M);
+        D2IC_CHECK_LAUNCH("pcg_blocks_df");
+        cudaError_t e = cudaMemsetAsync(r.out, 0, 2 * sizeof(int), s);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(pcg_resident, cudaFuncAttributeMaxDynamicSharedMemorySize, PR_BYTES);
+        if (e != cudaSuccess) return cuda_status(e, "pcg set-up");
+        for (int k0 = 0; k0 < K; k0 += plan.cols) {
+            PrArgs A;
+            A.idx = hv.idx;
+            A.blk = hv.blk;
+            A.overflow = hv.err;
+            A.M = r.M;
+            A.act = active;
+            A.B = B;
+            A.X = X;
+            A.P = r.P;
+            A.part = r.part;
+            A.tot = r.tot;
+            A.bar = r.bar;
+            A.out = r.out;
+            A.n_nodes = n_nodes;
+            A.K = K;
+            A.k0 = k0;
+            A.Kb = K - k0 < plan.cols ? K - k0 : plan.cols;
+            A.max_iter = max_iter;
+            A.staged = plan.staged;
+            A.rtol = rtol;
+            e = cudaMemsetAsync(r.part, 0, r.zero, s);
+            if (e != cudaSuccess) return cuda_status(e, "pcg records");
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(plan.blocks);
+            cfg.blockDim = dim3(PR_T);
+            cfg.dynamicSmemBytes = plan.smem;
+            cfg.stream = s;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeCooperative;      // the blocks wait for one another
+            attr[0].val.cooperative = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            e = cudaLaunchKernelEx(&cfg, pcg_resident, A);
+            if (e != cudaSuccess) return cuda_status(e, "cooperative launch of pcg_resident");
+        }
+        int out[2] = {0, 0}, err = 0;
+        e = cudaMemcpyAsync(out, r.out, sizeof(out), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&err, hv.err, sizeof(int), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) return cuda_status(e, "pcg");
+        D2IC_REQUIRE(err == 0, "hessian assembly: a node couples to more than %d nodes", HOP);
+        if (out[1]) {
+            set_error("d2ic_pcg_solve: a wait between blocks ran out");
+            return out[1];
+        }
+        if (iters_out) *iters_out = out[0];
+        return D2IC_OK;
+    }
+    PcgWork w;
+    carve(n_nodes, K, node_chunk_k, (char *)work, &w);
     int st = assemble(frame_dev, n_chunks, n_nodes, node_chunk_k, chunk_hess, inv_np, alpha_reg, w.op, s, &hv);
     if (st) return st;
     cudaError_t e = cudaMemsetAsync(w.ctl, 0, sizeof(PcgCtl), s);

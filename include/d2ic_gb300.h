@@ -172,8 +172,10 @@ D2IC_API size_t d2ic_pcg_work_bytes(int n_nodes, int K, int node_chunk_k);
 /* X = H^-1 B for B, X (n_nodes, 2, K) FP64 (column index fastest), H assembled from chunk_hess
  * into the work buffer (as d2ic_hessian_assemble) and applied in FP32, Minv (n_nodes, 2, 2) FP64
  * inverse diagonal blocks (zero for inactive dofs), active (n_nodes) 0/1 mask.  Stops when every
- * column has ||R|| <= rtol ||B|| or after max_iter iterations (*iters_out); convergence is decided
- * on the device and read by the host once per batch of 8 iterations. */
+ * column of a launch (up to 64 columns) has ||R|| <= rtol ||B|| or after max_iter iterations
+ * (*iters_out: the most of any launch).  The vectors stay on the chip as double-floats where a
+ * column of them fits (547,000 nodes on 152 SMs), else in memory as FP64.  Blocks wait for one
+ * another (a cooperative launch): D2IC_WAIT_TIMEOUT if a wait runs out. */
 D2IC_API int d2ic_pcg_solve(const d2ic_frame_t *frame_dev, int n_chunks, int n_nodes, int node_chunk_k,
                             const float *chunk_hess, float inv_np, float alpha_reg, const double *Minv,
                             const unsigned char *active, const double *B, double *X, int K, double rtol,
