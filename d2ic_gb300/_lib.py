@@ -105,7 +105,9 @@ _SIGS = {
     "d2ic_mixed_term": (i32, [vp, i32, i32, vp, vp, f32, vp, vp, i32, i32, vp]),
     "d2ic_mixed_term_batch": (i32, [vp, i32, i32, i32, vp, vp, i32, ctypes.c_longlong, f32, vp, vp, i32, i32, vp]),
     "d2ic_mixed_term_T": (i32, [vp, i32, vp, vp, f32, vp, vp]),
+    "d2ic_mixed_term_T_batch": (i32, [vp, i32, vp, vp, i32, f32, vp, ctypes.c_longlong, vp]),
     "d2ic_bspline_prefilter_T": (i32, [vp, i32, i32, i32, i32, vp, vp, vp]),
+    "d2ic_bspline_prefilter_T_batch": (i32, [vp, i32, i32, i32, i32, i32, vp, vp, vp]),
     "d2ic_zncc_match":(i32, [vp, i32, i32, vp, i32, i32, vp, i32, i32, i32, vp, vp, vp]),
     "d2ic_idw_project": (i32, [vp, i32, vp, vp, i32, f32, vp, vp]),
     "d2ic_strain_gl": (i32, [vp, vp, vp, vp, i32, i32, f32, f32, vp, vp, vp]),

@@ -163,18 +163,24 @@ class ImplicitAdjoint:
 
     def mixed_T(self, lam: torch.Tensor) -> torch.Tensor:
         """Adjoint: (Nn, 2, K) -> image-space (K, H, W)."""
+        return self._mixed_T(lam, self.inv_np)
+
+    def _mixed_T(self, lam: torch.Tensor, scale: float) -> torch.Tensor:
+        """``scale`` times the unscaled adjoint, up to MIXED_BATCH fields per launch."""
         L = self.L
         K = lam.shape[2]
         out = torch.empty((K, L.H, L.W), dtype=torch.float32, device=self.dev)
-        gco = torch.empty((L.H + 2 * PAD, L.cpitch), dtype=torch.float32, device=self.dev)
-        tmp = torch.empty((L.H, L.cpitch), dtype=torch.float32, device=self.dev)
-        for k in range(K):
-            lk = lam[:, :, k].to(torch.float32).contiguous()
-            gco.zero_()
-            _lib.call("d2ic_mixed_term_T", ptr(self.desc), L.n_chunks, ptr(self.u), ptr(lk), self.inv_np, ptr(gco),
-                      _lib.stream_handle())
-            _lib.call("d2ic_bspline_prefilter_T", ptr(gco), L.H, L.W, PAD, L.cpitch, ptr(tmp), ptr(out[k]),
-                      _lib.stream_handle())
+        B = min(self.MIXED_BATCH, max(K, 1))
+        gco = torch.empty((B, L.H + 2 * PAD, L.cpitch), dtype=torch.float32, device=self.dev)
+        tmp = torch.empty((B, L.H, L.cpitch), dtype=torch.float32, device=self.dev)
+        s = _lib.stream_handle()
+        for k0 in range(0, K, B):
+            nb = min(B, K - k0)
+            lk = lam[:, :, k0:k0 + nb].to(torch.float32).contiguous()
+            gco[:nb].zero_()
+            _lib.call("d2ic_mixed_term_T_batch", ptr(self.desc), L.n_chunks, ptr(self.u), ptr(lk), nb, scale,
+                      ptr(gco), (L.H + 2 * PAD) * L.cpitch, s)
+            _lib.call("d2ic_bspline_prefilter_T_batch", ptr(gco), nb, L.H, L.W, PAD, L.cpitch, ptr(tmp), ptr(out[k0]), s)
         return out
 
     def jvp(self, dI: torch.Tensor, **kw) -> torch.Tensor:
@@ -185,7 +191,7 @@ class ImplicitAdjoint:
     def vjp(self, gu: torch.Tensor, **kw) -> torch.Tensor:
         """(du*/dI2)^T gu for gu (K, Nn, 2) -> (K, H, W)."""
         lam = self.solve(gu.to(torch.float64).permute(1, 2, 0).contiguous(), **kw)
-        return -self.mixed_T(lam)
+        return self._mixed_T(lam, -self.inv_np)
 
 
 def newton_polish(solver, state, def_image, u, alpha_reg: float, steps: int = 3, exact: bool = True):

@@ -409,8 +409,13 @@ D2IC_API int d2ic_mixed_term_batch(const d2ic_frame_t *frame_dev, int n_chunks, 
  * (d grad_u J / dI2 coefficients)^T lambda, by atomic scatter (backward of the bicubic sampling). */
 D2IC_API int d2ic_mixed_term_T(const d2ic_frame_t *frame_dev, int n_chunks, const float *u, const float *lam,
                                float scale, float *gcoeff, void *stream);
+/* The same for K fields lambda (n_nodes, 2, K), field k into gcoeff + k * coeff_stride floats. */
+D2IC_API int d2ic_mixed_term_T_batch(const d2ic_frame_t *frame_dev, int n_chunks, const float *u, const float *lam,
+                                     int K, float scale, float *gcoeff, long long coeff_stride, void *stream);
 /* Transpose of d2ic_bspline_prefilter: image-space gradient from a coefficient-space one.
- * tmp: H x cpitch floats. */
+ * tmp: H x cpitch floats; _batch: n_images contiguous images and buffers. */
+D2IC_API int d2ic_bspline_prefilter_T_batch(const float *gcoeff, int n_images, int H, int W, int pad, int cpitch,
+                                            float *tmp, float *gimg, void *stream);
 D2IC_API int d2ic_bspline_prefilter_T(const float *gcoeff, int H, int W, int pad, int cpitch, float *tmp, float *gimg,
                                       void *stream);
 
