@@ -27,11 +27,6 @@ from ._lib import ptr
 from .engine import PAD, FrameLayout, FrameSlot, descriptors_to_device, prepare_coefficients
 
 
-def _pair(a, b):
-    a, b = min(a, b), max(a, b)
-    return a * 4 - (a * (a - 1)) // 2 + (b - a)
-
-
 class ImplicitAdjoint:
     """Linearisation of one converged frame: JVP and VJP with respect to the deformed image."""
 
@@ -48,43 +43,28 @@ class ImplicitAdjoint:
         self.hess = torch.empty(max(L.n_chunks, 1) * 32, dtype=torch.float32, device=self.dev)
         _lib.call("d2ic_hessian_chunks", ptr(self.desc), L.n_chunks, ptr(self.u), int(exact), ptr(self.hess),
                   _lib.stream_handle(stream))
-        self._precond()
+        self._prepare(stream)
+        self._pcg_work = None
         self._slots_cap = 0
         self._slots = None
 
-    # -- preconditioner: inverse 2x2 diagonal blocks, inactive dofs masked -------------------------------
-    def _precond(self):
+    # -- the node operator and its preconditioner: inverse 2x2 diagonal blocks, inactive dofs masked --------
+    def _prepare(self, stream):
         L = self.L
-        h = self.hess.cpu().numpy().reshape(-1, 32)[: L.n_chunks]
-        cn = L.chunk_nodes.cpu().numpy().reshape(-1, 4)
-        D = np.zeros((L.n_nodes, 3))
-        for a in range(4):
-            k = 3 * _pair(a, a)
-            np.add.at(D, cn[:, a], h[:, k:k + 3] * self.inv_np)
-        nbi = L.nbr_index.cpu().numpy().reshape(L.max_deg, L.n_nodes) if L.max_deg else np.zeros((0, L.n_nodes), int)
-        nbw = L.nbr_weight.cpu().numpy().reshape(L.max_deg, L.n_nodes) if L.max_deg else np.zeros((0, L.n_nodes))
-        spring = np.where(nbi >= 0, nbw, 0.0).sum(axis=0)
-        D[:, 0] += self.alpha * spring
-        D[:, 2] += self.alpha * spring
-        det = D[:, 0] * D[:, 2] - D[:, 1] ** 2
-        active = (np.abs(D).sum(axis=1) > 0) & (det > 0)
-        inv = np.zeros((L.n_nodes, 2, 2))
-        inv[active, 0, 0] = D[active, 2] / det[active]
-        inv[active, 1, 1] = D[active, 0] / det[active]
-        inv[active, 0, 1] = inv[active, 1, 0] = -D[active, 1] / det[active]
-        self.Minv = torch.as_tensor(inv, dtype=torch.float64, device=self.dev).contiguous()
-        self.active = torch.as_tensor(active, device=self.dev)
-        self._active_u8 = self.active.to(torch.uint8).contiguous()
-        self._pcg_work = None
+        nb = int(_lib.load().d2ic_hessian_op_bytes(L.n_nodes, L.node_chunk_k))
+        self._op = torch.empty(nb, dtype=torch.uint8, device=self.dev)
+        self._op_checked = False
+        self.Minv = torch.empty((L.n_nodes, 2, 2), dtype=torch.float64, device=self.dev)
+        self.active = torch.empty(L.n_nodes, dtype=torch.bool, device=self.dev)
+        _lib.call("d2ic_hessian_prepare", ptr(self.desc), L.n_chunks, L.n_nodes, L.node_chunk_k, ptr(self.hess),
+                  self.inv_np, self.alpha, ptr(self._op), nb, ptr(self.Minv), ptr(self.active),
+                  _lib.stream_handle(stream))
 
     def operator(self) -> torch.Tensor:
-        """The Hessian assembled into its node operator (d2ic_hessian_assemble), built once."""
-        if getattr(self, "_op", None) is None:
-            L = self.L
-            nb = int(_lib.load().d2ic_hessian_op_bytes(L.n_nodes, L.node_chunk_k))
-            self._op = torch.empty(nb, dtype=torch.uint8, device=self.dev)
-            _lib.call("d2ic_hessian_assemble", ptr(self.desc), L.n_chunks, L.n_nodes, L.node_chunk_k, ptr(self.hess),
-                      self.inv_np, self.alpha, ptr(self._op), nb, _lib.stream_handle())
+        """The Hessian assembled into its node operator (d2ic_hessian_prepare)."""
+        if not self._op_checked:
+            _lib.call("d2ic_hessian_check", ptr(self._op), self.L.n_nodes, self.L.node_chunk_k, _lib.stream_handle())
+            self._op_checked = True
         return self._op
 
     def apply(self, Vf: torch.Tensor, Y: torch.Tensor):
@@ -117,7 +97,7 @@ class ImplicitAdjoint:
 
     def solve(self, B: torch.Tensor, rtol: float = 1e-7, max_iter: int = 2000):
         """X = H^-1 B column by column: block-Jacobi PCG, up to 64 columns in lock step, run by
-        ``d2ic_pcg_solve`` (double-float vectors, FP32 Hessian matvec, deterministic reductions)."""
+        ``d2ic_pcg_solve_op`` (double-float vectors, FP32 Hessian matvec, deterministic reductions)."""
         import ctypes
         L = self.L
         B = B.to(device=self.dev, dtype=torch.float64).contiguous()
@@ -127,10 +107,9 @@ class ImplicitAdjoint:
             self._pcg_work = torch.empty(nb, dtype=torch.uint8, device=self.dev)
         X = torch.empty_like(B)
         it = ctypes.c_int(0)
-        _lib.call("d2ic_pcg_solve", ptr(self.desc), L.n_chunks, L.n_nodes, L.node_chunk_k, ptr(self.hess),
-                  self.inv_np, self.alpha, ptr(self.Minv), ptr(self._active_u8), ptr(B), ptr(X), K, float(rtol),
-                  int(max_iter), ptr(self._pcg_work), self._pcg_work.numel(), ctypes.addressof(it),
-                  _lib.stream_handle())
+        _lib.call("d2ic_pcg_solve_op", ptr(self._op), L.n_nodes, L.node_chunk_k, ptr(self.Minv), ptr(self.active),
+                  ptr(B), ptr(X), K, float(rtol), int(max_iter), ptr(self._pcg_work), self._pcg_work.numel(),
+                  ctypes.addressof(it), _lib.stream_handle())
         self.last_iters = int(it.value)
         return X
 

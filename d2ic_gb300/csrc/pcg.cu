@@ -140,6 +140,30 @@ __global__ void __launch_bounds__(256) hop_merge(const d2ic_frame_t *__restrict_
     if (overflow && lane == 0) atomicExch(err, 1);
 }
 
+// The block-Jacobi preconditioner: the inverse of each node's diagonal block (FP64, row-major 2x2), zero
+// and inactive where the node has no block or one without a positive determinant.
+__global__ void hop_diagonal(const int *__restrict__ idx, const float4 *__restrict__ blk, int n_nodes,
+                             double *__restrict__ Minv, unsigned char *__restrict__ active) {
+    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= n_nodes) return;
+    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q = 0; q < HOP; ++q) {
+        const int j = __ldg(idx + (size_t)n * HOP + q);
+        if (j < 0) break;
+        if (j == n) {
+            b = __ldg(blk + (size_t)n * HOP + q);
+            break;
+        }
+    }
+    const double xx = b.x, xy = b.y, yy = b.z, det = xx * yy - xy * xy;
+    const bool on = fabs(xx) + fabs(xy) + fabs(yy) > 0.0 && det > 0.0;
+    double *m = Minv + 4 * (size_t)n;
+    m[0] = on ? yy / det : 0.0;
+    m[1] = m[2] = on ? -xy / det : 0.0;
+    m[3] = on ? xx / det : 0.0;
+    active[n] = on;
+}
+
 // one node (warp) x 32 columns (lanes): y = sum_q blk_q v_{idx_q}
 __device__ __forceinline__ void hop_row(const int *__restrict__ idx, const float4 *__restrict__ blk, int n, int K, int k,
                                         const float *__restrict__ V, int lane, float &yx, float &yy) {
@@ -1111,14 +1135,17 @@ extern "C" size_t d2ic_pcg_work_bytes(int n_nodes, int K, int node_chunk_k) {
     return a > b ? a : b;
 }
 
-extern "C" int d2ic_pcg_solve(const d2ic_frame_t *frame_dev, int n_chunks, int n_nodes, int node_chunk_k,
-                              const float *chunk_hess, float inv_np, float alpha_reg, const double *Minv,
-                              const unsigned char *active, const double *B, double *X, int K, double rtol,
-                              int max_iter, void *work, size_t work_bytes, int *iters_out, void *stream) {
-    D2IC_REQUIRE(frame_dev && chunk_hess && Minv && active && B && X && work && K >= 1 && n_nodes >= 1 &&
-                     node_chunk_k >= 1 && max_iter >= 0,
-                 "d2ic_pcg_solve: bad arguments");
+// op: an assembled operator, or null: assembled from chunk_hess into the work buffer first
+static int pcg_solve(const d2ic_frame_t *frame_dev, int n_chunks, int n_nodes, int node_chunk_k,
+                     const float *chunk_hess, float inv_np, float alpha_reg, const void *op, const double *Minv,
+                     const unsigned char *active, const double *B, double *X, int K, double rtol, int max_iter,
+                     void *work, size_t work_bytes, int *iters_out, void *stream) {
     D2IC_REQUIRE(((uintptr_t)work & 255) == 0, "d2ic_pcg_solve: work must be 256-byte aligned");
+    auto get_operator = [&](char *space, cudaStream_t st, HopView *hv) -> int {
+        if (!op) return assemble(frame_dev, n_chunks, n_nodes, node_chunk_k, chunk_hess, inv_np, alpha_reg, space, st, hv);
+        hop_layout(n_nodes, node_chunk_k, (char *)op, hv);
+        return D2IC_OK;
+    };
     const size_t need = d2ic_pcg_work_bytes(n_nodes, K, node_chunk_k);
     D2IC_REQUIRE(work_bytes >= need, "d2ic_pcg_solve: work %zu bytes < %zu needed", work_bytes, need);
     cudaStream_t s = (cudaStream_t)stream;
@@ -1134,7 +1161,7 @@ extern "C" int d2ic_pcg_solve(const d2ic_frame_t *frame_dev, int n_chunks, int n
     if (plan.cols > 0 && coop && (size_t)PR_BYTES + sizeof(PrShared) <= (size_t)smem) {
         PrWork r;
         pr_carve(n_nodes, K, node_chunk_k, (char *)work, &r);
-        int st = assemble(frame_dev, n_chunks, n_nodes, node_chunk_k, chunk_hess, inv_np, alpha_reg, r.op, s, &hv);
+        int st = get_operator(r.op, s, &hv);
         if (st) return st;
         pcg_blocks_df<<<(unsigned)((4 * (size_t)n_nodes + 255) / 256), 256, 0, s>>>(Minv, 4 * n_nodes, r.M);
         D2IC_CHECK_LAUNCH("pcg_blocks_df");
@@ -1193,7 +1220,7 @@ extern "C" int d2ic_pcg_solve(const d2ic_frame_t *frame_dev, int n_chunks, int n
     }
     PcgWork w;
     carve(n_nodes, K, node_chunk_k, (char *)work, &w);
-    int st = assemble(frame_dev, n_chunks, n_nodes, node_chunk_k, chunk_hess, inv_np, alpha_reg, w.op, s, &hv);
+    int st = get_operator(w.op, s, &hv);
     if (st) return st;
     cudaError_t e = cudaMemsetAsync(w.ctl, 0, sizeof(PcgCtl), s);
     if (e != cudaSuccess) return cuda_status(e, "pcg control");
@@ -1237,4 +1264,48 @@ extern "C" int d2ic_pcg_solve(const d2ic_frame_t *frame_dev, int n_chunks, int n
     }
     if (iters_out) *iters_out = host_ctl.iters;
     return D2IC_OK;
+}
+
+extern "C" int d2ic_pcg_solve(const d2ic_frame_t *frame_dev, int n_chunks, int n_nodes, int node_chunk_k,
+                              const float *chunk_hess, float inv_np, float alpha_reg, const double *Minv,
+                              const unsigned char *active, const double *B, double *X, int K, double rtol,
+                              int max_iter, void *work, size_t work_bytes, int *iters_out, void *stream) {
+    D2IC_REQUIRE(frame_dev && chunk_hess && Minv && active && B && X && work && K >= 1 && n_nodes >= 1 &&
+                     node_chunk_k >= 1 && max_iter >= 0,
+                 "d2ic_pcg_solve: bad arguments");
+    return pcg_solve(frame_dev, n_chunks, n_nodes, node_chunk_k, chunk_hess, inv_np, alpha_reg, nullptr, Minv, active, B,
+                     X, K, rtol, max_iter, work, work_bytes, iters_out, stream);
+}
+
+extern "C" int d2ic_pcg_solve_op(const void *op, int n_nodes, int node_chunk_k, const double *Minv,
+                                 const unsigned char *active, const double *B, double *X, int K, double rtol,
+                                 int max_iter, void *work, size_t work_bytes, int *iters_out, void *stream) {
+    D2IC_REQUIRE(op && Minv && active && B && X && work && K >= 1 && n_nodes >= 1 && node_chunk_k >= 1 && max_iter >= 0,
+                 "d2ic_pcg_solve_op: bad arguments");
+    return pcg_solve(nullptr, 0, n_nodes, node_chunk_k, nullptr, 0.f, 0.f, op, Minv, active, B, X, K, rtol, max_iter, work,
+                     work_bytes, iters_out, stream);
+}
+
+extern "C" int d2ic_hessian_prepare(const d2ic_frame_t *frame_dev, int n_chunks, int n_nodes, int node_chunk_k,
+                                    const float *chunk_hess, float inv_np, float alpha_reg, void *op, size_t op_bytes,
+                                    double *Minv, unsigned char *active, void *stream) {
+    D2IC_REQUIRE(frame_dev && op && Minv && active && (chunk_hess || n_chunks == 0) && n_nodes >= 1 && node_chunk_k >= 1 &&
+                     n_chunks >= 0,
+                 "d2ic_hessian_prepare: bad arguments");
+    D2IC_REQUIRE(((uintptr_t)op & 255) == 0, "d2ic_hessian_prepare: op must be 256-byte aligned");
+    D2IC_REQUIRE(op_bytes >= d2ic_hessian_op_bytes(n_nodes, node_chunk_k), "d2ic_hessian_prepare: op buffer too small");
+    cudaStream_t s = (cudaStream_t)stream;
+    HopView hv;
+    int st = assemble(frame_dev, n_chunks, n_nodes, node_chunk_k, chunk_hess, inv_np, alpha_reg, (char *)op, s, &hv);
+    if (st) return st;
+    hop_diagonal<<<(n_nodes + 127) / 128, 128, 0, s>>>(hv.idx, hv.blk, n_nodes, Minv, active);
+    D2IC_CHECK_LAUNCH("hop_diagonal");
+    return D2IC_OK;
+}
+
+extern "C" int d2ic_hessian_check(const void *op, int n_nodes, int node_chunk_k, void *stream) {
+    D2IC_REQUIRE(op && n_nodes >= 1 && node_chunk_k >= 1, "d2ic_hessian_check: bad arguments");
+    HopView hv;
+    hop_layout(n_nodes, node_chunk_k, (char *)op, &hv);
+    return check_overflow(hv, (cudaStream_t)stream);
 }

@@ -391,6 +391,18 @@ D2IC_API size_t d2ic_hessian_op_bytes(int n_nodes, int node_chunk_k);
 D2IC_API int d2ic_hessian_assemble(const d2ic_frame_t *frame_dev, int n_chunks, int n_nodes, int node_chunk_k,
                                    const float *chunk_hess, float inv_np, float alpha_reg, void *op, size_t op_bytes,
                                    void *stream);
+/* Assembly and block-Jacobi preconditioner without waiting: the operator into op, the inverse 2x2
+ * diagonal blocks into Minv (n_nodes, 2, 2; zero for inactive nodes) and the mask of active nodes.  An
+ * operator that does not fit (a node couples to more than D2IC_HOP_MAX nodes) is reported by
+ * d2ic_hessian_check, which waits for the stream, and by d2ic_pcg_solve_op. */
+D2IC_API int d2ic_hessian_prepare(const d2ic_frame_t *frame_dev, int n_chunks, int n_nodes, int node_chunk_k,
+                                  const float *chunk_hess, float inv_np, float alpha_reg, void *op, size_t op_bytes,
+                                  double *Minv, unsigned char *active, void *stream);
+D2IC_API int d2ic_hessian_check(const void *op, int n_nodes, int node_chunk_k, void *stream);
+/* d2ic_pcg_solve with an operator assembled before. */
+D2IC_API int d2ic_pcg_solve_op(const void *op, int n_nodes, int node_chunk_k, const double *Minv,
+                               const unsigned char *active, const double *B, double *X, int K, double rtol,
+                               int max_iter, void *work, size_t work_bytes, int *iters_out, void *stream);
 /* Y = H V with the assembled operator, V and Y (n_nodes, 2, K), K fastest: one coalesced row of V per
  * neighbour and 32 columns, no scratch. */
 D2IC_API int d2ic_hessian_apply(const void *op, int n_nodes, int node_chunk_k, const float *V, int K, float *Y,

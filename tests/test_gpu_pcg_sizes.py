@@ -90,3 +90,30 @@ def test_iteration_limit(cuda):
     assert not adj.solve(B, max_iter=0).any() and adj.last_iters == 0
     adj.solve(B, rtol=0.0, max_iter=5)
     assert adj.last_iters == 5
+
+
+@pytest.mark.parametrize("side,element", [(60, 16), (205, 13), (260, 32)])
+def test_preconditioner_inverts_the_diagonal_blocks(cuda, side, element):
+    """Minv of every node is the inverse of the 2x2 diagonal block of H (chunk blocks plus springs, summed in
+    FP64 here); nodes of no element are inactive.  The blocks are FP32 sums of at most 16 chunks and 8
+    springs: 24 * 6e-8, times the blocks' condition."""
+    adj = _adjoint(cuda, side, element)
+    L = adj.L
+    h = adj.hess.cpu().numpy().reshape(-1, 32)[: L.n_chunks].astype(np.float64)
+    cn = L.chunk_nodes.cpu().numpy()
+    D = np.zeros((L.n_nodes, 2, 2))
+    for a in range(4):
+        p = 3 * (a * 4 - (a * (a - 1)) // 2)
+        for (i, j), q in (((0, 0), 0), ((0, 1), 1), ((1, 0), 1), ((1, 1), 2)):
+            np.add.at(D[:, i, j], cn[:, a], h[:, p + q] * adj.inv_np)
+    w = np.where(L.nbr_index.cpu().numpy() >= 0, L.nbr_weight.cpu().numpy(), 0.0).astype(np.float64).sum(axis=0)
+    D[:, 0, 0] += adj.alpha * w
+    D[:, 1, 1] += adj.alpha * w
+    active = adj.active.cpu().numpy()
+    used = np.zeros(L.n_nodes, bool)
+    used[cn.ravel()] = True
+    assert np.array_equal(active, used | (w > 0))
+    M = adj.Minv.cpu().numpy()
+    assert not M[~active].any()
+    cond = np.linalg.cond(D[active]).max()
+    assert np.abs(M[active] @ D[active] - np.eye(2)).max() <= 24 * 6e-8 * cond * 4
