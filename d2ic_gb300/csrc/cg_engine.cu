@@ -33,7 +33,7 @@
 // it took 17.9 us on a 512 x 512 frame with 16-px elements, 23.5 us at
 // 1024 x 1024 and 41.1 us at 2048 x 2048; with tagged records, rolled and
 // smaller once-per-round code and even shares of the chunks 11.6, 14.0 and
-// 31.4 us.  What bounds it now: the L2 round trips of the hand-overs (about
+// 31.4 us, and with the pixel pass below 9.9, 13.9 and 27.0 us.  What bounds it now: the L2 round trips of the hand-overs (about
 // 0.7 us each), the fences that order the node data (0.4 us each) and, from
 // 2048 x 2048 on, the pixel pass.
 //
@@ -389,24 +389,34 @@ __device__ __forceinline__ int checked_index(int v, int n, CtlHeader *H) {
 }
 
 // ---------------------------------------------------------------------------
-// P phase: one chunk per warp, software-pipelined
+// P phase: one chunk per warp at a time
 // ---------------------------------------------------------------------------
 // Each warp walks its chunks (a contiguous range for one frame, c, c + W,
-// c + 2W, ... for W warps in the grid with several) with three stages in flight:
-//   chunk i + 2: metadata (pixel range, nodes, slots) loaded into registers;
+// c + 2W, ... for W warps in the grid with several) in batches of 32, one chunk
+// per lane.  What a chunk needs besides its pixels is done for the batch at once,
+// by the chunk's lane and with all loads in flight together: its metadata (pixel
+// range, nodes, slots, tile origin), the nodal candidates (u + alpha dir at its
+// four nodes), whether its stencils all lie inside its tile, and the tile origin
+// of the next pass.  The warp then takes the chunks one by one:
 //   chunk i + 1: pixel records copied into the warp's shared-memory buffer by
 //                one TMA bulk copy (cp.async.bulk, completion on an mbarrier),
-//                nodal candidate inputs (u, g, d) copied by cp.async onto the
-//                same mbarrier;
-//   chunk i:     sampled and reduced.
-// A warp therefore never waits on a metadata -> records / candidates round
-// trip.
-// Each chunk also stages its window of the deformed image's coefficients
-// (tile_w x tile_h floats) with a 2-D TMA copy on the same mbarrier.  The
-// window is placed from the chunk's candidate of the previous pass, with a
+//                and its window of the deformed image's coefficients (tile_w x
+//                tile_h floats) by a 2-D TMA copy on the same mbarrier, both
+//                issued by the chunk's lane;
+//   chunk i:     values broadcast from its lane, sampled and reduced.
+// The window is placed from the chunk's candidate of the previous pass, with a
 // margin of TILE_MARGIN pixels on every side (stored per chunk in
 // chunk_tile); a pixel whose 4x4 stencil is not inside it (a larger move, the
 // first pass) reads global memory with the same arithmetic.
+//
+// With the per-chunk work done by the whole warp and scalar pixel arithmetic a
+// 256-pixel chunk took about 2,000 issue slots, 650 of them besides the pixels, and
+// the pass ran at 92 % of the issue rate.  Lane batches and two pixels per
+// instruction leave about 1,150: per evaluation 31.4 -> 27.0 us at 2048 x 2048 with
+// 16-px elements, 62.7 -> 40.3 us with 8-px elements, 219 -> 149 us at 4096 x 4096
+// with 8-px elements.  A pass without the coefficient tiles' traffic takes 0.5 us
+// less at 2048 x 2048: what bounds it now is the FMA pipe (60 % busy during the pass)
+// with 4 warps per scheduler to hide its latencies, not the L2.
 constexpr int CHUNK_BYTES = D2IC_CHUNK_MAX * 16;            // one staged record buffer
 constexpr int TILE_BYTES = D2IC_TILE_MAX_FLOATS * 4;        // one staged coefficient tile
 static_assert(TILE_BYTES % 128 == 0, "tile buffers keep 128-byte alignment");
@@ -414,8 +424,7 @@ constexpr int WARP_SMEM = 2 * CHUNK_BYTES + 2 * TILE_BYTES;
 constexpr int TILE_MARGIN = 2;
 constexpr int TILE_NONE = (int)0x80008000u;                 // no valid origin (col = row = -32768)
 constexpr unsigned long long TMA_WAIT_NS = 200ull * 1000ull * 1000ull;
-constexpr int FCACHE = 64;
-constexpr int CAND_N = 12;    // candidate copies per staged chunk (lanes 0..11)    // active frames whose per-round lookup data is kept in shared memory
+constexpr int FCACHE = 64;    // active frames whose per-round lookup data is kept in shared memory
 
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 
@@ -440,17 +449,6 @@ __device__ __forceinline__ void tensor_load_2d(void *dst, const void *map, int x
         "l"(map), "r"(x), "r"(y), "r"(smem_addr(b))
         : "memory");
 }
-// 8-byte asynchronous copy global -> shared (no register holds the value); the mbarrier's
-// pending count is decremented when this thread's earlier cp.async copies have completed
-__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_arrive(unsigned long long *b) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(b)) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(unsigned long long *b) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(b)) : "memory");
-}
 __device__ __forceinline__ bool mbar_test(unsigned long long *b, unsigned parity) {
     unsigned ok;
     asm volatile(
@@ -469,37 +467,42 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity
     return true;
 }
 
-// One chunk's metadata as the pipeline carries it.  nd / slot hold local node
-// (lane) a's index and slot rank in lanes 0..3.
+// A chunk as its lane holds it from the load to the candidates.
 struct ChunkMeta {
-    int s, f, c, pb, pe, nd, slot;   // active slot, frame, chunk within the frame, ...
-    int box0, box1, tile;            // packed pixel-box corners and tile origin (col | row << 16)
+    int f, c, pb, n;                 // frame, chunk within the frame, first pixel, pixels
+    int box0, box1;                  // packed pixel-box corners
+    int origin, flags;               // packed tile origin (TMA column, row), CH_* bits
+    int4 nd;                         // nodes
+    unsigned slot;                   // slot rank of node a in byte a
 };
+enum { CH_STAGED = 1, CH_TILED = 2, CH_FAST = 4 };   // records / tile in shared memory; no pixel leaves the tile
 
-__device__ __forceinline__ ChunkMeta load_meta(const d2ic_frame_t &F, int f, int c, int lane) {
+// Lane's chunk c of frame f.  chunk_tile is rewritten every pass: read from L2.
+template <int KIND>
+__device__ __forceinline__ ChunkMeta load_meta(const d2ic_frame_t &F, int f, int c, bool tiles_ok) {
     ChunkMeta m;
-    m.s = 0;
     m.f = f;
     m.c = c;
     m.pb = __ldg(F.chunk_begin + c);
-    m.pe = __ldg(F.chunk_begin + c + 1);
+    m.n = max(__ldg(F.chunk_begin + c + 1) - m.pb, 0);
     m.box0 = __ldg(F.chunk_box + 2 * c);
     m.box1 = __ldg(F.chunk_box + 2 * c + 1);
-    m.tile = F.tile_w > 0 ? __ldcg(F.chunk_tile + c) : TILE_NONE;   // rewritten every pass: L2
-    m.nd = 0;
-    m.slot = 0;
-    if (lane < 4) {
-        m.nd = __ldg(F.chunk_nodes + 4 * c + lane);
-        m.slot = (int)(((unsigned)__ldg(F.chunk_slot + c) >> (8 * lane)) & 0xffu);
+    m.nd = make_int4(__ldg(F.chunk_nodes + 4 * c), __ldg(F.chunk_nodes + 4 * c + 1), __ldg(F.chunk_nodes + 4 * c + 2),
+                     __ldg(F.chunk_nodes + 4 * c + 3));
+    m.slot = (unsigned)__ldg(F.chunk_slot + c);
+    m.flags = m.n > 0 && ((reinterpret_cast<uintptr_t>(F.pix) & 15) == 0) ? CH_STAGED : 0;
+    m.origin = 0;
+    if (KIND == D2IC_INTERP_CUBIC && tiles_ok && F.tile_w > 0) {
+        const int tile = __ldcg(F.chunk_tile + c);
+        const int tx0 = (int)(short)(tile & 0xffff) & ~3;            // TMA x: a multiple of 4 floats
+        const int ty0 = (int)(short)((unsigned)tile >> 16);
+        m.origin = (tx0 & 0xffff) | (int)((unsigned)ty0 << 16);
+        if (tile != TILE_NONE && tx0 >= -F.pad && ty0 >= -F.pad && tx0 + F.tile_w <= F.W + F.pad &&
+            ty0 + F.tile_h <= F.H + F.pad)                           // inside the halo'd array: no fill
+            m.flags |= CH_TILED;
     }
     return m;
 }
-
-// Where a chunk's records and coefficient tile come from in this pass.
-struct Stage {
-    bool staged, tiled;   // records in shared memory; coefficient tile in shared memory
-    int tx0, ty0;         // tile origin (pixel column / row of tile element (0, 0))
-};
 
 // Tile origin for the next pass from this pass's nodal candidates: the
 // smallest tap column / row any pixel of the chunk can reach, less the margin.
@@ -518,83 +521,114 @@ __device__ __forceinline__ int atom_acq_rel_add(int *p, int v) {
     return old;
 }
 
+// Whole chunk inside its tile: a pixel's displacement is a convex combination of its
+// element's nodal candidates, so its stencil corner lies in the chunk's pixel box shifted by
+// [floor(min u), floor(max u)] (taken with 0.5 px of slack).  Then no pixel needs the
+// per-pixel test or the global-memory path.
+__device__ __forceinline__ bool inside_tile(const d2ic_frame_t &F, const ChunkMeta &m, const float ux[4], const float uy[4]) {
+    bool fin = true;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) fin = fin && isfinite(ux[a]) && isfinite(uy[a]);
+    if (!fin) return false;
+    const float mnx = fminf(fminf(ux[0], ux[1]), fminf(ux[2], ux[3]));
+    const float mxx = fmaxf(fmaxf(ux[0], ux[1]), fmaxf(ux[2], ux[3]));
+    const float mny = fminf(fminf(uy[0], uy[1]), fminf(uy[2], uy[3]));
+    const float mxy = fmaxf(fmaxf(uy[0], uy[1]), fmaxf(uy[2], uy[3]));
+    const int tx0 = (int)(short)(m.origin & 0xffff), ty0 = (int)(short)((unsigned)m.origin >> 16);
+    const int lx0 = (m.box0 & 0xffff) + (int)safe_floor(mnx - 0.5f) - 1 - tx0;
+    const int lx1 = (m.box1 & 0xffff) + (int)safe_floor(mxx + 0.5f) - 1 - tx0;
+    const int ly0 = (int)((unsigned)m.box0 >> 16) + (int)safe_floor(mny - 0.5f) - 1 - ty0;
+    const int ly1 = (int)((unsigned)m.box1 >> 16) + (int)safe_floor(mxy + 0.5f) - 1 - ty0;
+    return lx0 >= 0 && lx1 <= F.tile_w - 4 && ly0 >= 0 && ly1 <= F.tile_h - 4;
+}
+
+// What the chunk's lane keeps for the pixel loop
+struct ChunkWork {
+    int f, pb, n, origin;
+    unsigned flags;              // CH_* bits; bits 4 + 4a ..: low bits of node a's record (see gather_slots)
+    unsigned tag;                // the evaluation's tag
+    float ux[4], uy[4];          // nodal candidates
+    int rec[4];                  // node a's record among the frame's slots
+};
+
+// The sum over the warp of values v >= 0 (or NaN): the values as 54-bit fixed-point numbers relative to
+// the largest, summed by integer warp reductions (a double-float butterfly takes five dependent steps of
+// two shuffles and an 11-operation sum).  Error: 2^-47 of the sum.
+__device__ __forceinline__ DF warp_sum_nonneg(float v) {
+    const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(v)), e = m >> 23;
+    if (e < 27u || e >= 255u) return df_warp_sum(DF{v, 0.f});          // tiny, infinite or NaN: the same for all lanes
+    const float q = v * __uint_as_float((280u - e) << 23);             // < 2^27
+    const unsigned hi = (unsigned)q;
+    const unsigned lo = (unsigned)((q - (float)hi) * 134217728.f);     // 27 more bits
+    unsigned sh = __reduce_add_sync(0xffffffffu, hi);
+    const unsigned sl = __reduce_add_sync(0xffffffffu, lo);
+    sh += sl >> 27;
+    const float h = __uint2float_rz(sh);
+    const float l = __fmaf_rn((float)(sl & 0x7ffffffu), 7.450580596923828125e-9f, (float)(sh - (unsigned)h));
+    const float back = __uint_as_float((e - 26u) << 23);
+    return {h * back, l * back};
+}
+
+// One chunk by the whole warp, its values broadcast from lane `src`.
 template <int KIND>
-__device__ __forceinline__ void chunk_compute(const d2ic_frame_t &F, const ChunkMeta &m, float2 uc, const Stage &st,
-                                              const uint4 *srec, const float *tile, int lane,
-                                              const unsigned *tag_at) {
-    const bool staged = st.staged;
-    const bool tiled = KIND == D2IC_INTERP_CUBIC && st.tiled;
-    const int tw = F.tile_w, th = F.tile_h, tx0 = st.tx0, ty0 = st.ty0;
-    const int n = max(m.pe - m.pb, 0);
-    const uint4 *gpix = reinterpret_cast<const uint4 *>(F.pix) + m.pb;
+__device__ __forceinline__ void chunk_compute(const d2ic_frame_t &F, const ChunkWork &w, int src, const uint4 *srec,
+                                              const float *tile, int lane) {
+    const unsigned flags = __shfl_sync(0xffffffffu, w.flags, src);
+    const int origin = __shfl_sync(0xffffffffu, w.origin, src);
+    const int n = __shfl_sync(0xffffffffu, w.n, src);
+    const bool staged = (flags & CH_STAGED) != 0;
+    const bool tiled = KIND == D2IC_INTERP_CUBIC && (flags & CH_TILED) != 0;
+    const bool fast = KIND == D2IC_INTERP_CUBIC && (flags & CH_FAST) != 0;
+    const int tw = F.tile_w, th = F.tile_h;
+    const int tx0 = (int)(short)(origin & 0xffff), ty0 = (int)(short)((unsigned)origin >> 16);
     float ux[4], uy[4];
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-        ux[a] = __shfl_sync(0xffffffffu, uc.x, a);
-        uy[a] = __shfl_sync(0xffffffffu, uc.y, a);
-    }
-    const Img im{F.coeff, F.W, F.H, F.cpitch, F.pad};
-    // Whole chunk inside the tile: a pixel's displacement is a convex combination of its
-    // element's nodal candidates, so its stencil corner lies in the chunk's pixel box shifted by
-    // [floor(min u), floor(max u)] (taken with 0.5 px of slack).  Then no pixel needs the
-    // per-pixel test or the global-memory path.
-    bool fast = false;
-    if (tiled && staged && n <= D2IC_CHUNK_MAX) {
-        bool fin = true;
-#pragma unroll
-        for (int a = 0; a < 4; ++a) fin = fin && isfinite(ux[a]) && isfinite(uy[a]);
-        if (fin) {
-            const float mnx = fminf(fminf(ux[0], ux[1]), fminf(ux[2], ux[3]));
-            const float mxx = fmaxf(fmaxf(ux[0], ux[1]), fmaxf(ux[2], ux[3]));
-            const float mny = fminf(fminf(uy[0], uy[1]), fminf(uy[2], uy[3]));
-            const float mxy = fmaxf(fmaxf(uy[0], uy[1]), fmaxf(uy[2], uy[3]));
-            const int lx0 = (m.box0 & 0xffff) + (int)safe_floor(mnx - 0.5f) - 1 - tx0;
-            const int lx1 = (m.box1 & 0xffff) + (int)safe_floor(mxx + 0.5f) - 1 - tx0;
-            const int ly0 = (int)((unsigned)m.box0 >> 16) + (int)safe_floor(mny - 0.5f) - 1 - ty0;
-            const int ly1 = (int)((unsigned)m.box1 >> 16) + (int)safe_floor(mxy + 0.5f) - 1 - ty0;
-            fast = lx0 >= 0 && lx1 <= tw - 4 && ly0 >= 0 && ly1 <= th - 4;
-        }
+        ux[a] = __shfl_sync(0xffffffffu, w.ux[a], src);
+        uy[a] = __shfl_sync(0xffffffffu, w.uy[a], src);
     }
     float jr = 0.f;
     float gxa[4] = {0.f, 0.f, 0.f, 0.f}, gya[4] = {0.f, 0.f, 0.f, 0.f};
-    // fast path: the stencil corner is clamped into the tile only as a guard of the shared-memory
-    // bounds (it is already inside)
-    auto one_fast = [&](const uint4 r4) {
-        const int x = (int)(r4.x & 0xffffu), y = (int)(r4.x >> 16);
-        const float I1 = __uint_as_float(r4.y), xi = __uint_as_float(r4.z), eta = __uint_as_float(r4.w);
-        const float a0 = 0.5f * (1.f - xi), a1 = 0.5f * (1.f + xi);
-        const float b0 = 0.5f * (1.f - eta), b1 = 0.5f * (1.f + eta);
-        const float N[4] = {a0 * b0, a1 * b0, a1 * b1, a0 * b1};
-        const float dx = N[0] * ux[0] + N[1] * ux[1] + N[2] * ux[2] + N[3] * ux[3];
-        const float dy = N[0] * uy[0] + N[1] * uy[1] + N[2] * uy[2] + N[3] * uy[3];
-        int ix, iy;
-        float tx, ty;
-        split_coord(x, dx, ix, tx);
-        split_coord(y, dy, iy, ty);
-        float gx, gy;
-        const int lx = min(max(ix - 1 - tx0, 0), tw - 4), ly = min(max(iy - 1 - ty0, 0), th - 4);
-        const float v = sample_cubic_tile(tile, tw, lx, ly, tx, ty, gx, gy);
-        const float r = v - I1;
-        jr += r * r;
-        const float rgx = r * gx, rgy = r * gy;
+    // fast path, two pixels per lane and step (p and p + 32): the arithmetic of `one`, in packed operations
+    // (174 instead of about 330 issue slots per step; one pixel per lane and instruction: 2 us more per
+    // evaluation at 2048 x 2048).
+    // floor(d) is d + 1.5 * 2^23 rounded down, less 1.5 * 2^23 (exact: here |d| < 2^16), whose low bits are the
+    // integer for the tap index; the index is limited to the tile only as a guard of the shared-memory
+    // bounds (it is already inside).
+    auto two_fast = [&](int p, const Pair ux2[4], const Pair uy2[4], unsigned corner, unsigned limit) {
+        const uint4 ra = srec[min(p, n - 1)], rb = srec[min(p + 32, n - 1)];
+        constexpr float MAGIC = 12582912.f;
+        Pair N[4];
+        shape4(pair(__uint_as_float(ra.z), __uint_as_float(rb.z)), pair(__uint_as_float(ra.w), __uint_as_float(rb.w)), N);
+        const Pair dx = dot4(N, ux2), dy = dot4(N, uy2);
+        const Pair mx = pair_add_down(dx, pair(MAGIC)), my = pair_add_down(dy, pair(MAGIC));
+        const Pair tx = pair_add(dx, pair_fma(mx, pair(-1.f), pair(MAGIC)));
+        const Pair ty = pair_add(dy, pair_fma(my, pair(-1.f), pair(MAGIC)));
+        const unsigned ia = ((ra.x >> 16) + (unsigned)my) * (unsigned)tw + (ra.x & 0xffffu) + (unsigned)mx + corner;
+        const unsigned ib = ((rb.x >> 16) + (unsigned)(my >> 32)) * (unsigned)tw + (rb.x & 0xffffu) + (unsigned)(mx >> 32) + corner;
+        Pair gx, gy;
+        const Pair v = sample_cubic_tile2(tile, tw, min(ia, limit), min(ib, limit), tx, ty, gx, gy);
+        Pair r = pair_fma(pair(__uint_as_float(ra.y), __uint_as_float(rb.y)), pair(-1.f), v);
+        r = pair(p < n ? pair_lo(r) : 0.f, p + 32 < n ? pair_hi(r) : 0.f);
+        jr = __fmaf_rn(pair_lo(r), pair_lo(r), jr);
+        jr = __fmaf_rn(pair_hi(r), pair_hi(r), jr);
+        const Pair rgx = pair_mul(r, gx), rgy = pair_mul(r, gy);
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
-            gxa[a] += rgx * N[a];
-            gya[a] += rgy * N[a];
+            gxa[a] = __fmaf_rn(pair_hi(rgx), pair_hi(N[a]), __fmaf_rn(pair_lo(rgx), pair_lo(N[a]), gxa[a]));
+            gya[a] = __fmaf_rn(pair_hi(rgy), pair_hi(N[a]), __fmaf_rn(pair_lo(rgy), pair_lo(N[a]), gya[a]));
         }
     };
-    auto one = [&](const uint4 r4) {
+    auto one = [&](const Img &im, const uint4 r4) {
+
         const int x = (int)(r4.x & 0xffffu), y = (int)(r4.x >> 16);
-        const float I1 = __uint_as_float(r4.y), xi = __uint_as_float(r4.z), eta = __uint_as_float(r4.w);
-        const float a0 = 0.5f * (1.f - xi), a1 = 0.5f * (1.f + xi);
-        const float b0 = 0.5f * (1.f - eta), b1 = 0.5f * (1.f + eta);
-        const float N[4] = {a0 * b0, a1 * b0, a1 * b1, a0 * b1};
-        const float dx = N[0] * ux[0] + N[1] * ux[1] + N[2] * ux[2] + N[3] * ux[3];
-        const float dy = N[0] * uy[0] + N[1] * uy[1] + N[2] * uy[2] + N[3] * uy[3];
+        const float I1 = __uint_as_float(r4.y);
+        float N[4];
+        shape4(__uint_as_float(r4.z), __uint_as_float(r4.w), N);
         int ix, iy;
         float tx, ty;
-        split_coord(x, dx, ix, tx);
-        split_coord(y, dy, iy, ty);
+        split_coord(x, dot4(N, ux), ix, tx);
+        split_coord(y, dot4(N, uy), iy, ty);
         float gx, gy, v;
         const int lx = ix - 1 - tx0, ly = iy - 1 - ty0;   // stencil corner inside the tile
         if (tiled && (unsigned)lx <= (unsigned)(tw - 4) && (unsigned)ly <= (unsigned)(th - 4))
@@ -602,27 +636,35 @@ __device__ __forceinline__ void chunk_compute(const d2ic_frame_t &F, const Chunk
         else
             v = sample<KIND>(im, ix, iy, tx, ty, gx, gy);
         const float r = v - I1;
-        jr += r * r;
+        jr = __fmaf_rn(r, r, jr);
         const float rgx = r * gx, rgy = r * gy;
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
-            gxa[a] += rgx * N[a];
-            gya[a] += rgy * N[a];
+            gxa[a] = __fmaf_rn(rgx, N[a], gxa[a]);
+            gya[a] = __fmaf_rn(rgy, N[a], gya[a]);
         }
     };
     if (fast) {
-#pragma unroll 4
-        for (int i = 0; i < D2IC_CHUNK_MAX / 32; ++i) {
-            const int p = lane + 32 * i;
-            if (p < n) one_fast(srec[p]);
+        Pair ux2[4], uy2[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            ux2[a] = pair(ux[a]);
+            uy2[a] = pair(uy[a]);
         }
+        // a pixel's tap index: (y + floor(dy) - 1 - ty0) tw + (x + floor(dx) - 1 - tx0), modulo 2^32
+        const unsigned corner = 0u - (0x4b400000u + 1u + (unsigned)ty0) * (unsigned)tw - (0x4b400000u + 1u + (unsigned)tx0);
+        const unsigned limit = (unsigned)((th - 4) * tw + tw - 4);
+#pragma unroll 1
+        for (int p = lane; p - lane < n; p += 64) two_fast(p, ux2, uy2, corner, limit);
     } else {
         // boundary chunks and the first pass: one copy of the general per-pixel code (this loop's body
         // is several times the fast one's; the instruction cache matters more here than its speed)
+        const Img im{F.coeff, F.W, F.H, F.cpitch, F.pad};
+        const uint4 *gpix = reinterpret_cast<const uint4 *>(F.pix) + __shfl_sync(0xffffffffu, w.pb, src);
 #pragma unroll 1
-        for (int p = lane; p < n; p += 32) one(staged && p < D2IC_CHUNK_MAX ? srec[p] : __ldg(gpix + p));
+        for (int p = lane; p < n; p += 32) one(im, staged && p < D2IC_CHUNK_MAX ? srec[p] : __ldg(gpix + p));
     }
-    const DF js = df_warp_sum(DF{jr, 0.f});
+    const DF js = warp_sum_nonneg(jr);
     // The 8 nodal partials summed over the warp by a reduce-scatter butterfly: at each of the
     // steps over lane bits 4, 3, 2 a lane keeps half of its values and adds its partner's copy of
     // that half (7 shuffles instead of 40); bits 1, 0 finish the sums.  Value k = (gx_0..3,
@@ -660,27 +702,21 @@ __device__ __forceinline__ void chunk_compute(const d2ic_frame_t &F, const Chunk
     const int la = lane & 3;
     const float gxs = __shfl_sync(0xffffffffu, v1, 8 * ((la >> 1) & 1) + 4 * (la & 1));
     const float gys = __shfl_sync(0xffffffffu, v1, 16 + 8 * ((la >> 1) & 1) + 4 * (la & 1));
-    if (lane == 0 && tw > 0) F.chunk_tile[m.c] = tile_origin(m.box0, ux, uy);
     // Lane a stores node a's partial in the chunk's slot of that node as one tagged record; the slots
     // of nodes 0 and 1 also carry the two words of the chunk's sum of r^2, so every chunk is counted
-    // exactly once.  The last word holds the evaluation's tag and, for the waiting group (see
-    // gather_slots), whether this is the chunk's first node in its group and how many it has there.
-    {
-        const int grp = m.nd / GN;
-        int cnt = 0;
-        bool first = true;
+    // exactly once.
+    int rec = __shfl_sync(0xffffffffu, w.rec[0], src);
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const bool same = __shfl_sync(0xffffffffu, grp, a) == grp;
-            cnt += same;
-            first = first && !(same && a < lane);
-        }
-        if (lane < 4)
-            st_record(reinterpret_cast<float4 *>(F.node_grad) + (size_t)m.slot * F.n_nodes + m.nd,
-                      make_uint4(__float_as_uint(gxs), __float_as_uint(gys),
-                                 __float_as_uint(lane == 0 ? js.hi : (lane == 1 ? js.lo : 0.f)),
-                                 (*tag_at << 4) | ((unsigned)cnt << 1) | (first ? 1u : 0u)));
+    for (int a = 1; a < 4; ++a) {
+        const int t = __shfl_sync(0xffffffffu, w.rec[a], src);
+        if (lane == a) rec = t;
     }
+    const unsigned tag = __shfl_sync(0xffffffffu, w.tag, src);
+    if (lane < 4)
+        st_record(reinterpret_cast<float4 *>(F.node_grad) + rec,
+                  make_uint4(__float_as_uint(gxs), __float_as_uint(gys),
+                             __float_as_uint(lane == 0 ? js.hi : (lane == 1 ? js.lo : 0.f)),
+                             (tag << 4) | ((flags >> (4 + 4 * lane)) & 15u)));
     __syncwarp();                                   // every lane is done with the staged buffers
 }
 
@@ -1365,9 +1401,6 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                                                    double *J_out, float *grad_out, unsigned long long *trace,
                                                    int trace_rounds, int max_rounds, int stop_flags) {
     __shared__ unsigned long long s_bar[NWARP][2];   // per-warp mbarriers of the two record buffers
-    // per warp and buffer: the nodal candidate inputs of the staged chunk, u of node a at [a], g at
-    // [4 + a], the previous direction at [8 + a] (cp.async, completing on the buffer's mbarrier)
-    __shared__ __align__(16) float2 s_cand[NWARP][2][CAND_N];
     const int n_frames = ONE ? 1 : n_frames_arg;     // ONE: the control block's offsets are constants
     constexpr int FC = ONE ? 1 : FCACHE;
     __shared__ int s_cpre[FC + 1];                   // per-round copies of the active list (na <= FCACHE)
@@ -1377,7 +1410,6 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
     __shared__ __align__(16) unsigned long long s_frame[ONE ? sizeof(d2ic_frame_t) / 8 : 1];   // ONE: the descriptor
     __shared__ FrameState s_state;                   // ONE: the state in the control step (one warp of the grid)
     __shared__ int2 s_range[NWARP];                  // each warp's chunk range (one active frame)
-    __shared__ unsigned s_tag[NWARP];                // the current chunk's tag when the list is not cached
     __shared__ int s_hdr[10];                         // n_active, total_chunks, total_groups, abort, slice stop,
                                                      // what to refresh, rounds completed, list_buf, list version
     __shared__ DF s_gq[NWARP][D2IC_NPART];           // group partials of this block's supergroup
@@ -1389,8 +1421,8 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
     unsigned char *wbuf = s_dyn + (size_t)wid * WARP_SMEM;
     unsigned pipe_i = 0;   // chunks this warp has staged: buffer i & 1, completion parity (i >> 1) & 1
     if (lane == 0) {
-        mbar_init(&s_bar[wid][0], 1 + CAND_N);   // lane 0's expect_tx + one per candidate copy
-        mbar_init(&s_bar[wid][1], 1 + CAND_N);
+        mbar_init(&s_bar[wid][0], 1);            // the issuing lane's expect_tx
+        mbar_init(&s_bar[wid][1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // descriptors (and their tensor maps) may have been rewritten since the previous launch
@@ -1413,13 +1445,11 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
     const bool tr = trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0;
     int round = 0;
     if (threadIdx.x == 0) s_sgcnt = 0;
-    // A warp's first chunk of the next round, staged before the round's release (its records,
-    // coefficient tile and the metadata of the chunk after it do not depend on the control step);
-    // used if the active list is unchanged, else drained.
+    // A warp's first batch of the next round, loaded before the round's release, with its first chunk
+    // staged (neither depends on the control step); used if the active list is unchanged, else drained.
     bool pf = false;
     int pf_na = 0, pf_total = 0;
-    ChunkMeta pf_m0{}, pf_m1{};
-    Stage pf_st0{};
+    ChunkMeta pf_m{};
 
     // ---- init of newly admitted frames: u <- u0, zero g/d buffers and gradient slots, NaN history ----
     for (int f = 0; f < n_frames; ++f) {
@@ -1489,7 +1519,6 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
         // the active list only shrinks within a launch: the same count means the same list
         const bool pf_use = pf && na == pf_na && total == pf_total;
         if (pf && !pf_use) {
-            if (lane < CAND_N) mbar_arrive(&s_bar[wid][pipe_i & 1]);   // no candidates for the dropped chunk
             if (!mbar_wait(&s_bar[wid][pipe_i & 1], (pipe_i >> 1) & 1u) && lane == 0) {   // bounded
                 C.h->err = D2IC_WAIT_TIMEOUT;
                 atomicExch(&C.h->abort, 1);
@@ -1497,78 +1526,45 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
             ++pipe_i;
         }
         pf = false;
-        const ChunkMeta pm0 = pf_m0, pm1 = pf_m1;
-        const Stage pst0 = pf_st0;
-        pf_m0 = ChunkMeta{};   // constants while the round runs (nothing to keep in registers)
-        pf_m1 = ChunkMeta{};
-        pf_st0 = Stage{};
+        const ChunkMeta pm = pf_m;
+        pf_m = ChunkMeta{};    // constants while the round runs (nothing to keep in registers)
         // ---- P phase: chunks of the active list spread over the warps (see below) ----
         {
             const bool cached = ONE || na <= FCACHE;
             const int gw = (int)((blockIdx.x * NT + threadIdx.x) >> 5);
             const int nw = (int)((gridDim.x * NT) >> 5);
-            int cur = 0;   // active slot of the last located chunk (chunks ascend per warp)
-            auto fetch_meta = [&](int g) {
-                int s = 0, f = 0, base = 0;
-                if (ONE) {
-                } else if (cached) {
-                    while (cur + 1 < na && s_cpre[cur + 1] <= g) ++cur;
-                    s = cur;
-                    f = s_act[s];
-                    base = s_cpre[s];
-                } else {
-                    s = find_slot(C.cp(lb), na, g);
-                    f = checked_index(__ldcg(C.act(lb) + s), n_frames, C.h);
-                    base = __ldcg(C.cp(lb) + s);
+            auto slot_of = [&](int g) {
+                return ONE ? 0 : cached ? find_slot_smem(s_cpre, na, g) : find_slot(C.cp(lb), na, g);
+            };
+            // lane's chunk g of the active list (nothing if g >= end)
+            auto fetch_meta = [&](int g, int end) {
+                ChunkMeta m{};
+                if (g < end) {
+                    const int s = slot_of(g);
+                    const int f = ONE ? 0 : cached ? s_act[s] : checked_index(__ldcg(C.act(lb) + s), n_frames, C.h);
+                    const int base = ONE ? 0 : cached ? s_cpre[s] : __ldcg(C.cp(lb) + s);
+                    m = load_meta<KIND>(frame(f), f, checked_index(g - base, frame(f).n_chunks, C.h), tiles_ok);
                 }
-                ChunkMeta m = load_meta(frame(f), f, checked_index(g - base, frame(f).n_chunks, C.h), lane);
-                m.s = s;
                 return m;
             };
-            // stage a chunk: TMA bulk copy of its records, 2-D TMA copy of its coefficient tile
-            auto issue_tma = [&](const ChunkMeta &m, unsigned i) {
-                const d2ic_frame_t &F = frame(m.f);
-                const int n = max(m.pe - m.pb, 0);
-                const unsigned bytes = (unsigned)min(n, D2IC_CHUNK_MAX) * 16u;
-                const uint4 *src = reinterpret_cast<const uint4 *>(F.pix) + m.pb;
-                Stage st;
-                st.staged = bytes > 0 && ((reinterpret_cast<uintptr_t>(src) & 15) == 0);
-                st.tiled = false;
-                st.tx0 = 0;
-                st.ty0 = 0;
-                if (KIND == D2IC_INTERP_CUBIC && tiles_ok && F.tile_w > 0 && m.tile != TILE_NONE) {
-                    st.tx0 = (int)(short)(m.tile & 0xffff) & ~3;   // TMA x: a multiple of 4 floats
-                    st.ty0 = (int)(short)((unsigned)m.tile >> 16);
-                    st.tiled = st.tx0 >= -F.pad && st.ty0 >= -F.pad && st.tx0 + F.tile_w <= F.W + F.pad &&
-                               st.ty0 + F.tile_h <= F.H + F.pad;   // inside the halo'd array: no fill
-                }
-                unsigned long long *bar = &s_bar[wid][i & 1];
-                if (lane == 0) {
+            // stage the chunk of lane `src` in buffer i & 1: TMA bulk copy of its records, 2-D TMA copy of its tile
+            auto stage = [&](int src, int f, int pb, int n, int flags, int origin, unsigned i) {
+                if (lane == src) {
+                    const d2ic_frame_t &F = frame(f);
+                    unsigned long long *bar = &s_bar[wid][i & 1];
+                    const unsigned bytes = (flags & CH_STAGED) ? (unsigned)min(n, D2IC_CHUNK_MAX) * 16u : 0u;
+                    const unsigned tbytes = (flags & CH_TILED) ? (unsigned)(F.tile_w * F.tile_h) * 4u : 0u;
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // after the buffers' generic reads
-                    const unsigned tbytes = st.tiled ? (unsigned)(F.tile_w * F.tile_h) * 4u : 0u;
-                    mbar_arrive_tx(bar, (st.staged ? bytes : 0u) + tbytes);
-                    if (st.staged) bulk_load(wbuf + (i & 1) * CHUNK_BYTES, src, bytes, bar);
-                    if (st.tiled)
-                        tensor_load_2d(wbuf + 2 * CHUNK_BYTES + (i & 1) * TILE_BYTES, frames[ONE ? 0 : m.f].coeff_map, st.tx0 + F.pad,
-                                       st.ty0 + F.pad, bar);
+                    mbar_arrive_tx(bar, bytes + tbytes);
+                    if (bytes)
+                        bulk_load(wbuf + (i & 1) * CHUNK_BYTES, reinterpret_cast<const uint4 *>(F.pix) + pb, bytes, bar);
+                    if (tbytes)
+                        tensor_load_2d(wbuf + 2 * CHUNK_BYTES + (i & 1) * TILE_BYTES, frames[ONE ? 0 : f].coeff_map,
+                                       (int)(short)(origin & 0xffff) + F.pad,
+                                       (int)(short)((unsigned)origin >> 16) + F.pad, bar);
                 }
-                return st;
+                __syncwarp();
             };
-            // the chunk's nodal candidate inputs into s_cand (lane 4 k + a copies array k of node a),
-            // counted on the chunk's mbarrier
-            auto load_cand = [&](const ChunkMeta &m, unsigned i) {
-                const int a = lane & 3, k = lane >> 2;
-                const int nd = __shfl_sync(0xffffffffu, m.nd, a);
-                if (lane < CAND_N) {
-                    const d2ic_frame_t &F = frame(m.f);
-                    const FInfo fi = cached ? s_fi[m.s].info() : frame_info(C.fs + m.f);
-                    const int j = k == 0 ? fi.iu : (k == 1 ? 2 + fi.igc : 5 + fi.idp);
-                    cp_async8(&s_cand[wid][i & 1][lane], nbuf(F, j) + nd);
-                    cp_async_arrive(&s_bar[wid][i & 1]);
-                }
-            };
-            ChunkMeta m0{}, m1{}, m2{};
-            Stage st0{}, st1{};
             bool p_ok = true;
             // One frame: the warp's contiguous share (chunk_share).  Several frames: chunk g goes to warp
             // g mod (warps), warps counted across the blocks, so that every step of the pass spans few
@@ -1577,51 +1573,71 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
             const int2 range = contiguous ? s_range[wid] : make_int2(wid * (int)gridDim.x + (int)blockIdx.x, total);
             const int cb = range.x, ce = range.y;
             const int cs = contiguous ? 1 : nw;
-            if (cb < ce) {
-                if (pf_use) {
-                    m0 = pm0;
-                    st0 = pst0;
-                    m1 = pm1;
-                } else {
-                    m0 = fetch_meta(cb);
-                    st0 = issue_tma(m0, pipe_i);
-                    if (cb + cs < ce) m1 = fetch_meta(cb + cs);
-                }
-                load_cand(m0, pipe_i);
-            }
-            for (int g = cb; g < ce; g += cs) {
-                const bool has1 = g + cs < ce;
-                if (g + 2 * cs < ce) m2 = fetch_meta(g + 2 * cs);
-                if (has1) {
-                    st1 = issue_tma(m1, pipe_i + 1);
-                    load_cand(m1, pipe_i + 1);
-                }
-                const bool got = mbar_wait(&s_bar[wid][pipe_i & 1], (pipe_i >> 1) & 1u);
-                if (!__all_sync(0xffffffffu, got)) {
-                    if (lane == 0) {
-                        C.h->err = D2IC_WAIT_TIMEOUT;
-                        atomicExch(&C.h->abort, 1);
+            for (int g0 = cb; g0 < ce && p_ok; g0 += 32 * cs) {
+                const int cnt = min(32, (ce - g0 + cs - 1) / cs);
+                ChunkWork w{};
+                {
+                    const bool have = pf_use && g0 == cb;
+                    ChunkMeta m = pm;
+                    if (!have) {
+                        m = fetch_meta(g0 + lane * cs, ce);
+                        stage(0, m.f, m.pb, m.n, m.flags, m.origin, pipe_i);
                     }
-                    if (has1) mbar_wait(&s_bar[wid][(pipe_i + 1) & 1], ((pipe_i + 1) >> 1) & 1u);   // bounded
-                    p_ok = false;
-                    break;
+                    w.f = m.f;
+                    w.pb = m.pb;
+                    w.n = m.n;
+                    w.origin = m.origin;
+                    w.flags = (unsigned)m.flags;
+                    if (lane < cnt) {
+                        const d2ic_frame_t &F = frame(m.f);
+                        const FInfo fi = cached ? s_fi[slot_of(g0 + lane * cs)].info() : frame_info(C.fs + m.f);
+                        const Cand cand = make_cand(F, fi);
+                        w.tag = fi.tag;
+                        const int nd[4] = {m.nd.x, m.nd.y, m.nd.z, m.nd.w};
+#pragma unroll
+                        for (int a = 0; a < 4; ++a) {
+                            float2 dir;
+                            const float2 v = cand.at(nd[a], dir);
+                            w.ux[a] = v.x;
+                            w.uy[a] = v.y;
+                            w.rec[a] = (int)((m.slot >> (8 * a)) & 0xffu) * F.n_nodes + nd[a];
+                            // for the waiting group: the chunk's first node there, and how many it has there
+                            unsigned c2 = 0, first = 1;
+#pragma unroll
+                            for (int b = 0; b < 4; ++b) {
+                                const unsigned same = nd[b] / GN == nd[a] / GN;
+                                c2 += same;
+                                if (b < a) first &= same ^ 1u;
+                            }
+                            w.flags |= ((c2 << 1) | first) << (4 + 4 * a);
+                        }
+                        if (F.tile_w > 0) F.chunk_tile[m.c] = tile_origin(m.box0, w.ux, w.uy);
+                        if ((m.flags & (CH_STAGED | CH_TILED)) == (CH_STAGED | CH_TILED) && m.n <= D2IC_CHUNK_MAX &&
+                            inside_tile(F, m, w.ux, w.uy))
+                            w.flags |= CH_FAST;
+                    }
+                    __syncwarp();
                 }
-                float2 uc = make_float2(0.f, 0.f);
-                if (lane < 4) {
-                    const FInfo fi = cached ? s_fi[m0.s].info() : frame_info(C.fs + m0.f);
-                    const float2 *sc = s_cand[wid][pipe_i & 1];
-                    float2 dir;
-                    uc = cand_value(sc[lane], sc[4 + lane], sc[8 + lane], fi.alpha, fi.beta, fi.mode, dir);
-                    if (!cached) s_tag[wid] = fi.tag;
+#pragma unroll 1
+                for (int i = 0; i < cnt; ++i) {
+                    const bool more = i + 1 < cnt;
+                    if (more) stage(i + 1, w.f, w.pb, w.n, (int)w.flags, w.origin, pipe_i + 1);
+                    const bool got = mbar_wait(&s_bar[wid][pipe_i & 1], (pipe_i >> 1) & 1u);
+                    if (!__all_sync(0xffffffffu, got)) {
+                        if (lane == 0) {
+                            C.h->err = D2IC_WAIT_TIMEOUT;
+                            atomicExch(&C.h->abort, 1);
+                        }
+                        if (more) mbar_wait(&s_bar[wid][(pipe_i + 1) & 1], ((pipe_i + 1) >> 1) & 1u);   // bounded
+                        p_ok = false;
+                        break;
+                    }
+                    chunk_compute<KIND>(frame(ONE ? 0 : __shfl_sync(0xffffffffu, w.f, i)), w, i,
+                                        reinterpret_cast<const uint4 *>(wbuf + (pipe_i & 1) * CHUNK_BYTES),
+                                        reinterpret_cast<const float *>(wbuf + 2 * CHUNK_BYTES + (pipe_i & 1) * TILE_BYTES),
+                                        lane);
+                    ++pipe_i;
                 }
-                chunk_compute<KIND>(frame(m0.f), m0, uc, st0,
-                                    reinterpret_cast<const uint4 *>(wbuf + (pipe_i & 1) * CHUNK_BYTES),
-                                    reinterpret_cast<const float *>(wbuf + 2 * CHUNK_BYTES + (pipe_i & 1) * TILE_BYTES),
-                                    lane, cached ? &s_fi[m0.s].tag : &s_tag[wid]);
-                ++pipe_i;
-                m0 = m1;
-                st0 = st1;
-                m1 = m2;
             }
             if (trr) trace[7 * round + 1] = gtimer();
             // ---- N work: group gi of the active list goes to global warp gi mod (warps in grid); the
@@ -1739,13 +1755,11 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                 }
             }
             if (trr) trace[7 * round + 2] = gtimer();
-            // stage the next round's first chunk (same ranges if the active list is unchanged).  Only
+            // load the next round's first batch (same ranges if the active list is unchanged).  Only
             // from the shared-memory copy of the list: the global one may be rebuilt meanwhile.
             if (cached && p_ok && cb < ce && round + 1 < max_rounds && !ld_vol(&C.h->abort)) {
-                cur = 0;
-                pf_m0 = fetch_meta(cb);
-                pf_st0 = issue_tma(pf_m0, pipe_i);
-                if (cb + cs < ce) pf_m1 = fetch_meta(cb + cs);
+                pf_m = fetch_meta(cb + lane * cs, ce);
+                stage(0, pf_m.f, pf_m.pb, pf_m.n, pf_m.flags, pf_m.origin, pipe_i);
                 pf = true;
                 pf_na = na;
                 pf_total = total;
@@ -1823,7 +1837,6 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
     }
 
     if (pf) {                                       // no copy in flight at exit (bounded wait)
-        if (lane < CAND_N) mbar_arrive(&s_bar[wid][pipe_i & 1]);
         mbar_wait(&s_bar[wid][pipe_i & 1], (pipe_i >> 1) & 1u);
     }
 

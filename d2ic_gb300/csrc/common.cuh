@@ -27,18 +27,79 @@ int cuda_status(cudaError_t e, const char *what);
         }                                       \
     } while (0)
 
+// Two FP32 values in a 64-bit register pair, and IEEE operations on both with one instruction
+// (add/mul/fma.rn.f32x2): the same bits as two scalar operations in half the issue slots.
+typedef unsigned long long Pair;
+__device__ __forceinline__ Pair pair(float lo, float hi) {
+    Pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ Pair pair(float v) { return pair(v, v); }
+__device__ __forceinline__ float pair_lo(Pair p) { return __uint_as_float((unsigned)p); }
+__device__ __forceinline__ float pair_hi(Pair p) { return __uint_as_float((unsigned)(p >> 32)); }
+__device__ __forceinline__ Pair pair_fma(Pair a, Pair b, Pair c) {
+    Pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
+    Pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
+    Pair r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ Pair pair_add_down(Pair a, Pair b) {   // rounded towards minus infinity
+    Pair r;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// The arithmetic shared by one pixel (float) and two pixels (Pair): the same operations, the same bits.
+__device__ __forceinline__ float op_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float op_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ Pair op_fma(Pair a, Pair b, Pair c) { return pair_fma(a, b, c); }
+__device__ __forceinline__ Pair op_mul(Pair a, Pair b) { return pair_mul(a, b); }
+template <class T> __device__ __forceinline__ T op_const(float v);
+template <> __device__ __forceinline__ float op_const<float>(float v) { return v; }
+template <> __device__ __forceinline__ Pair op_const<Pair>(float v) { return pair(v); }
+
 // ---- cubic B-spline weights for taps -1..2 at fractional offset t in [0,1) ----
-__device__ __forceinline__ void bspline_w(float t, float w[4], float dw[4]) {
-    const float t2 = t * t, t3 = t2 * t, o = 1.0f - t;
-    const float s = 1.0f / 6.0f;
-    w[0] = o * o * o * s;
-    w[1] = (3.0f * t3 - 6.0f * t2 + 4.0f) * s;
-    w[2] = (-3.0f * t3 + 3.0f * t2 + 3.0f * t + 1.0f) * s;
-    w[3] = t3 * s;
-    dw[0] = -0.5f * o * o;
-    dw[1] = 1.5f * t2 - 2.0f * t;
-    dw[2] = -1.5f * t2 + t + 0.5f;
-    dw[3] = 0.5f * t2;
+// w = ((1 - t)^3, 4 - 6 t^2 + 3 t^3, 1 + 3 t + 3 t^2 - 3 t^3, t^3) / 6 in Horner form: 18 operations with the
+// derivatives where the expanded polynomials took 23, and no larger errors (at most 9e-8 against 1.1e-7; the
+// weights' sum is 1 within 1.3e-7, on average 2e-8 off).
+template <class T>
+__device__ __forceinline__ void bspline_w(T t, T w[4], T dw[4]) {
+    const T s = op_const<T>(1.f / 6.f), half = op_const<T>(0.5f), mhalf = op_const<T>(-0.5f), mone = op_const<T>(-1.f);
+    const T o = op_fma(t, mone, op_const<T>(1.f)), t2 = op_mul(t, t), o2 = op_mul(o, o);
+    w[0] = op_mul(o2, op_mul(o, s));
+    w[1] = op_fma(t2, op_fma(half, t, mone), op_const<T>(2.f / 3.f));
+    w[2] = op_fma(t, op_fma(t, op_fma(mhalf, t, half), half), s);
+    w[3] = op_mul(t2, op_mul(t, s));
+    dw[0] = op_mul(mhalf, o2);
+    dw[1] = op_mul(t, op_fma(op_const<T>(1.5f), t, op_const<T>(-2.f)));
+    dw[2] = op_fma(t, op_fma(op_const<T>(-1.5f), t, op_const<T>(1.f)), half);
+    dw[3] = op_mul(half, t2);
+}
+
+// The bilinear shape functions of an element at (xi, eta)
+template <class T>
+__device__ __forceinline__ void shape4(T xi, T eta, T N[4]) {
+    const T half = op_const<T>(0.5f), mhalf = op_const<T>(-0.5f);
+    const T a0 = op_fma(xi, mhalf, half), a1 = op_fma(xi, half, half);
+    const T b0 = op_fma(eta, mhalf, half), b1 = op_fma(eta, half, half);
+    N[0] = op_mul(a0, b0);
+    N[1] = op_mul(a1, b0);
+    N[2] = op_mul(a1, b1);
+    N[3] = op_mul(a0, b1);
+}
+template <class T>
+__device__ __forceinline__ T dot4(const T a[4], const T b[4]) {
+    return op_fma(a[3], b[3], op_fma(a[2], b[2], op_fma(a[1], b[1], op_mul(a[0], b[0]))));
 }
 
 struct Img {
@@ -54,22 +115,19 @@ __device__ __forceinline__ int clampi(int v, int lo, int hi) { return min(max(v,
 // The 4x4 tap arithmetic of the cubic B-spline, shared by every source of
 // coefficients (global memory, clamped global, shared-memory tile) so that all
 // paths produce identical bits.  Taps c[a][b]: row iy - 1 + a, column ix - 1 + b.
-__device__ __forceinline__ float cubic_taps(const float c[4][4], float tx, float ty, float &gx, float &gy) {
-    float wx[4], dwx[4], wy[4], dwy[4];
+template <class T>
+__device__ __forceinline__ T cubic_taps(const T c[4][4], T tx, T ty, T &gx, T &gy) {
+    T wx[4], dwx[4], wy[4], dwy[4], rv[4], rd[4];
     bspline_w(tx, wx, dwx);
     bspline_w(ty, wy, dwy);
-    float v = 0.f, ax = 0.f, ay = 0.f;
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-        const float rv = __fmaf_rn(wx[3], c[a][3], __fmaf_rn(wx[2], c[a][2], __fmaf_rn(wx[1], c[a][1], wx[0] * c[a][0])));
-        const float rd = __fmaf_rn(dwx[3], c[a][3], __fmaf_rn(dwx[2], c[a][2], __fmaf_rn(dwx[1], c[a][1], dwx[0] * c[a][0])));
-        v = __fmaf_rn(wy[a], rv, v);
-        ax = __fmaf_rn(wy[a], rd, ax);
-        ay = __fmaf_rn(dwy[a], rv, ay);
+        rv[a] = dot4(wx, c[a]);
+        rd[a] = dot4(dwx, c[a]);
     }
-    gx = ax;
-    gy = ay;
-    return v;
+    gx = dot4(wy, rd);
+    gy = dot4(dwy, rv);
+    return dot4(wy, rv);
 }
 
 // Cubic B-spline value and gradient at pixel (ix + tx, iy + ty), with integer
@@ -110,6 +168,18 @@ __device__ __forceinline__ float sample_cubic_tile(const float *tile, int tw, in
     for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int b = 0; b < 4; ++b) c[a][b] = base[a * tw + b];
+    return cubic_taps(c, tx, ty, gx, gy);
+}
+
+// Two pixels at once, with the taps at elements ia and ib of the tile.
+__device__ __forceinline__ Pair sample_cubic_tile2(const float *tile, int tw, unsigned ia, unsigned ib, Pair tx, Pair ty,
+                                                   Pair &gx, Pair &gy) {
+    Pair c[4][4];
+    const float *pa = tile + ia, *pb = tile + ib;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) c[a][b] = pair(pa[a * tw + b], pb[a * tw + b]);
     return cubic_taps(c, tx, ty, gx, gy);
 }
 

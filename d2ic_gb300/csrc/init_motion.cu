@@ -71,22 +71,6 @@ __device__ __forceinline__ void running_sums(int k0, int k1, int win, F &&f, O &
 constexpr int ZNCC_SEG = 7;   // outputs per thread of a running sum
 constexpr int ZNCC_MAX_THREADS = 384, ZNCC_TPT = 2;   // column tasks per thread
 
-// Two FP32 values in a 64-bit register pair and their fused multiply-add (fma.rn.f32x2: one instruction
-// for two IEEE multiply-adds).
-typedef unsigned long long Pair;
-__device__ __forceinline__ Pair pair(float lo, float hi) {
-    Pair r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ float pair_lo(Pair p) { return __uint_as_float((unsigned)p); }
-__device__ __forceinline__ float pair_hi(Pair p) { return __uint_as_float((unsigned)(p >> 32)); }
-__device__ __forceinline__ Pair pair_fma(Pair a, Pair b, Pair c) {
-    Pair r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
 template <int R>
 __global__ void __launch_bounds__(ZNCC_MAX_THREADS) zncc_kernel(const float *__restrict__ ref, int Hr, int Wr,
                                                                 const float *__restrict__ def, int Hd, int Wd,

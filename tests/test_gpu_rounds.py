@@ -78,3 +78,39 @@ def test_uneven_frames_finish_in_different_rounds(cuda, slots):
         alone = solve_batch([w])[0]
         assert got[1] == alone[1] and np.array_equal(got[0], alone[0])
         assert np.array_equal(got[3], alone[3], equal_nan=True)
+
+
+@pytest.mark.parametrize("side,element,move", [
+    (1700, 6, 0.0),      # 36-pixel chunks, 32 per lane batch and more: about 33 chunks per warp
+    (331, 7, 0.0),       # 49-pixel chunks: the second pixel of a pair is missing in lanes 17..31
+    (300, 16, 0.0),      # full 256-pixel chunks
+    (300, 16, 9.0),      # every stencil outside the tile placed before: the general path, then the packed one
+    (95, 5, 3.0),        # 25-pixel chunks: no lane has a second pixel
+])
+def test_packed_pixels_and_lane_batches(cuda, side, element, move):
+    """Chunks taken in batches of 32 and pixels two at a time: one evaluation against FP64 torch sums.
+
+    The chunk boundaries and the last, partly filled batch are where a chunk or a pixel could be lost or
+    counted twice; the tolerance is that of the other evaluations (FP32 residuals, sums of up to 2e6 terms)."""
+    import d2ic_gb300 as d2
+    from d2ic_gb300.engine import Engine, FrameLayout, FrameSlot, descriptors_to_device
+    from d2ic_gb300.synthetic import Translation, rect_mask, speckle_sequence_device
+    ref, frames = speckle_sequence_device(side, side, [Translation(0.4 + move, -0.3 - move)], seed=5, noise_seeds=[5, 6])
+    ref, frame = (np.asarray(x.cpu()) if torch.is_tensor(x) else np.asarray(x) for x in (ref, frames[0]))
+    mesh, assets = d2.mask_to_mesh_assets(rect_mask(side, side, side - 24, side - 24), element)
+    pix = d2.build_pixel_assets(mesh, ref, 1.0, assets.roi_mask)
+    n_nodes = np.asarray(mesh.nodes_xy).shape[0]
+    layout = FrameLayout(pix, n_nodes, ref, "cubic", cuda)
+    slot = FrameSlot(layout, 4)
+    slot.set_params(1e-6, 0.1)
+    slot.load_image(frame)
+    engine, desc = Engine(cuda, 1), descriptors_to_device([slot.desc], cuda)
+    rng = np.random.default_rng(1)
+    u = torch.as_tensor(rng.normal(0.0, 0.2, (n_nodes, 2)) + [move, -move], dtype=torch.float32, device=cuda)
+    J, g = engine.eval_objective(desc, u, layout.kind)
+    from oracle import objective, pixels
+    oa = pixels.build_pixel_assets(np.asarray(mesh.nodes_xy), np.asarray(mesh.elements), side, side, assets.roi_mask)
+    pb = objective.Problem.build(ref, frame, oa, "cubic")
+    J64, g64 = objective.J_total_and_grad(u.cpu().numpy().astype(np.float64), pb, 0.1)
+    assert abs(float(J) - J64) <= 1e-5 * J64
+    assert np.abs(g.cpu().numpy() - g64).max() <= 1e-5 * np.abs(g64).max()
