@@ -600,7 +600,7 @@ __device__ __forceinline__ void chunk_compute(const d2ic_frame_t &F, const Chunk
         constexpr float MAGIC = 12582912.f;
         Pair N[4];
         shape4(pair(__uint_as_float(ra.z), __uint_as_float(rb.z)), pair(__uint_as_float(ra.w), __uint_as_float(rb.w)), N);
-        const Pair dx = dot4(N, ux2), dy = dot4(N, uy2);
+        const Pair dx = shape_sum(N, ux2), dy = shape_sum(N, uy2);
         const Pair mx = pair_add_down(dx, pair(MAGIC)), my = pair_add_down(dy, pair(MAGIC));
         const Pair tx = pair_add(dx, pair_fma(mx, pair(-1.f), pair(MAGIC)));
         const Pair ty = pair_add(dy, pair_fma(my, pair(-1.f), pair(MAGIC)));
@@ -627,8 +627,8 @@ __device__ __forceinline__ void chunk_compute(const d2ic_frame_t &F, const Chunk
         shape4(__uint_as_float(r4.z), __uint_as_float(r4.w), N);
         int ix, iy;
         float tx, ty;
-        split_coord(x, dot4(N, ux), ix, tx);
-        split_coord(y, dot4(N, uy), iy, ty);
+        split_coord(x, shape_sum(N, ux), ix, tx);
+        split_coord(y, shape_sum(N, uy), iy, ty);
         float gx, gy, v;
         const int lx = ix - 1 - tx0, ly = iy - 1 - ty0;   // stencil corner inside the tile
         if (tiled && (unsigned)lx <= (unsigned)(tw - 4) && (unsigned)ly <= (unsigned)(th - 4))
@@ -1793,7 +1793,7 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
             if (!dead) {
                 s_hdr[4] = (int)(r.y & REL_STOP);
                 s_hdr[6] = (int)r.x;
-                if (r.y & REL_INLINE) {                 // na == 1 and the list unchanged
+                if ((r.y & REL_INLINE) && (int)(r.y >> 16) == s_hdr[8]) {   // na == 1 and the list unchanged
                     s_fi[0] = FRule{__uint_as_float(r.z), __uint_as_float(r.w), r.y,
                                     (s_fi[0].tag + (r.x - (unsigned)round)) & TAG_MASK};
                     s_hdr[5] = REFRESH_NONE;
@@ -1817,6 +1817,8 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                         s_hdr[5] = REFRESH_RULES;
                     }
                 }
+                // rounds passed over: their list reads are done as well
+                if (r.x > target) atomicAdd(&C.h->blocks_past, r.x - target);
             }
         }
         __syncthreads();

@@ -62,6 +62,8 @@ __device__ __forceinline__ Pair pair_add_down(Pair a, Pair b) {   // rounded tow
 // The arithmetic shared by one pixel (float) and two pixels (Pair): the same operations, the same bits.
 __device__ __forceinline__ float op_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ float op_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float op_add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ Pair op_add(Pair a, Pair b) { return pair_add(a, b); }
 __device__ __forceinline__ Pair op_fma(Pair a, Pair b, Pair c) { return pair_fma(a, b, c); }
 __device__ __forceinline__ Pair op_mul(Pair a, Pair b) { return pair_mul(a, b); }
 template <class T> __device__ __forceinline__ T op_const(float v);
@@ -69,21 +71,23 @@ template <> __device__ __forceinline__ float op_const<float>(float v) { return v
 template <> __device__ __forceinline__ Pair op_const<Pair>(float v) { return pair(v); }
 
 // ---- cubic B-spline weights for taps -1..2 at fractional offset t in [0,1) ----
-// w = ((1 - t)^3, 4 - 6 t^2 + 3 t^3, 1 + 3 t + 3 t^2 - 3 t^3, t^3) / 6 in Horner form: 18 operations with the
-// derivatives where the expanded polynomials took 23, and no larger errors (at most 9e-8 against 1.1e-7; the
-// weights' sum is 1 within 1.3e-7, on average 2e-8 off).
+// w = ((1 - t)^3, 4 - 6 t^2 + 3 t^3, 1 + 3 t + 3 t^2 - 3 t^3, t^3) / 6, dw its derivative; the order of the
+// operations is written out, so that one and two pixels give the same bits.  (A Horner form with 18 operations
+// instead of 23 gains 1 % of a round at 2048 x 2048; other bits let a solve near its rounding floor stop some
+// iterations earlier or later.)
 template <class T>
 __device__ __forceinline__ void bspline_w(T t, T w[4], T dw[4]) {
-    const T s = op_const<T>(1.f / 6.f), half = op_const<T>(0.5f), mhalf = op_const<T>(-0.5f), mone = op_const<T>(-1.f);
-    const T o = op_fma(t, mone, op_const<T>(1.f)), t2 = op_mul(t, t), o2 = op_mul(o, o);
-    w[0] = op_mul(o2, op_mul(o, s));
-    w[1] = op_fma(t2, op_fma(half, t, mone), op_const<T>(2.f / 3.f));
-    w[2] = op_fma(t, op_fma(t, op_fma(mhalf, t, half), half), s);
-    w[3] = op_mul(t2, op_mul(t, s));
-    dw[0] = op_mul(mhalf, o2);
-    dw[1] = op_mul(t, op_fma(op_const<T>(1.5f), t, op_const<T>(-2.f)));
-    dw[2] = op_fma(t, op_fma(op_const<T>(-1.5f), t, op_const<T>(1.f)), half);
-    dw[3] = op_mul(half, t2);
+    const T s = op_const<T>(1.f / 6.f), three = op_const<T>(3.f), mone = op_const<T>(-1.f);
+    const T o = op_fma(t, mone, op_const<T>(1.f)), t2 = op_mul(t, t), t3 = op_mul(t2, t);
+    const T m3 = op_mul(op_const<T>(-3.f), t3);
+    w[0] = op_mul(op_mul(op_mul(o, o), o), s);
+    w[1] = op_mul(op_fma(op_fma(op_const<T>(6.f), t2, m3), mone, op_const<T>(4.f)), s);
+    w[2] = op_mul(op_add(op_fma(three, t, op_fma(three, t2, m3)), op_const<T>(1.f)), s);
+    w[3] = op_mul(t3, s);
+    dw[0] = op_mul(op_mul(op_const<T>(-0.5f), o), o);
+    dw[1] = op_fma(op_const<T>(1.5f), t2, op_mul(op_const<T>(-2.f), t));
+    dw[2] = op_add(op_fma(op_const<T>(-1.5f), t2, t), op_const<T>(0.5f));
+    dw[3] = op_mul(op_const<T>(0.5f), t2);
 }
 
 // The bilinear shape functions of an element at (xi, eta)
@@ -100,6 +104,11 @@ __device__ __forceinline__ void shape4(T xi, T eta, T N[4]) {
 template <class T>
 __device__ __forceinline__ T dot4(const T a[4], const T b[4]) {
     return op_fma(a[3], b[3], op_fma(a[2], b[2], op_fma(a[1], b[1], op_mul(a[0], b[0]))));
+}
+// a displacement component at a pixel
+template <class T>
+__device__ __forceinline__ T shape_sum(const T N[4], const T u[4]) {
+    return op_fma(N[3], u[3], op_fma(N[2], u[2], op_fma(N[0], u[0], op_mul(N[1], u[1]))));
 }
 
 struct Img {
