@@ -23,9 +23,10 @@
 //   control      one warp per frame waits for the supergroup records and runs
 //                the CG control of d2ic/solver_global_cg.py:362-461 (stop test,
 //                PR+ beta, restart on g.d >= 0, Armijo with 10 halvings and
-//                the forced 2^-10 step); the round's last frame releases the
-//                next round with one tagged record, which also carries the
-//                next candidate rule when a single frame is active.
+//                the forced 2^-10 step) and publishes the frame's next candidate
+//                rule as a tagged record; a block goes on when it has the records
+//                of all active frames (more than FS frames: the round's last
+//                frame releases the next round for all).
 //
 // A round of a small frame is a chain of such hand-overs.  With counters and
 // fences (count the chunks of a group, poll the counter, gather; supergroup
@@ -128,6 +129,7 @@ struct Ctl {
     int *cpre;     // two copies of n_frames + 1
     int *gpre;     // two copies of n_frames + 1
     FrameState *fs;
+    uint4 *rule;   // n_frames: candidate rule of the next round, as a tagged record (direct rounds)
     int n;         // n_frames
     __device__ __forceinline__ int *act(int b) const { return active + b * n; }
     __device__ __forceinline__ int *cp(int b) const { return cpre + b * (n + 1); }
@@ -136,8 +138,9 @@ struct Ctl {
 
 __host__ __device__ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// control block: header | cmd | active | cpre | gpre | frame states
-__host__ __device__ inline size_t ctl_layout(int n, size_t *o_active, size_t *o_cpre, size_t *o_gpre, size_t *o_fs) {
+// control block: header | cmd | active | cpre | gpre | frame states | rule records
+__host__ __device__ inline size_t ctl_layout(int n, size_t *o_active, size_t *o_cpre, size_t *o_gpre, size_t *o_fs,
+                                             size_t *o_rule) {
     size_t off = align256(sizeof(CtlHeader));
     off = align256(off + sizeof(int) * (size_t)n);          // cmd
     *o_active = off;                                        // two copies of each list array
@@ -148,12 +151,14 @@ __host__ __device__ inline size_t ctl_layout(int n, size_t *o_active, size_t *o_
     off = align256(off + 2 * sizeof(int) * (size_t)(n + 1));
     *o_fs = off;
     off = align256(off + sizeof(FrameState) * (size_t)n);
+    *o_rule = off;
+    off = align256(off + sizeof(uint4) * (size_t)n);
     return off;
 }
 
 __device__ inline Ctl make_ctl(char *base, int n) {
-    size_t oa, oc, og, of;
-    ctl_layout(n, &oa, &oc, &og, &of);
+    size_t oa, oc, og, of, orl;
+    ctl_layout(n, &oa, &oc, &og, &of, &orl);
     Ctl c;
     c.h = (CtlHeader *)base;
     c.cmd = (int *)(base + align256(sizeof(CtlHeader)));
@@ -162,6 +167,7 @@ __device__ inline Ctl make_ctl(char *base, int n) {
     c.gpre = (int *)(base + og);
     c.n = n;
     c.fs = (FrameState *)(base + of);
+    c.rule = (uint4 *)(base + orl);
     return c;
 }
 
@@ -261,7 +267,18 @@ __device__ __forceinline__ FInfo frame_info(const FrameState *S) {
 // this launch; y: bit 0 the launch's slice ends, bit 1 the candidate rule of the only active frame
 // is in the record (mode, buffer indices in bits 2-9; alpha, beta in z, w), bits 16-31 the version
 // of the active list.  With several active frames the rules are read from the frame states.
-constexpr unsigned REL_STOP = 1u, REL_INLINE = 2u;
+//
+// Several frames, up to FS of them with a control warp each ("direct" rounds): there is no common
+// release.  Each control warp publishes its frame's next rule as a record of the same form (x: rounds
+// completed, REL_FIN: the frame is finished), and a block goes on when it has seen the records of all
+// active frames.  Only after a round in which a frame finished does everybody wait for a release record, with
+// the new list.  A frame without work in a block may be ahead of that block by a round; its flags count
+// only in the record of the round that the block waits for.
+constexpr unsigned REL_STOP = 1u, REL_INLINE = 2u, REL_FIN = 1u << 12;
+//
+// 2 frames of 911 and 1,535 chunks: 19.2 -> 14.9 us per round; 12 frames of together 46,106 chunks: 85.4 ->
+// 81.7 us (with the descriptors of the active frames in shared memory).
+constexpr int FS = 16;         // frames with direct rounds: their descriptors fit the block's static shared memory
 enum { REFRESH_NONE = 0, REFRESH_RULES = 1, REFRESH_LIST = 2 };   // what a block reads after a release
 __device__ __forceinline__ unsigned rel_pack(const FInfo &fi) {
     return REL_INLINE | ((unsigned)fi.mode << 2) | ((unsigned)fi.iu << 4) | ((unsigned)fi.igc << 5) |
@@ -469,7 +486,7 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity
 
 // A chunk as its lane holds it from the load to the candidates.
 struct ChunkMeta {
-    int f, c, pb, n;                 // frame, chunk within the frame, first pixel, pixels
+    int f, c, pb, n;                 // frame (its key), chunk within the frame, first pixel, pixels
     int box0, box1;                  // packed pixel-box corners
     int origin, flags;               // packed tile origin (TMA column, row), CH_* bits
     int4 nd;                         // nodes
@@ -1073,6 +1090,7 @@ __device__ void rebuild_active(const d2ic_frame_t *frames, int n_frames, Ctl &C)
 // marked reported (their outputs were written at the end of that launch).
 __device__ void r_init(const d2ic_frame_t *frames, int n_frames, Ctl &C) {
     for (int f = threadIdx.x; f < n_frames; f += NT) {
+        C.rule[f] = make_uint4(0u, 0u, 0u, 0u);
         const int cmd = ld_vol(C.cmd + f);
         if (cmd == CMD_INIT) {
             FrameState S;
@@ -1284,19 +1302,64 @@ __device__ __forceinline__ FInfo info_of(const FrameState &S) {
     return fi;
 }
 
+// The round's frames have all run their control step and one has finished: the active list is rebuilt
+// (whole warp).  Returns the release word.
+__device__ __forceinline__ unsigned rebuild_for_release(const d2ic_frame_t *frames, int n_frames, Ctl &C, int round,
+                                                        int list_version, int stop_flags, int lane) {
+    // no block still reads the list copy of an earlier round (bounded)
+    int past = 1;
+    if (lane == 0) past = wait_blocks_past(C.h, gridDim.x * (unsigned)round);
+    if (__shfl_sync(0xffffffffu, past, 0)) rebuild_active_warp(frames, n_frames, C, lane);
+    return ((unsigned)((list_version + 1) & 0xffff) << 16) | ((stop_flags & STOP_ON_FINISH) ? REL_STOP : 0u);
+}
+
 // Control step of frame f (one warp), and the round's release if it is the round's last frame.
+// direct: f is in slot `slot` of the na active frames `act`.
 template <bool SHARED>
 __device__ __forceinline__ void control_step(const d2ic_frame_t *frames, const d2ic_frame_t &F, int n_frames, Ctl &C, int f, unsigned tag,
-                                             int na, bool blockred, int round, int list_version, int eval_only,
-                                             int stop_flags, unsigned long long *trace, int trace_rounds, int lane,
-                                             FrameState &S) {
+                                             int na, bool blockred, bool direct, int slot, const int *act, int round,
+                                             int list_version, int eval_only, int stop_flags, unsigned long long *trace,
+                                             int trace_rounds, int lane, FrameState &S) {
     const bool rt = trace != nullptr && lane == 0 && round < trace_rounds;
+    const int irq = direct && slot == 0 && (stop_flags & STOP_ON_IRQ) ? ld_vol(&C.h->irq) : 0;
     if (!frame_r<SHARED>(F, f, C, eval_only, lane, tag, S)) return;
     if (rt) trace[7 * round + 3] = gtimer();
     // With one active frame whose control stays on this warp the release carries the next candidate
     // rule, and the state is stored after it.  (A finished frame's state is read by every block after
     // the release, so it is stored before.)
     const bool done = SHARED ? S.state == ST_DONE : __shfl_sync(0xffffffffu, lane == 0 ? (S.state == ST_DONE) : 0, 0);
+    if (!SHARED && direct) {
+        if (done) frame_store<SHARED>(S, C.fs + f, lane);
+        if (lane == 0) {
+            const FInfo nx = info_of(S);
+            if (done) fence_acq_rel();
+            st_record(C.rule + f, make_uint4((unsigned)(round + 1), rel_pack(nx) | (done ? REL_FIN : 0u) | (irq ? REL_STOP : 0u),
+                                             __float_as_uint(nx.alpha), __float_as_uint(nx.beta)));
+        }
+        if (rt) trace[7 * round + 4] = gtimer();
+        if (!done) {
+            frame_store<SHARED>(S, C.fs + f, lane);
+            return;
+        }
+        // the first of the frames that finished in this round waits for the others' records and rebuilds the list
+        const uint4 *mine = C.rule + (lane < na ? act[lane] : f);
+        uint4 r;
+        unsigned long long t0 = 0;
+        for (unsigned it = 0;; ++it) {
+            r = ld_record(mine);
+            if (__all_sync(0xffffffffu, r.x > (unsigned)round)) break;
+            if ((it & 63) == 63 && !keep_waiting(C.h, t0, lane)) return;
+        }
+        fence_acq_rel();
+        const unsigned fin = __ballot_sync(0xffffffffu, lane < na && r.x == (unsigned)(round + 1) && (r.y & REL_FIN));
+        if (__ffs((int)fin) - 1 != slot) return;
+        const unsigned rel = rebuild_for_release(frames, n_frames, C, round, list_version, stop_flags, lane);
+        if (lane == 0) {
+            fence_acq_rel();
+            st_record(&C.h->rel, make_uint4((unsigned)(round + 1), rel, 0u, 0u));
+        }
+        return;
+    }
     const bool inlined = na == 1 && blockred && !done;
     int last_frame = 1;
     if (!inlined) frame_store<SHARED>(S, C.fs + f, lane);
@@ -1313,13 +1376,8 @@ __device__ __forceinline__ void control_step(const d2ic_frame_t *frames, const d
         if (!inlined) {
             if (lane == 0 && na > 1) C.h->frames_done = 0;
             if (ld_vol(&C.h->finished)) {
-                // no block still reads the list copy of an earlier round (bounded)
-                int past = 1;
-                if (lane == 0) past = wait_blocks_past(C.h, gridDim.x * (unsigned)round);
-                if (__shfl_sync(0xffffffffu, past, 0)) rebuild_active_warp(frames, n_frames, C, lane);
+                rel = rebuild_for_release(frames, n_frames, C, round, list_version, stop_flags, lane);
                 if (lane == 0) C.h->finished = 0;
-                rel = (unsigned)((list_version + 1) & 0xffff) << 16;
-                if (stop_flags & STOP_ON_FINISH) rel |= REL_STOP;
             }
         }
         if (lane == 0) {
@@ -1395,6 +1453,9 @@ __device__ __forceinline__ int2 chunk_share(const d2ic_frame_t &F, int total, in
 // ONE: a launch of exactly one frame; the pixel pass then reads that frame's descriptor at a
 // fixed address, so its fields are loop invariants (loaded once, not per chunk; measured 2-5%
 // faster per round).
+constexpr int FRAME_BEGIN = (int)offsetof(d2ic_frame_t, coeff), FRAME_END = (int)offsetof(d2ic_frame_t, reserved_);
+static_assert(FRAME_BEGIN % 8 == 0 && FRAME_END % 8 == 0, "the kept part of a descriptor is whole words");
+
 template <int KIND, bool ONE = false>
 __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_frame_t *__restrict__ frames, int n_frames_arg,
                                                    char *ctl_base, int eval_only, const float *u_eval,
@@ -1407,7 +1468,10 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
     __shared__ int s_gpre[FC + 1];
     __shared__ int s_act[FC];
     __shared__ FRule s_fi[FC];
-    __shared__ __align__(16) unsigned long long s_frame[ONE ? sizeof(d2ic_frame_t) / 8 : 1];   // ONE: the descriptor
+    // descriptors of the active frames (na <= FS) without their tensor maps and reserved words
+    constexpr int FS_N = ONE ? 1 : FS, FS_WORDS = (FRAME_END - FRAME_BEGIN) / 8;
+    __shared__ __align__(16) unsigned long long s_frame[FS_N * FS_WORDS];
+    __shared__ unsigned s_tag0[FS_N];                // direct rounds: a frame's tag less the rounds completed
     __shared__ FrameState s_state;                   // ONE: the state in the control step (one warp of the grid)
     __shared__ int2 s_range[NWARP];                  // each warp's chunk range (one active frame)
     __shared__ int s_hdr[10];                         // n_active, total_chunks, total_groups, abort, slice stop,
@@ -1430,13 +1494,19 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
         if (frames[f].tile_w > 0)
             asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(frames[f].coeff_map) : "memory");
     const bool tiles_ok = (smem_addr(s_dyn) & 127) == 0;   // tile buffers need 128-byte alignment
-    // ONE: the block's copy of the descriptor.  Every round begins with an acquire that empties the L1,
+    // The block's copies of the descriptors.  Every round begins with an acquire that empties the L1,
     // so fields read from global memory cost an L2 round trip at each step of the round.
-    if (ONE)
-        for (int i = threadIdx.x; i < (int)(sizeof(d2ic_frame_t) / 8); i += NT)
-            s_frame[i] = reinterpret_cast<const unsigned long long *>(frames)[i];
-    auto frame = [&](int f) -> const d2ic_frame_t & {
-        return ONE ? *reinterpret_cast<const d2ic_frame_t *>(s_frame) : frames[f];
+    auto keep_frames = [&](int n) {                  // the frames of s_act[0..n), n <= FS
+        for (int i = threadIdx.x; i < n * FS_WORDS; i += NT)
+            s_frame[i] = reinterpret_cast<const unsigned long long *>(frames + (ONE ? 0 : s_act[i / FS_WORDS]))[FRAME_BEGIN / 8 + i % FS_WORDS];
+    };
+    if (ONE) keep_frames(1);
+    // a frame by its key: the active slot if the descriptors are kept, else its index
+    bool kept = ONE;
+    auto frame = [&](int key) -> const d2ic_frame_t & {
+        const char *own = reinterpret_cast<const char *>(s_frame) - FRAME_BEGIN;
+        if (ONE) return *reinterpret_cast<const d2ic_frame_t *>(own);
+        return kept ? *reinterpret_cast<const d2ic_frame_t *>(own + key * (FS_WORDS * 8)) : frames[key];
     };
     __syncthreads();
     // optional phase trace per round: warp 0 of block 0 stamps [0] round start, [1] end of its pixel
@@ -1505,7 +1575,13 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
     __syncthreads();
     load_list(C, s_hdr[7], s_hdr[0], s_cpre, s_gpre, s_act, s_fi);
     __syncthreads();
-    if (lane == 0 && s_hdr[0] == 1) s_range[wid] = chunk_share(frame(s_act[0]), s_hdr[1], s_hdr[2], wid);
+    if (!ONE && s_hdr[0] <= FS) {
+        keep_frames(s_hdr[0]);
+        if ((int)threadIdx.x < s_hdr[0]) s_tag0[threadIdx.x] = s_fi[threadIdx.x].tag;
+        __syncthreads();
+    }
+    if (!ONE) kept = s_hdr[0] <= FS;
+    if (lane == 0 && s_hdr[0] == 1) s_range[wid] = chunk_share(frame(0), s_hdr[1], s_hdr[2], wid);
     __syncthreads();
 
     while (round < max_rounds) {                    // a slice: at most max_rounds rounds, state kept in HBM
@@ -1514,6 +1590,7 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
         const int tg = s_hdr[2];
         const int lb = s_hdr[7];
         if (na == 0 || s_hdr[3] || s_hdr[4]) break;
+        const bool direct = !ONE && na >= 2 && na <= FS && tg <= (int)(gridDim.x * NWARP);
         const bool trr = tr && round < trace_rounds;
         if (trr) trace[7 * round + 0] = gtimer();
         // the active list only shrinks within a launch: the same count means the same list
@@ -1543,7 +1620,8 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                     const int s = slot_of(g);
                     const int f = ONE ? 0 : cached ? s_act[s] : checked_index(__ldcg(C.act(lb) + s), n_frames, C.h);
                     const int base = ONE ? 0 : cached ? s_cpre[s] : __ldcg(C.cp(lb) + s);
-                    m = load_meta<KIND>(frame(f), f, checked_index(g - base, frame(f).n_chunks, C.h), tiles_ok);
+                    const int key = kept ? s : f;
+                    m = load_meta<KIND>(frame(key), key, checked_index(g - base, frame(key).n_chunks, C.h), tiles_ok);
                 }
                 return m;
             };
@@ -1559,7 +1637,7 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                     if (bytes)
                         bulk_load(wbuf + (i & 1) * CHUNK_BYTES, reinterpret_cast<const uint4 *>(F.pix) + pb, bytes, bar);
                     if (tbytes)
-                        tensor_load_2d(wbuf + 2 * CHUNK_BYTES + (i & 1) * TILE_BYTES, frames[ONE ? 0 : f].coeff_map,
+                        tensor_load_2d(wbuf + 2 * CHUNK_BYTES + (i & 1) * TILE_BYTES, frames[ONE ? 0 : kept ? s_act[f] : f].coeff_map,
                                        (int)(short)(origin & 0xffff) + F.pad,
                                        (int)(short)((unsigned)origin >> 16) + F.pad, bar);
                 }
@@ -1568,9 +1646,12 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
             bool p_ok = true;
             // One frame: the warp's contiguous share (chunk_share).  Several frames: chunk g goes to warp
             // g mod (warps), warps counted across the blocks, so that every step of the pass spans few
-            // frames (measured faster for batches of small frames).
+            // frames (measured faster for batches of small frames); blocks that reduce node groups come last,
+            // so that the warps with a chunk more than the others are not theirs.
             const bool contiguous = ONE || na == 1;
-            const int2 range = contiguous ? s_range[wid] : make_int2(wid * (int)gridDim.x + (int)blockIdx.x, total);
+            const int reducers = min((tg + NWARP - 1) / NWARP, (int)gridDim.x);
+            const int order = (int)blockIdx.x - reducers + ((int)blockIdx.x < reducers ? (int)gridDim.x : 0);
+            const int2 range = contiguous ? s_range[wid] : make_int2(wid * (int)gridDim.x + order, total);
             const int cb = range.x, ce = range.y;
             const int cs = contiguous ? 1 : nw;
             for (int g0 = cb; g0 < ce && p_ok; g0 += 32 * cs) {
@@ -1590,7 +1671,7 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                     w.flags = (unsigned)m.flags;
                     if (lane < cnt) {
                         const d2ic_frame_t &F = frame(m.f);
-                        const FInfo fi = cached ? s_fi[slot_of(g0 + lane * cs)].info() : frame_info(C.fs + m.f);
+                        const FInfo fi = kept ? s_fi[m.f].info() : cached ? s_fi[slot_of(g0 + lane * cs)].info() : frame_info(C.fs + m.f);
                         const Cand cand = make_cand(F, fi);
                         w.tag = fi.tag;
                         const int nd[4] = {m.nd.x, m.nd.y, m.nd.z, m.nd.w};
@@ -1649,7 +1730,7 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
             const bool blockred = tg <= nw;
             int gcur = 0;
             for (int gi = gw, cslot = nw - 1 - gw;;) {
-                int cf = -1;
+                int cf = -1, cs_slot = 0;
                 unsigned ctag = 0;
                 if (gi < tg) {
                     int s = 0, f = 0, base = 0;
@@ -1664,7 +1745,7 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                         f = checked_index(__ldcg(C.act(lb) + s), n_frames, C.h);
                         base = __ldcg(C.gp(lb) + s);
                     }
-                    const d2ic_frame_t &F = frame(f);
+                    const d2ic_frame_t &F = frame(kept ? s : f);
                     const int g = gi - base;
                     gi += nw;
                     if (g >= F.n_groups) continue;         // padding of the frame's group range
@@ -1737,6 +1818,7 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                             __syncwarp();
                             if (__shfl_sync(0xffffffffu, lastf, 0)) {   // the frame's last supergroup
                                 cf = f;
+                                cs_slot = s;
                                 ctag = fi.tag;
                             }
                         }
@@ -1744,14 +1826,16 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                 } else if (blockred && cslot < na) {
                     cf = ONE ? 0 : cached ? s_act[cslot] : checked_index(__ldcg(C.act(lb) + cslot), n_frames, C.h);
                     ctag = cached ? s_fi[cslot].tag : frame_info(C.fs + cf).tag;
+                    cs_slot = cslot;
                     cslot += nw;
                 } else {
                     break;
                 }
                 if (cf >= 0) {
                     FrameState local;
-                    control_step<ONE>(frames, frame(cf), n_frames, C, cf, ctag, ONE ? 1 : na, blockred, round, s_hdr[8],
-                                      eval_only, stop_flags, trace, trace_rounds, lane, ONE ? s_state : local);
+                    control_step<ONE>(frames, frame(kept ? cs_slot : cf), n_frames, C, cf, ctag, ONE ? 1 : na, blockred, direct,
+                                      cs_slot, s_act, round, s_hdr[8], eval_only, stop_flags, trace, trace_rounds, lane,
+                                      ONE ? s_state : local);
                 }
             }
             if (trr) trace[7 * round + 2] = gtimer();
@@ -1765,12 +1849,10 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                 pf_total = total;
             }
         }
-        // ---- end of round: one thread per block polls the release record.  Records only move
-        // forward; a block that had no work in a round may find a later one. ----
+        // ---- end of round: one thread per block polls the release record (direct rounds: one warp the
+        // rule records).  Records only move forward; a block that had no work in a round may find a later one. ----
         __syncthreads();
-        if (threadIdx.x == 0) {
-            atomicAdd(&C.h->blocks_past, 1u);           // this block's list reads of the round are done
-            const unsigned target = (unsigned)(round + 1);
+        auto wait_release = [&](unsigned target) {       // one thread
             uint4 r = ld_record(&C.h->rel);
             unsigned long long t0 = 0;
             int dead = 0;
@@ -1820,6 +1902,37 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                 // rounds passed over: their list reads are done as well
                 if (r.x > target) atomicAdd(&C.h->blocks_past, r.x - target);
             }
+        };
+        const unsigned target = (unsigned)(round + 1);
+        if (threadIdx.x == 0) atomicAdd(&C.h->blocks_past, 1u);   // this block's list reads of the round are done
+        if (!direct) {
+            if (threadIdx.x == 0) wait_release(target);
+        } else if (wid == 0) {
+            const uint4 *mine = C.rule + s_act[min(lane, na - 1)];
+            uint4 r;
+            unsigned long long t0 = 0;
+            bool dead = false;
+            for (unsigned it = 0;; ++it) {
+                r = ld_record(mine);
+                if (__all_sync(0xffffffffu, r.x >= target)) break;
+                if ((it & 63) == 63 && !keep_waiting(C.h, t0, lane)) {
+                    dead = true;
+                    break;
+                }
+            }
+            fence_acq_rel();
+            const bool now = r.x == target;
+            const bool fin = __any_sync(0xffffffffu, now && (r.y & REL_FIN)), stop = __any_sync(0xffffffffu, now && (r.y & REL_STOP));
+            if (!dead && lane < na)
+                s_fi[lane] = FRule{__uint_as_float(r.z), __uint_as_float(r.w), r.y, (s_tag0[lane] + r.x) & TAG_MASK};
+            if (lane == 0) {
+                s_hdr[3] = dead;
+                s_hdr[4] = 0;
+                s_hdr[5] = REFRESH_NONE;
+                s_hdr[6] = (int)target;
+                if (fin && !dead) wait_release(target);
+                if (stop) s_hdr[4] = 1;
+            }
         }
         __syncthreads();
         if (s_hdr[5] != REFRESH_NONE && !s_hdr[3]) {    // rules from the frame states; a changed list is reloaded
@@ -1827,9 +1940,33 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                 if (na <= FCACHE)
                     for (int s = threadIdx.x; s < na; s += NT) s_fi[s] = make_rule(frame_info(C.fs + s_act[s]));
             } else if (s_hdr[0] > 0) {
-                load_list(C, s_hdr[7], s_hdr[0], s_cpre, s_gpre, s_act, s_fi);
+                // after direct rounds the rules are the records' (the states may still be on their way); the
+                // new list's frames are among the old one's
+                const int n2 = s_hdr[0], t = (int)threadIdx.x;
+                FRule rule{};
+                unsigned tag0 = 0;
+                bool have = false;
+                if (direct && t < n2) {
+                    const int f = checked_index(__ldcg(C.act(s_hdr[7]) + t), C.n, C.h);
+                    for (int o = 0; o < na; ++o)
+                        if (s_act[o] == f) {
+                            tag0 = s_tag0[o];
+                            have = true;
+                        }
+                    const uint4 r = ld_record(C.rule + f);
+                    rule = FRule{__uint_as_float(r.z), __uint_as_float(r.w), r.y, (tag0 + r.x) & TAG_MASK};
+                }
                 __syncthreads();
-                if (lane == 0 && s_hdr[0] == 1) s_range[wid] = chunk_share(frame(s_act[0]), s_hdr[1], s_hdr[2], wid);
+                load_list(C, s_hdr[7], n2, s_cpre, s_gpre, s_act, s_fi);
+                if (have) s_fi[t] = rule;                // written by this thread in load_list, too
+                __syncthreads();
+                if (!ONE && n2 <= FS) {
+                    keep_frames(n2);
+                    if (t < n2) s_tag0[t] = have ? tag0 : s_fi[t].tag - (unsigned)s_hdr[6];
+                    __syncthreads();
+                }
+                if (!ONE) kept = n2 <= FS;
+                if (lane == 0 && n2 == 1) s_range[wid] = chunk_share(frame(0), s_hdr[1], s_hdr[2], wid);
             }
             __syncthreads();
         }
@@ -1973,8 +2110,8 @@ using namespace d2ic;
 
 extern "C" size_t d2ic_cg_control_bytes(int n_frames) {
     if (n_frames < 1) n_frames = 1;
-    size_t a, b, c, d;
-    return ctl_layout(n_frames, &a, &b, &c, &d);
+    size_t a, b, c, d, e;
+    return ctl_layout(n_frames, &a, &b, &c, &d, &e);
 }
 
 // Workspace of one frame: 7 node buffers (u x2, g x3, dir x2), the K gradient

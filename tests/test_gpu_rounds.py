@@ -114,3 +114,31 @@ def test_packed_pixels_and_lane_batches(cuda, side, element, move):
     J64, g64 = objective.J_total_and_grad(u.cpu().numpy().astype(np.float64), pb, 0.1)
     assert abs(float(J) - J64) <= 1e-5 * J64
     assert np.abs(g.cpu().numpy() - g64).max() <= 1e-5 * np.abs(g64).max()
+
+
+@pytest.mark.parametrize("frames,grid", [
+    (2, 0), (16, 0), (17, 0),      # the most frames with their descriptors in shared memory, and one more
+    (5, 9),                        # node groups on most warps of the grid
+    (5, 3),                        # more groups than warps
+    (16, 40),
+])
+def test_direct_rounds_of_several_frames(cuda, frames, grid):
+    """Frames that hand over their own rules: pairs that finish in the same round, the list rebuilt down to one."""
+    import d2ic_gb300 as d2
+    from d2ic_gb300.engine import FrameLayout
+    from d2ic_gb300.serving import solve_batch
+    from d2ic_gb300.synthetic import Translation, rect_mask, speckle_sequence
+    work = []
+    for i in range(frames):
+        k = i // 2                                     # frames 2k and 2k + 1 are the same
+        side = 64 + 24 * (k % 4)
+        ref, images = speckle_sequence(side, side, [Translation(0.3, -0.2)], seed=40 + k, noise_seeds=[k, k + 50])
+        mesh, assets = d2.mask_to_mesh_assets(rect_mask(side, side, side - 12, side - 12), 12 - 4 * (k % 2))
+        pix = d2.build_pixel_assets(mesh, ref, 1.0, assets.roi_mask)
+        layout = FrameLayout(pix, mesh.nodes_xy.shape[0], ref, "cubic", cuda)
+        work.append((layout, images[0], None, d2.MeshDICConfig(max_iters=4 + 3 * k, tol=1e-6, reg_strength=0.1)))
+    together = solve_batch(work, grid_blocks=grid)
+    for w, got in zip(work, together):
+        alone = solve_batch([w])[0]
+        assert got[1] == alone[1] and np.array_equal(got[0], alone[0])
+        assert np.array_equal(got[3], alone[3], equal_nan=True)
