@@ -33,100 +33,157 @@ static int ensure_fir() {
     return D2IC_OK;
 }
 
-// rows: tmp[y][cx] = sum_k h[k] img[y][clamp(cx - pad + k)], cx in [0, W + 2 pad); image
-// blockIdx.z of a batch (contiguous images and buffers).  T: float or 8-bit camera pixels.  A block
-// takes an even share (at most RT_OUT outputs, a multiple of 4) of one row, its edge-extended
-// segment staged once in shared memory; a thread makes 4 consecutive outputs from 10 float4 reads
-// of the segment (each output's taps still summed in order k = 0 .. 2 KF).  The host sizes the
-// block to the share (rows_launch), so that no warp idles on 1024- or 2048-pixel rows.
-constexpr int RT_OUT = 4096;
-template <class T>
-__global__ void __launch_bounds__(1024) prefilter_rows(const T *__restrict__ img, int H, int W, int pad,
-                                                      int cpitch, float *__restrict__ tmp) {
-    __shared__ __align__(16) float s[RT_OUT + 2 * KF + 4];
-    img += (size_t)blockIdx.z * H * W;
-    tmp += (size_t)blockIdx.z * H * cpitch;
-    const int y = blockIdx.y;
-    const int CW = W + 2 * pad;
-    const int per = (((CW + gridDim.x - 1) / gridDim.x) + 3) & ~3;   // <= RT_OUT
-    const int cx0 = blockIdx.x * per;
-    const int n_out = min(per, CW - cx0);
-    const T *row = img + (size_t)y * W;
-    for (int i = threadIdx.x; i < ((n_out + 3) & ~3) + 2 * KF + 4; i += blockDim.x) {
-        const int src = clampi(cx0 - pad - KF + i, 0, W - 1);
-        s[i] = (float)__ldg(row + src);
-    }
-    __syncthreads();
-    const int o0 = 4 * threadIdx.x;
-    if (o0 >= n_out) return;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    const float4 *s4 = reinterpret_cast<const float4 *>(s) + threadIdx.x;
-#pragma unroll
-    for (int m = 0; m < (2 * KF + 4) / 4 + 1; ++m) {
-        const float4 q = s4[m];
-        const float v[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-#pragma unroll
-            for (int o = 0; o < 4; ++o) {
-                const int k = 4 * m + e - o;
-                if (k >= 0 && k <= 2 * KF) acc[o] += c_fir[k] * v[e];
-            }
-    }
-    float *out = tmp + (size_t)y * cpitch + cx0 + o0;
-#pragma unroll
-    for (int o = 0; o < 4; ++o)
-        if (o0 + o < n_out) out[o] = acc[o];
-}
+// One launch filters rows and columns: coeff[cy][cx] = sum_k h[k] f[clamp(cy - pad + k)][cx], with
+// f[y][cx] = sum_k h[k] img[y][clamp(cx - pad + k)], k = -KF .. KF, for cy in [0, H + 2 pad), cx in [0, W + 2 pad),
+// of image blockIdx.z of a batch (contiguous images and buffers).  T: float or 8-bit camera pixels.
+//
+// A block makes PF_W columns x `rows` rows of the result.  It filters the rows + 2 KF image rows that these need,
+// PF_STAGE at a time from an edge-extended copy in shared memory (the next ones are loaded while a stage is
+// filtered), keeps the filtered rows in shared memory and filters their columns.  A thread makes 8 neighbouring
+// outputs of two rows, then 8 of two columns, two per instruction; every output's taps are summed in order
+// k = -KF .. KF.
+//
+// 66 multiply-adds per pixel, and 33 more for the 2 KF extra rows per block, bound it (58 % of the FMA rate; the
+// rest is the barriers between the stages of two blocks per SM).  Two launches with the row sums in memory took
+// 482 us for 64 images of 1024 x 1024, 144 us for one of 4096 x 4096 and 15.4 us for one of 512 x 512 (two more
+// passes over memory, loads that nothing overlapped); this takes 270, 68 and 9.6 us, and 302, 74 and 8.9 us with one
+// output per instruction.  128 rows per block are best when there are blocks enough for the chip (64 rows and three
+// blocks per SM: 275 us for the 64 images); smaller images take 64 or 32 rows (prefilter_rows_per_block).
+constexpr int PF_W = 128, PF_STAGE = 32, PF_THREADS = 256;
+constexpr int PF_IN = PF_W + 2 * KF;                       // staged columns
+constexpr int PF_PITCH = 2 * PF_IN + PF_IN / 16 * 4;       // two staged rows side by side (see pf_at)
+constexpr int PF_LOADS = PF_STAGE * PF_IN / PF_THREADS;    // staged elements per thread
+static_assert(PF_IN % 32 == 0 && PF_STAGE % (PF_THREADS / 32) == 0, "a warp stages whole rows");
+// Element i of a pair of staged rows (a float of each), with 4 floats after every 16: a quarter warp's 16-byte
+// reads at a stride of 8 elements then fall into different banks.
+__device__ __forceinline__ int pf_at(int i) { return 2 * i + ((i >> 4) << 2); }
 
-// columns: coeff[cy][cx] = sum_k h[k] tmp[clamp(cy - pad + k)][cx], cy in [0, H + 2 pad).  A block
-// takes CT_W columns x CT_H rows; thread (x, y) makes the CT_R consecutive rows y CT_R .. of column x
-// from CT_R + 2 KF shared-memory reads (sliding window, taps in order k = 0 .. 2 KF per output).
-constexpr int CT_W = 32, CT_H = 128, CT_R = CT_H / 8;
-__global__ void __launch_bounds__(256) prefilter_cols(const float *__restrict__ tmp, int H, int W, int pad,
-                                                      int cpitch, float *__restrict__ coeff) {
-    __shared__ float s[CT_H + 2 * KF][CT_W + 1];
-    tmp += (size_t)blockIdx.z * H * cpitch;
+template <class T>
+__global__ void __launch_bounds__(PF_THREADS, 2) prefilter_kernel(const T *__restrict__ img, int H, int W, int pad, int cpitch,
+                                                                  int rows, float *__restrict__ coeff) {
+    extern __shared__ __align__(16) float pf_smem[];
+    float *stage = pf_smem;                                // PF_STAGE / 2 x PF_PITCH
+    float *filt = pf_smem + PF_STAGE / 2 * PF_PITCH;       // (rows + 2 KF) x PF_W: the filtered rows
+    img += (size_t)blockIdx.z * H * W;
     coeff += (size_t)blockIdx.z * (H + 2 * pad) * cpitch;
-    const int cx = blockIdx.x * CT_W + threadIdx.x;
-    const int cy0 = blockIdx.y * CT_H;
-    const int CW = W + 2 * pad;
-    for (int r = threadIdx.y; r < CT_H + 2 * KF; r += 8) {
-        const int src = clampi(cy0 - pad - KF + r, 0, H - 1);
-        s[r][threadIdx.x] = (cx < CW) ? tmp[(size_t)src * cpitch + cx] : 0.f;
-    }
-    __syncthreads();
-    if (cx >= CW) return;
-    const int r0 = threadIdx.y * CT_R;
-    float acc[CT_R];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int cx0 = blockIdx.x * PF_W, cy0 = blockIdx.y * rows;
+    const int out_rows = min(rows, H + 2 * pad - cy0), in_rows = out_rows + 2 * KF;
+    const int n_cols = min(PF_W, W + 2 * pad - cx0);
+    Pair h[KF + 1];                                        // h[k] = h[-k]
 #pragma unroll
-    for (int o = 0; o < CT_R; ++o) acc[o] = 0.f;
+    for (int k = 0; k <= KF; ++k) h[k] = pair(c_fir[KF + k]);
+    int col[PF_IN / 32];
 #pragma unroll
-    for (int j = 0; j < CT_R + 2 * KF; ++j) {
-        const float v = s[r0 + j][threadIdx.x];
+    for (int j = 0; j < PF_IN / 32; ++j) col[j] = clampi(cx0 - pad - KF + 32 * j + lane, 0, W - 1);
+    constexpr int RPW = PF_STAGE / (PF_THREADS / 32);      // staged rows per warp
+    float next[PF_LOADS];
+    auto load = [&](int r0) {                              // rows r0 .. of the block's image rows
 #pragma unroll
-        for (int o = 0; o < CT_R; ++o) {
-            const int k = j - o;
-            if (k >= 0 && k <= 2 * KF) acc[o] += c_fir[k] * v;
+        for (int r = 0; r < RPW; ++r) {
+            const T *row = img + (size_t)clampi(cy0 - pad - KF + r0 + warp * RPW + r, 0, H - 1) * W;
+#pragma unroll
+            for (int j = 0; j < PF_IN / 32; ++j) next[r * (PF_IN / 32) + j] = (float)__ldg(row + col[j]);
+        }
+    };
+    load(0);
+    const int lg = 32 - __clz((n_cols - 1) / 8);           // 2^lg threads per row, 8 outputs each
+    for (int r0 = 0; r0 < in_rows; r0 += PF_STAGE) {
+        __syncthreads();                                   // the previous stage is filtered
+#pragma unroll
+        for (int r = 0; r < RPW; r += 2)
+#pragma unroll
+            for (int j = 0; j < PF_IN / 32; ++j)
+                *reinterpret_cast<float2 *>(stage + (warp * RPW + r) / 2 * PF_PITCH + pf_at(32 * j + lane)) =
+                    make_float2(next[r * (PF_IN / 32) + j], next[(r + 1) * (PF_IN / 32) + j]);
+        __syncthreads();
+        if (r0 + PF_STAGE < in_rows) load(r0 + PF_STAGE);
+#pragma unroll 1
+        for (int i = threadIdx.x; i < (PF_STAGE / 2) << lg; i += PF_THREADS) {
+            const int r = 2 * (i >> lg), x = 8 * (i & ((1 << lg) - 1));
+            if (r0 + r >= in_rows) break;
+            const float *src = stage + r / 2 * PF_PITCH;
+            Pair acc[8];
+#pragma unroll
+            for (int o = 0; o < 8; ++o) acc[o] = 0ull;
+#pragma unroll
+            for (int m = 0; m < (2 * KF + 8) / 2; ++m) {
+                const ulonglong2 q = *reinterpret_cast<const ulonglong2 *>(src + pf_at(x + 2 * m));
+                const Pair v[2] = {q.x, q.y};
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+#pragma unroll
+                    for (int o = 0; o < 8; ++o) {
+                        const int k = 2 * m + e - o - KF;
+                        if (k >= -KF && k <= KF) acc[o] = pair_fma(h[k < 0 ? -k : k], v[e], acc[o]);
+                    }
+            }
+            float4 *dst = reinterpret_cast<float4 *>(filt + (size_t)(r0 + r) * PF_W + x);
+            dst[0] = make_float4(pair_lo(acc[0]), pair_lo(acc[1]), pair_lo(acc[2]), pair_lo(acc[3]));
+            dst[1] = make_float4(pair_lo(acc[4]), pair_lo(acc[5]), pair_lo(acc[6]), pair_lo(acc[7]));
+            dst += PF_W / 4;
+            dst[0] = make_float4(pair_hi(acc[0]), pair_hi(acc[1]), pair_hi(acc[2]), pair_hi(acc[3]));
+            dst[1] = make_float4(pair_hi(acc[4]), pair_hi(acc[5]), pair_hi(acc[6]), pair_hi(acc[7]));
         }
     }
+    __syncthreads();
+    constexpr int R = 8;
+    const int lg2 = 32 - __clz((n_cols - 1) / 2);          // 2^lg2 threads per strip of R rows, 2 columns each
+    const int x = 2 * ((int)threadIdx.x & ((1 << lg2) - 1));
+    if (x >= n_cols) return;
+    const bool both = x + 1 < n_cols;
+#pragma unroll 1
+    for (int y0 = R * ((int)threadIdx.x >> lg2); y0 < out_rows; y0 += R * (PF_THREADS >> lg2)) {
+        Pair acc[R];
 #pragma unroll
-    for (int o = 0; o < CT_R; ++o) {
-        const int cy = cy0 + r0 + o;
-        if (cy < H + 2 * pad) coeff[(size_t)cy * cpitch + cx] = acc[o];
+        for (int o = 0; o < R; ++o) acc[o] = 0ull;
+#pragma unroll
+        for (int j = 0; j < R + 2 * KF; ++j) {
+            // rows past in_rows: of outputs that are not stored
+            const Pair v = *reinterpret_cast<const Pair *>(filt + (y0 + j) * PF_W + x);
+#pragma unroll
+            for (int o = 0; o < R; ++o) {
+                const int k = j - o - KF;
+                if (k >= -KF && k <= KF) acc[o] = pair_fma(h[k < 0 ? -k : k], v, acc[o]);
+            }
+        }
+#pragma unroll
+        for (int o = 0; o < R; ++o)
+            if (y0 + o < out_rows) {
+                float *out = coeff + (size_t)(cy0 + y0 + o) * cpitch + cx0 + x;
+                out[0] = pair_lo(acc[o]);
+                if (both) out[1] = pair_hi(acc[o]);
+            }
     }
 }
 
-// blocks per row and threads per block of prefilter_rows for rows of CW outputs: the fewest blocks
-// of at most RT_OUT outputs, and one thread per 4 outputs of the (even, 4-aligned) share
-struct RowsLaunch {
-    unsigned blocks, threads;
-};
-static RowsLaunch rows_launch(int CW) {
-    const int blocks = (CW + RT_OUT - 1) / RT_OUT;
-    const int per = (((CW + blocks - 1) / blocks) + 3) & ~3;
-    const int quads = per / 4;
-    return RowsLaunch{(unsigned)blocks, (unsigned)(((quads + 31) / 32) * 32)};
+static size_t prefilter_smem(int rows) {
+    return sizeof(float) * ((size_t)PF_STAGE / 2 * PF_PITCH + (size_t)(rows + 2 * KF) * PF_W);
+}
+
+// The most rows per block that still give the chip two blocks per SM; small images take the fewest.
+static int prefilter_rows_per_block(int CW, int CH, int n_images, int sms) {
+    for (int rows = 128; rows > 32; rows /= 2)
+        if ((long long)((CW + PF_W - 1) / PF_W) * ((CH + rows - 1) / rows) * n_images >= 2ll * sms) return rows;
+    return 32;
+}
+
+template <class T>
+static int prefilter_launch(const T *img, int n_images, int H, int W, int pad, int cpitch, float *coeff, cudaStream_t s) {
+    int st = ensure_fir();
+    if (st) return st;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(prefilter_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prefilter_smem(128));
+    if (e != cudaSuccess) return cuda_status(e, "prefilter");
+    const int CW = W + 2 * pad, CH = H + 2 * pad;
+    const int rows = prefilter_rows_per_block(CW, CH, n_images, sms);
+    prefilter_kernel<T><<<dim3((CW + PF_W - 1) / PF_W, (CH + rows - 1) / rows, n_images), PF_THREADS, prefilter_smem(rows), s>>>(
+        img, H, W, pad, cpitch, rows, coeff);
+    D2IC_CHECK_LAUNCH("prefilter");
+    return D2IC_OK;
 }
 
 template <class T>
@@ -145,16 +202,7 @@ static int prefilter_one(const T *img, int H, int W, int pad, int cpitch, float 
     D2IC_REQUIRE(img && tmp && coeff, "%s: null pointer", name);
     D2IC_REQUIRE(H > 0 && W > 0 && H < 65536 && W < 65536, "%s: bad image size %dx%d", name, H, W);
     D2IC_REQUIRE(pad >= KF && cpitch >= W + 2 * pad, "%s: need pad >= %d and cpitch >= W + 2 pad", name, KF);
-    int st = ensure_fir();
-    if (st) return st;
-    const int CW = W + 2 * pad;
-    const RowsLaunch rl = rows_launch(CW);
-    prefilter_rows<T><<<dim3(rl.blocks, H), rl.threads, 0, s>>>(img, H, W, pad, cpitch, tmp);
-    D2IC_CHECK_LAUNCH("prefilter_rows");
-    prefilter_cols<<<dim3((CW + CT_W - 1) / CT_W, (H + 2 * pad + CT_H - 1) / CT_H), dim3(CT_W, 8), 0, s>>>(
-        tmp, H, W, pad, cpitch, coeff);
-    D2IC_CHECK_LAUNCH("prefilter_cols");
-    return D2IC_OK;
+    return prefilter_launch(img, 1, H, W, pad, cpitch, coeff, s);
 }
 
 template <class T>
@@ -206,17 +254,7 @@ extern "C" int d2ic_bspline_prefilter_batch(const float *img, int n_images, int 
     D2IC_REQUIRE(H > 0 && W > 0 && H < 65536 && W < 65536, "d2ic_bspline_prefilter_batch: bad image size %dx%d", H, W);
     D2IC_REQUIRE(pad >= KF && cpitch >= W + 2 * pad,
                  "d2ic_bspline_prefilter_batch: need pad >= %d and cpitch >= W + 2 pad", KF);
-    int st = ensure_fir();
-    if (st) return st;
-    cudaStream_t s = (cudaStream_t)stream;
-    const int CW = W + 2 * pad;
-    const RowsLaunch rl = rows_launch(CW);
-    prefilter_rows<float><<<dim3(rl.blocks, H, n_images), rl.threads, 0, s>>>(img, H, W, pad, cpitch, tmp);
-    D2IC_CHECK_LAUNCH("prefilter_rows");
-    prefilter_cols<<<dim3((CW + CT_W - 1) / CT_W, (H + 2 * pad + CT_H - 1) / CT_H, n_images), dim3(CT_W, 8), 0, s>>>(
-        tmp, H, W, pad, cpitch, coeff);
-    D2IC_CHECK_LAUNCH("prefilter_cols");
-    return D2IC_OK;
+    return prefilter_launch(img, n_images, H, W, pad, cpitch, coeff, (cudaStream_t)stream);
 }
 
 extern "C" int d2ic_bspline_prefilter(const float *img, int H, int W, int pad, int cpitch, float *tmp,

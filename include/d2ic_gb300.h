@@ -132,7 +132,8 @@ D2IC_API int d2ic_device_info(int device, int *num_sms, int *engine_blocks_per_s
 
 /* Cubic B-spline coefficients of an HxW float image extended by edge
  * replication, written with a `pad`-wide halo into coeff ((H+2pad) x cpitch).
- * tmp: H x cpitch floats of scratch.  pad >= 16, cpitch >= W + 2 pad. */
+ * tmp: H x cpitch floats of scratch (rows and columns are filtered in one launch that leaves it
+ * unused; it must still be given).  pad >= 16, cpitch >= W + 2 pad. */
 D2IC_API int d2ic_bspline_prefilter(const float *img, int H, int W, int pad, int cpitch,
                            float *tmp, float *coeff, void *stream);
 /* The same for n_images contiguous HxW images in one launch: image i's scratch at
