@@ -127,7 +127,11 @@ _SIGS = {
     "d2ic_hessian_prepare": (i32, [vp, i32, i32, i32, vp, f32, f32, vp, szt, vp, vp, vp]),
     "d2ic_hessian_check": (i32, [vp, i32, i32, vp]),
     "d2ic_pcg_solve": (i32, [vp, i32, i32, i32, vp, f32, f32, vp, vp, vp, vp, i32, f64, i32, vp, szt, vp, vp]),
+    "d2ic_bspline_prefilter_gradients": (i32, [vp, i32, i32, i32, i32, vp, vp, vp, vp]),
     "d2ic_local_gn_slot_bytes": (szt, [i32, i32]),
+    "d2ic_local_gn_history_sweeps": (i32, []),
+    "d2ic_local_gn_run": (i32, [vp, i32, i32, i32, i32, i32, vp, vp, vp, vp, i32, vp, vp, vp, vp, vp, i32, vp, f32, f32,
+                                f32, f32, vp, vp, vp]),
     "d2ic_local_gn_sweep": (i32, [vp, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, i32, vp, f32, f32, f32,
                                   f32, vp, vp, vp]),
 }

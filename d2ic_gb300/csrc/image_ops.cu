@@ -58,14 +58,22 @@ static_assert(PF_IN % 32 == 0 && PF_STAGE % (PF_THREADS / 32) == 0, "a warp stag
 // reads at a stride of 8 elements then fall into different banks.
 __device__ __forceinline__ int pf_at(int i) { return 2 * i + ((i >> 4) << 2); }
 
-template <class T>
+// GRADIENTS: the batch is one image and its central-difference gradient images (zero on the first and last column, row),
+// formed while the rows are loaded, with their results at coeff, coeff_gx and coeff_gy.
+template <class T, bool GRADIENTS = false>
 __global__ void __launch_bounds__(PF_THREADS, 2) prefilter_kernel(const T *__restrict__ img, int H, int W, int pad, int cpitch,
-                                                                  int rows, float *__restrict__ coeff) {
+                                                                  int rows, float *__restrict__ coeff,
+                                                                  float *__restrict__ coeff_gx, float *__restrict__ coeff_gy) {
     extern __shared__ __align__(16) float pf_smem[];
     float *stage = pf_smem;                                // PF_STAGE / 2 x PF_PITCH
     float *filt = pf_smem + PF_STAGE / 2 * PF_PITCH;       // (rows + 2 KF) x PF_W: the filtered rows
-    img += (size_t)blockIdx.z * H * W;
-    coeff += (size_t)blockIdx.z * (H + 2 * pad) * cpitch;
+    const int which = GRADIENTS ? (int)blockIdx.z : 0;
+    if (!GRADIENTS) {
+        img += (size_t)blockIdx.z * H * W;
+        coeff += (size_t)blockIdx.z * (H + 2 * pad) * cpitch;
+    } else if (which) {
+        coeff = which == 1 ? coeff_gx : coeff_gy;
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int cx0 = blockIdx.x * PF_W, cy0 = blockIdx.y * rows;
     const int out_rows = min(rows, H + 2 * pad - cy0), in_rows = out_rows + 2 * KF;
@@ -81,9 +89,18 @@ __global__ void __launch_bounds__(PF_THREADS, 2) prefilter_kernel(const T *__res
     auto load = [&](int r0) {                              // rows r0 .. of the block's image rows
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
-            const T *row = img + (size_t)clampi(cy0 - pad - KF + r0 + warp * RPW + r, 0, H - 1) * W;
+            const int y = clampi(cy0 - pad - KF + r0 + warp * RPW + r, 0, H - 1);
+            const T *row = img + (size_t)y * W;
 #pragma unroll
-            for (int j = 0; j < PF_IN / 32; ++j) next[r * (PF_IN / 32) + j] = (float)__ldg(row + col[j]);
+            for (int j = 0; j < PF_IN / 32; ++j) {
+                float v = 0.f;
+                if (which == 0) v = (float)__ldg(row + col[j]);
+                else if (which == 1 && col[j] > 0 && col[j] < W - 1)
+                    v = 0.5f * ((float)__ldg(row + col[j] + 1) - (float)__ldg(row + col[j] - 1));
+                else if (which == 2 && y > 0 && y < H - 1)
+                    v = 0.5f * ((float)__ldg(row + W + col[j]) - (float)__ldg(row - W + col[j]));
+                next[r * (PF_IN / 32) + j] = v;
+            }
         }
     };
     load(0);
@@ -168,20 +185,22 @@ static int prefilter_rows_per_block(int CW, int CH, int n_images, int sms) {
     return 32;
 }
 
-template <class T>
-static int prefilter_launch(const T *img, int n_images, int H, int W, int pad, int cpitch, float *coeff, cudaStream_t s) {
+template <class T, bool GRADIENTS = false>
+static int prefilter_launch(const T *img, int n_images, int H, int W, int pad, int cpitch, float *coeff, cudaStream_t s,
+                            float *coeff_gx = nullptr, float *coeff_gy = nullptr) {
     int st = ensure_fir();
     if (st) return st;
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(prefilter_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prefilter_smem(128));
+        e = cudaFuncSetAttribute(prefilter_kernel<T, GRADIENTS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)prefilter_smem(128));
     if (e != cudaSuccess) return cuda_status(e, "prefilter");
     const int CW = W + 2 * pad, CH = H + 2 * pad;
     const int rows = prefilter_rows_per_block(CW, CH, n_images, sms);
-    prefilter_kernel<T><<<dim3((CW + PF_W - 1) / PF_W, (CH + rows - 1) / rows, n_images), PF_THREADS, prefilter_smem(rows), s>>>(
-        img, H, W, pad, cpitch, rows, coeff);
+    prefilter_kernel<T, GRADIENTS><<<dim3((CW + PF_W - 1) / PF_W, (CH + rows - 1) / rows, n_images), PF_THREADS,
+                                     prefilter_smem(rows), s>>>(img, H, W, pad, cpitch, rows, coeff, coeff_gx, coeff_gy);
     D2IC_CHECK_LAUNCH("prefilter");
     return D2IC_OK;
 }
@@ -265,6 +284,15 @@ extern "C" int d2ic_bspline_prefilter(const float *img, int H, int W, int pad, i
 extern "C" int d2ic_bspline_prefilter_u8(const unsigned char *img, int H, int W, int pad, int cpitch, float *tmp,
                                          float *coeff, void *stream) {
     return prefilter_one(img, H, W, pad, cpitch, tmp, coeff, (cudaStream_t)stream, "d2ic_bspline_prefilter_u8");
+}
+
+extern "C" int d2ic_bspline_prefilter_gradients(const float *img, int H, int W, int pad, int cpitch, float *coeff,
+                                                float *coeff_gx, float *coeff_gy, void *stream) {
+    D2IC_REQUIRE(img && coeff && coeff_gx && coeff_gy, "d2ic_bspline_prefilter_gradients: null pointer");
+    D2IC_REQUIRE(H > 0 && W > 0 && H < 65536 && W < 65536, "d2ic_bspline_prefilter_gradients: bad image size %dx%d", H, W);
+    D2IC_REQUIRE(pad >= KF && cpitch >= W + 2 * pad,
+                 "d2ic_bspline_prefilter_gradients: need pad >= %d and cpitch >= W + 2 pad", KF);
+    return prefilter_launch<float, true>(img, 3, H, W, pad, cpitch, coeff, (cudaStream_t)stream, coeff_gx, coeff_gy);
 }
 
 extern "C" int d2ic_pad_image(const float *img, int H, int W, int pad, int cpitch, float *out, void *stream) {

@@ -6,8 +6,9 @@ constructor (``lam``, ``max_step``, ``omega``, ``interpolation``,
 ``LocalGNResult(u_nodal, strain, history)``; ``state.config.max_iters`` sweeps
 of the relaxed nodal Jacobi update, ``state.config.reg_strength`` as the spring
 weight, history rows ``[rms residual, rms step]`` when ``save_history``.
-Each sweep is two CUDA kernels (``d2ic_local_gn_sweep``); the gradient images
-and their sampling arrays are built on the device once per frame.  In the
+Each sweep is two CUDA kernels (``d2ic_local_gn_run`` launches all sweeps and their
+history); the sampling arrays of the frame and its gradient images are built on the
+device once per frame, by one launch for cubic interpolation.  In the
 reference pipeline it runs after the global CG (``BatchMeshBased(dic_local=...)``).
 """
 from __future__ import annotations
@@ -20,7 +21,7 @@ import torch
 
 from . import _lib
 from ._lib import ptr
-from .engine import FrameLayout, FrameSlot, as_device_image, descriptors_to_device, prepare_coefficients
+from .engine import PAD, FrameLayout, FrameSlot, as_device_image, descriptors_to_device, prepare_coefficients
 from .solver_base import SolverBase
 from .solver_global_cg import _normalize_interpolation
 from .types import Array
@@ -84,12 +85,14 @@ class LocalGaussNewtonSolver(SolverBase):
         self._has_pix = T(has, torch.int32)
         self._slots = torch.zeros(_lib.load().d2ic_local_gn_slot_bytes(nn, L.node_chunk_k) // 4, dtype=torch.float32,
                                   device=dev)
-        self._r2 = torch.zeros(max(L.n_chunks, 1), dtype=torch.float64, device=dev)
-        self._st = torch.zeros((nn + 255) // 256, dtype=torch.float64, device=dev)
+        rows = _lib.load().d2ic_local_gn_history_sweeps()
+        self._r2 = torch.zeros(rows * max(L.n_chunks, 1), dtype=torch.float64, device=dev)
+        self._st = torch.zeros(rows * ((nn + 255) // 256), dtype=torch.float64, device=dev)
         self._cgx = torch.empty_like(self._slot.coeff)
         self._cgy = torch.empty_like(self._slot.coeff)
-        self._gx = torch.empty((L.H, L.W), dtype=torch.float32, device=dev)
-        self._gy = torch.empty_like(self._gx)
+        if L.kind != _lib.INTERP_CUBIC:
+            self._gx = torch.empty((L.H, L.W), dtype=torch.float32, device=dev)
+            self._gy = torch.empty_like(self._gx)
         self._key = key
 
     def solve(self, state, def_image: Array) -> LocalGNResult:
@@ -100,10 +103,14 @@ class LocalGaussNewtonSolver(SolverBase):
         self._ensure(state)
         L, dev = self._layout, self._device
         img = as_device_image(def_image, dev)
-        self._slot.load_image(img)
-        _lib.call("d2ic_central_gradient", ptr(img), L.H, L.W, ptr(self._gx), ptr(self._gy), _lib.stream_handle())
-        prepare_coefficients(self._gx, L.kind, self._cgx, self._slot.tmp)
-        prepare_coefficients(self._gy, L.kind, self._cgy, self._slot.tmp)
+        if L.kind == _lib.INTERP_CUBIC:
+            _lib.call("d2ic_bspline_prefilter_gradients", ptr(img), L.H, L.W, PAD, L.cpitch, ptr(self._slot.coeff),
+                      ptr(self._cgx), ptr(self._cgy), _lib.stream_handle())
+        else:
+            self._slot.load_image(img)
+            _lib.call("d2ic_central_gradient", ptr(img), L.H, L.W, ptr(self._gx), ptr(self._gy), _lib.stream_handle())
+            prepare_coefficients(self._gx, L.kind, self._cgx)
+            prepare_coefficients(self._gy, L.kind, self._cgy)
         nn = L.n_nodes
         if state.u0_nodal is None:
             u = torch.zeros((nn, 2), dtype=torch.float32, device=dev)
@@ -114,14 +121,12 @@ class LocalGaussNewtonSolver(SolverBase):
         n_sweeps = int(state.config.max_iters)
         hist = torch.full((max(n_sweeps, 1), 2), float("nan"), dtype=torch.float64, device=dev)
         alpha = float(state.config.reg_strength)
-        for k in range(n_sweeps):
-            _lib.call("d2ic_local_gn_sweep", ptr(self._desc), L.n_chunks, nn, L.node_chunk_k, L.kind, ptr(self._cgx),
-                      ptr(self._cgy), ptr(u), ptr(self._slots), ptr(self._r2), ptr(self._has_pix), ptr(self._nbr),
-                      ptr(self._nbw), self._md, ptr(self._rho), self._lam, self._max_step, alpha, self._omega,
-                      ptr(v), ptr(self._st), _lib.stream_handle())
-            hist[k, 0] = torch.sqrt(self._r2[: max(L.n_chunks, 1)].sum() / max(L.n_pix, 1))
-            hist[k, 1] = torch.sqrt(self._st.sum() / (2 * nn))
-            u, v = v, u
+        _lib.call("d2ic_local_gn_run", ptr(self._desc), L.n_pix, L.n_chunks, nn, L.node_chunk_k, L.kind, ptr(self._cgx),
+                  ptr(self._cgy), ptr(u), ptr(v), n_sweeps, ptr(self._slots), ptr(self._r2), ptr(self._has_pix),
+                  ptr(self._nbr), ptr(self._nbw), self._md, ptr(self._rho), self._lam, self._max_step, alpha, self._omega,
+                  ptr(self._st), ptr(hist), _lib.stream_handle())
+        if n_sweeps % 2:
+            u = v
         u_host = u.cpu().numpy()
         save_history = bool(getattr(state.config, "save_history", False))
         return LocalGNResult(u_nodal=u_host, strain=np.zeros((nn, 3), dtype=np.float32),

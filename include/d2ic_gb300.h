@@ -141,6 +141,11 @@ D2IC_API int d2ic_bspline_prefilter(const float *img, int H, int W, int pad, int
 D2IC_API int d2ic_bspline_prefilter_batch(const float *img, int n_images, int H, int W, int pad, int cpitch,
                                           float *tmp, float *coeff, void *stream);
 
+/* The coefficients of an image and of its central-difference gradient images (as d2ic_central_gradient forms
+ * them) in one launch, each (H + 2 pad) x cpitch. */
+D2IC_API int d2ic_bspline_prefilter_gradients(const float *img, int H, int W, int pad, int cpitch, float *coeff,
+                                              float *coeff_gx, float *coeff_gy, void *stream);
+
 /* Copy an image into the halo layout with edge replication (linear kind). */
 D2IC_API int d2ic_pad_image(const float *img, int H, int W, int pad, int cpitch, float *out, void *stream);
 
@@ -261,6 +266,18 @@ D2IC_API int d2ic_local_gn_sweep(const d2ic_frame_t *frame_dev, int n_chunks, in
                                  const float *nbr_weight, int max_deg, const float *node_reg_weight, float lam,
                                  float max_step, float alpha_reg, float omega, float *u_next, double *step_part,
                                  void *stream);
+
+/* n_sweeps sweeps u -> u_other -> u -> ... (the result is in u_other if n_sweeps is odd) and their history
+ * rows hist[2 k] = RMS residual over n_pix pixels, hist[2 k + 1] = RMS step (device, 2 * n_sweeps doubles).
+ * chunk_r2 and step_part hold the sums of d2ic_local_gn_history_sweeps() sweeps (max(n_chunks, 1) and
+ * ceil(n_nodes / 256) doubles each). */
+D2IC_API int d2ic_local_gn_history_sweeps(void);
+D2IC_API int d2ic_local_gn_run(const d2ic_frame_t *frame_dev, int n_pix, int n_chunks, int n_nodes, int node_chunk_k,
+                               int interp_kind, const float *coeff_gx, const float *coeff_gy, float *u, float *u_other,
+                               int n_sweeps, float *slots, double *chunk_r2, const int *has_pix, const int *nbr_index,
+                               const float *nbr_weight, int max_deg, const float *node_reg_weight, float lam,
+                               float max_step, float alpha_reg, float omega, double *step_part, double *hist,
+                               void *stream);
 
 /* ---- result maps (replaces compute_discrepancy_map_ref, d2ic/discrepancy.py:86-127) ---- */
 
