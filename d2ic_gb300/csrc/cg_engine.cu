@@ -151,7 +151,7 @@ __host__ __device__ inline size_t ctl_layout(int n, size_t *o_active, size_t *o_
     *o_gpre = off;
     off = align256(off + 2 * sizeof(int) * (size_t)(n + 1));
     *o_fs = off;
-    off = align256(off + sizeof(FrameState) * (size_t)n);
+    off = (off + sizeof(FrameState) * (size_t)n + 15) & ~(size_t)15;
     *o_rule = off;
     off = align256(off + sizeof(uint4) * (size_t)n);
     return off;
@@ -2145,7 +2145,11 @@ static size_t ws_layout(int n_nodes, int n_chunks, int node_chunk_k, size_t off[
     const size_t ns = (ng + SG - 1) / SG;                     // supergroups of SG groups
     o += align256(sg_record_offset((int)ng) + sizeof(uint4) * SG_RECORDS * ns);
     off[3] = o;                                               // group_cnt
-    o += align256(sizeof(int) * (ng + ns + 1));
+    o += align256(sizeof(int) * (ns + 1));
+    // no less than for double-float partials of the groups and supergroups and a counter for each: the size
+    // of a frame that the fixed scratch array takes does not depend on how the sums are handed over
+    const size_t least = off[2] + align256(sizeof(float) * 2 * D2IC_NPART * (ng + ns)) + align256(sizeof(int) * (ng + ns + 1));
+    if (o < least) o = least;
     off[4] = o;                                               // chunk_tile
     o += align256(sizeof(int) * (size_t)(n_chunks > 0 ? n_chunks : 1));
     return o;

@@ -533,7 +533,7 @@ class Engine:
                          t[:, 5] - t[:, 4], t[:, 5] - t[:, 0]], axis=1) / 1e3
 
     def eval_objective(self, desc_dev: torch.Tensor, u: torch.Tensor, kind: int, stream=None):
-        J = torch.zeros(1, dtype=torch.float64, device=self.device)
+        J = torch.empty(1, dtype=torch.float64, device=self.device)
         g = torch.empty_like(u)
         _lib.call("d2ic_eval_objective", ptr(desc_dev), ptr(u), ptr(self.control), self.control.numel(), kind,
                   ptr(J), ptr(g), _lib.stream_handle(stream))

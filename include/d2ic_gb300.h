@@ -103,8 +103,7 @@ typedef struct d2ic_frame {
                                       groups, then (16-byte aligned) D2IC_NPART tagged 16-byte
                                       records for each of the n_super = ceil(n_groups / 16)
                                       supergroups                                       */
-    int         *group_cnt;        /* n_super + 1 completion counters (all 0 between rounds;
-                                      room for n_groups + n_super + 1)                  */
+    int         *group_cnt;        /* n_super + 1 completion counters (all 0 between rounds) */
     int         *chunk_tile;       /* n_chunks: origin (col | row << 16, int16 each) of the
                                       chunk's coefficient tile for the next pass        */
     double       tol;

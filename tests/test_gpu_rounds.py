@@ -142,3 +142,15 @@ def test_direct_rounds_of_several_frames(cuda, frames, grid):
         alone = solve_batch([w])[0]
         assert got[1] == alone[1] and np.array_equal(got[0], alone[0])
         assert np.array_equal(got[3], alone[3], equal_nan=True)
+
+
+@pytest.mark.parametrize("n_nodes,k", [(1889, 4), (20_000, 1), (263_169, 4), (420_000, 3)])
+def test_workspace_of_a_frame(n_nodes, k):
+    """The workspace of a frame near the fixed scratch array's size: the buffers' sizes as the descriptor states them,
+    double-float partials of the groups and supergroups, a counter for each, 256-byte aligned."""
+    from d2ic_gb300 import _lib
+    up = lambda x: (x + 255) // 256 * 256
+    groups = (n_nodes + 31) // 32
+    supers = (groups + 15) // 16
+    want = up(56 * n_nodes) + up(16 * k * n_nodes) + up(40 * (groups + supers)) + up(4 * (groups + supers + 1)) + up(4 * n_nodes)
+    assert _lib.load().d2ic_frame_workspace_bytes(n_nodes, n_nodes, k) == want
