@@ -523,9 +523,18 @@ extern "C" int d2ic_zncc_match(const float *ref, int Hr, int Wr, const float *de
     int threads = ((tasks + 31) / 32) * 32;
     threads = threads < 64 ? 64 : (threads > ZNCC_MAX_THREADS ? ZNCC_MAX_THREADS : threads);
     const size_t smem = sizeof(float) * (base + R + 2 * (size_t)ps * npa);
-    // the register-blocked form where its row sums fit in shared memory and its column tasks in the block
-    // (search <= 34 at win 41); the wide form, one offset per thread, beyond
-    if (smem <= 200 * 1024 && npa * ((npa + ZNCC_SEG - 1) / ZNCC_SEG) <= ZNCC_TPT * threads) {
+    // The register-blocked form where its row sums fit in shared memory and its column tasks in the block
+    // (search <= 34 at win 41); the wide form, one offset per thread, beyond, and where there is too little to do
+    // for the blocked form's running sums: below 24,000 pixels x offsets per centre (10,000 centres, win 11: search 4
+    // 64 us wide, 129 us blocked; search 6 124 and 149; search 8 203 and 153), or, with fewer centres than SMs,
+    // below 300,000 (49 centres, win 21: search 6 27 and 32 us, win 31: search 8 40 and 44, search 12 54 and 41).
+    int dev = 0, sms = 0;
+    cudaError_t de = cudaGetDevice(&dev);
+    if (de == cudaSuccess) de = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (de != cudaSuccess) return cuda_status(de, "d2ic_zncc_match");
+    const long long work = (long long)npa * npa * win * win;
+    const bool little = work < 24000 || (n_centers <= sms && work < 300000);
+    if (!little && smem <= 200 * 1024 && npa * ((npa + ZNCC_SEG - 1) / ZNCC_SEG) <= ZNCC_TPT * threads) {
         auto launch = [&](auto kernel) {
             if (smem > 48 * 1024) {
                 cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -61,3 +61,19 @@ def test_flat_bright_and_missing_pixels(cuda):
     img2[60, 100] = np.nan
     far = np.array([[30, 60], [40, 40]], np.float32)
     assert np.array_equal(_match(ref, img2, far, 11, 9, cuda)[0], match_centers(far, ref, img2, 11, 9)[0])
+
+
+@pytest.mark.parametrize("win,search", [(11, 6), (11, 7), (17, 8), (21, 5), (15, 9), (9, 20), (31, 3)])
+def test_many_centres(cuda, win, search):
+    """More centres than SMs: the blocked form at its small sizes and the line to the wide one."""
+    from oracle.init_motion import match_centers
+    rng = np.random.default_rng(win + search)
+    size = 150
+    ref = (120 + 60 * rng.standard_normal((size, size + 3))).astype(np.float32)
+    img = np.roll(ref, (2, -1), (0, 1)) + rng.normal(0, 3, ref.shape).astype(np.float32)
+    centres = np.stack([rng.uniform(0, size + 3, 200), rng.uniform(0, size, 200)], axis=1).astype(np.float32)
+    u, s = _match(ref, img, centres, win, search, cuda)
+    u64, s64 = match_centers(centres, ref, img, win, search)
+    assert np.array_equal(np.isnan(s), np.isnan(s64))
+    ok = ~np.isnan(s64)
+    assert ok.any() and np.array_equal(u, u64) and np.abs(s[ok] - s64[ok]).max() <= SCORE_TOL
