@@ -62,7 +62,8 @@ def test_mixed_transpose(cuda, element, K, shift):
         assert abs(a - b) <= 2e-5 * scale
 
 
-@pytest.mark.parametrize("element,K,spread", [(8, 1, 0.2), (13, 9, 0.2), (16, 33, 0.2), (24, 12, 0.2), (16, 6, 8.0)])
+@pytest.mark.parametrize("element,K,spread", [(8, 1, 0.2), (13, 9, 0.2), (16, 33, 0.2), (24, 17, 0.2), (16, 40, 8.0),
+                                              (12, 16, 0.2)])
 def test_mixed_batch_matches_single_images_and_fp64(cuda, element, K, spread):
     """Image counts around the images a warp and a block take at a time, coefficients that cannot be copied 16 bytes
     at a time, windows that do not fit: the same bits as one image per call, and the FP64 oracle."""
