@@ -206,18 +206,6 @@ __device__ __forceinline__ DF df_reduce5(const DF q[5], int lane) {
     return df_add(v, df_shfl_xor(v, 1));
 }
 
-// Control data is rewritten by other blocks during the launch: read it through
-// L2 (never a possibly stale L1 line).
-__device__ __forceinline__ FrameState load_fs(const FrameState *p) {
-    static_assert(sizeof(FrameState) % 8 == 0, "FrameState size");
-    FrameState s;
-    const unsigned long long *src = reinterpret_cast<const unsigned long long *>(p);
-    unsigned long long *dst = reinterpret_cast<unsigned long long *>(&s);
-#pragma unroll
-    for (int i = 0; i < (int)(sizeof(FrameState) / 8); ++i) dst[i] = __ldcg(src + i);
-    return s;
-}
-
 // node buffers of a frame: 0,1 = u ; 2,3,4 = g ; 5,6 = d
 __device__ __forceinline__ float2 *nbuf(const d2ic_frame_t &F, int j) {
     return reinterpret_cast<float2 *>(F.node_ws) + (size_t)j * F.n_nodes;
@@ -243,7 +231,7 @@ __device__ __forceinline__ float2 cand_value(float2 un, float2 gn, float2 dn, fl
 }
 
 // The candidate rule of a frame for the current round, read from its state
-// with L2 loads (not volatile) so that the reads are in flight together.
+// with L2 loads (rewritten by other blocks; not volatile, so that the reads are in flight together).
 struct FInfo {
     float alpha, beta;
     int mode, iu, igc, idp, igt;
@@ -326,10 +314,6 @@ __device__ __forceinline__ Cand make_cand(const d2ic_frame_t &F, const FInfo &fi
     c.beta = fi.beta;
     c.mode = fi.mode;
     return c;
-}
-
-__device__ __forceinline__ Cand make_cand(const d2ic_frame_t &F, const FrameState *S) {
-    return make_cand(F, frame_info(S));
 }
 
 // ---------------------------------------------------------------------------
