@@ -34,7 +34,7 @@
 // it took 17.9 us on a 512 x 512 frame with 16-px elements, 23.5 us at
 // 1024 x 1024 and 41.1 us at 2048 x 2048; with tagged records, rolled and
 // smaller once-per-round code and even shares of the chunks 11.6, 14.0 and
-// 31.4 us, and with the pixel pass below 9.9, 13.9 and 27.0 us.  What bounds it now: the L2 round trips of the hand-overs (about
+// 31.4 us, and with the pixel pass below 10.1, 14.0 and 27.0 us.  What bounds it now: the L2 round trips of the hand-overs (about
 // 0.7 us each), the fences that order the node data (0.4 us each) and, from
 // 2048 x 2048 on, the pixel pass.
 //
@@ -414,8 +414,8 @@ __device__ __forceinline__ int checked_index(int v, int n, CtlHeader *H) {
 // With the per-chunk work done by the whole warp and scalar pixel arithmetic a
 // 256-pixel chunk took about 2,000 issue slots, 650 of them besides the pixels, and
 // the pass ran at 92 % of the issue rate.  Lane batches and two pixels per
-// instruction leave about 1,150: per evaluation 31.4 -> 27.0 us at 2048 x 2048 with
-// 16-px elements, 62.7 -> 40.3 us with 8-px elements, 219 -> 149 us at 4096 x 4096
+// instruction leave about 1,150: per evaluation 31.4 -> 27.4 us at 2048 x 2048 with
+// 16-px elements, 62.7 -> 40.5 us with 8-px elements, 219 -> 149 us at 4096 x 4096
 // with 8-px elements.  A pass without the coefficient tiles' traffic takes 0.5 us
 // less at 2048 x 2048: what bounds it now is the FMA pipe (60 % busy during the pass)
 // with 4 warps per scheduler to hide its latencies, not the L2.
@@ -592,8 +592,7 @@ __device__ __forceinline__ void chunk_compute(const d2ic_frame_t &F, const Chunk
     float jr = 0.f;
     float gxa[4] = {0.f, 0.f, 0.f, 0.f}, gya[4] = {0.f, 0.f, 0.f, 0.f};
     // fast path, two pixels per lane and step (p and p + 32): the arithmetic of `one`, in packed operations
-    // (174 instead of about 330 issue slots per step; one pixel per lane and instruction: 2 us more per
-    // evaluation at 2048 x 2048).
+    // (about 180 instead of 330 issue slots per step).
     // floor(d) is d + 1.5 * 2^23 rounded down, less 1.5 * 2^23 (exact: here |d| < 2^16), whose low bits are the
     // integer for the tap index; the index is limited to the tile only as a guard of the shared-memory
     // bounds (it is already inside).
