@@ -124,6 +124,8 @@ __global__ void strain_geom_kernel(const double *__restrict__ u, const double2 *
     o[7] = 1.0 + G11;
 }
 
+// WIDE: du starts on a 16-byte boundary and a direction's value at a node is one load; else it is two.
+template <bool WIDE>
 __global__ void strain_jvp_kernel(const double *__restrict__ du, int K, const double2 *__restrict__ X,
                                   const int *__restrict__ idx, const int *__restrict__ deg, int n, int md,
                                   const double *__restrict__ work, const double *__restrict__ wk,
@@ -131,14 +133,17 @@ __global__ void strain_jvp_kernel(const double *__restrict__ du, int K, const do
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int k0 = blockIdx.y * JD, nk = min(JD, K - k0);
     if (i >= n) return;
-    const double2 *v = reinterpret_cast<const double2 *>(du) + (size_t)k0 * n;
+    const double *v = du + 2 * (size_t)k0 * n;
+    auto at = [&](size_t e) {
+        return WIDE ? __ldg(reinterpret_cast<const double2 *>(v) + e) : make_double2(__ldg(v + 2 * e), __ldg(v + 2 * e + 1));
+    };
     const double2 xi = X[i];
     const int d = min(deg[i], md);
     double2 vi[JD];
     double b00[JD], b01[JD], b10[JD], b11[JD];
 #pragma unroll
     for (int q = 0; q < JD; ++q) {
-        vi[q] = q < nk ? v[(size_t)q * n + i] : make_double2(0.0, 0.0);
+        vi[q] = q < nk ? at((size_t)q * n + i) : make_double2(0.0, 0.0);
         b00[q] = b01[q] = b10[q] = b11[q] = 0.0;
     }
     for (int k = 0; k < d; ++k) {
@@ -148,7 +153,7 @@ __global__ void strain_jvp_kernel(const double *__restrict__ du, int K, const do
         const double wx = w * (X[j].x - xi.x), wy = w * (X[j].y - xi.y);
         double2 vj[JD];
 #pragma unroll
-        for (int q = 0; q < JD; ++q) vj[q] = q < nk ? v[(size_t)q * n + j] : vi[q];
+        for (int q = 0; q < JD; ++q) vj[q] = q < nk ? at((size_t)q * n + j) : vi[q];
 #pragma unroll
         for (int q = 0; q < JD; ++q) {
             const double dvx = vj[q].x - vi[q].x, dvy = vj[q].y - vi[q].y;
@@ -205,9 +210,10 @@ extern "C" int d2ic_strain_gl_jvp(const double *u, const double *du, int K, cons
     strain_geom_kernel<<<(n_nodes + STRAIN_T - 1) / STRAIN_T, STRAIN_T, 0, s>>>(
         u, (const double2 *)nodes, nbr_index, nbr_degree, n_nodes, max_deg, gauge_il2(gauge_length), eps, work, wk);
     D2IC_CHECK_LAUNCH("strain_geom_kernel");
-    strain_jvp_kernel<<<dim3((n_nodes + 127) / 128, (K + JD - 1) / JD), 128, 0, s>>>(du, K, (const double2 *)nodes, nbr_index,
-                                                                     nbr_degree, n_nodes, max_deg, work, wk,
-                                                                     dvoigt_out);
+    auto kernel = ((uintptr_t)du & 15) == 0 ? strain_jvp_kernel<true> : strain_jvp_kernel<false>;
+    kernel<<<dim3((n_nodes + 127) / 128, (K + JD - 1) / JD), 128, 0, s>>>(du, K, (const double2 *)nodes, nbr_index,
+                                                                         nbr_degree, n_nodes, max_deg, work, wk,
+                                                                         dvoigt_out);
     D2IC_CHECK_LAUNCH("strain_jvp_kernel");
     return D2IC_OK;
 }
