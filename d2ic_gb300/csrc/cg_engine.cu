@@ -131,6 +131,7 @@ struct Ctl {
     int *gpre;     // two copies of n_frames + 1
     FrameState *fs;
     uint4 *rule;   // n_frames: candidate rule of the next round, as a tagged record (direct rounds)
+    unsigned *tag0;   // n_frames: tag of the evaluation of the launch's first round, constant while it runs
     int n;         // n_frames
     __device__ __forceinline__ int *act(int b) const { return active + b * n; }
     __device__ __forceinline__ int *cp(int b) const { return cpre + b * (n + 1); }
@@ -139,9 +140,9 @@ struct Ctl {
 
 __host__ __device__ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// control block: header | cmd | active | cpre | gpre | frame states | rule records
+// control block: header | cmd | active | cpre | gpre | frame states | rule records | first tags
 __host__ __device__ inline size_t ctl_layout(int n, size_t *o_active, size_t *o_cpre, size_t *o_gpre, size_t *o_fs,
-                                             size_t *o_rule) {
+                                             size_t *o_rule, size_t *o_tag) {
     size_t off = align256(sizeof(CtlHeader));
     off = align256(off + sizeof(int) * (size_t)n);          // cmd
     *o_active = off;                                        // two copies of each list array
@@ -153,13 +154,15 @@ __host__ __device__ inline size_t ctl_layout(int n, size_t *o_active, size_t *o_
     *o_fs = off;
     off = (off + sizeof(FrameState) * (size_t)n + 15) & ~(size_t)15;
     *o_rule = off;
-    off = align256(off + sizeof(uint4) * (size_t)n);
+    off += sizeof(uint4) * (size_t)n;
+    *o_tag = off;
+    off = align256(off + sizeof(unsigned) * (size_t)n);
     return off;
 }
 
 __device__ inline Ctl make_ctl(char *base, int n) {
-    size_t oa, oc, og, of, orl;
-    ctl_layout(n, &oa, &oc, &og, &of, &orl);
+    size_t oa, oc, og, of, orl, ot;
+    ctl_layout(n, &oa, &oc, &og, &of, &orl, &ot);
     Ctl c;
     c.h = (CtlHeader *)base;
     c.cmd = (int *)(base + align256(sizeof(CtlHeader)));
@@ -169,6 +172,7 @@ __device__ inline Ctl make_ctl(char *base, int n) {
     c.n = n;
     c.fs = (FrameState *)(base + of);
     c.rule = (uint4 *)(base + orl);
+    c.tag0 = (unsigned *)(base + ot);
     return c;
 }
 
@@ -238,7 +242,16 @@ struct FInfo {
     unsigned tag;   // this evaluation's tag: the frame's evaluations so far, plus one (28 bits used)
 };
 constexpr unsigned TAG_MASK = 0x0fffffffu;
-__device__ __forceinline__ FInfo frame_info(const FrameState *S) {
+// Every active frame takes one evaluation per round, so its tag is that of the launch's first round plus the
+// rounds completed.  It is not read from the state: a block that has no work of the frame waits for none of the
+// frame's control steps and may read a state that is already an evaluation ahead.  The rest of such a rule is
+// never used (a list in which the block has work of the frame is followed by another read), a tag kept from it
+// would stay wrong.
+__device__ __forceinline__ unsigned frame_tag(const Ctl &C, int f, int rounds) {
+    return (__ldcg(C.tag0 + f) + (unsigned)rounds) & TAG_MASK;
+}
+__device__ __forceinline__ FInfo frame_info(const Ctl &C, int f, int rounds) {
+    const FrameState *S = C.fs + f;
     FInfo fi;
     fi.iu = __ldcg(&S->iu);
     fi.igc = __ldcg(&S->igc);
@@ -248,7 +261,7 @@ __device__ __forceinline__ FInfo frame_info(const FrameState *S) {
     fi.alpha = __ldcg(&S->alpha);
     fi.beta = __ldcg(&S->beta);
     fi.mode = (st == ST_EVAL) ? 0 : ((rs || k == 0) ? 2 : 1);
-    fi.tag = ((unsigned)__ldcg(&S->n_evals) + 1u) & TAG_MASK;
+    fi.tag = frame_tag(C, f, rounds);
     return fi;
 }
 
@@ -1094,6 +1107,7 @@ __device__ void r_init(const d2ic_frame_t *frames, int n_frames, Ctl &C) {
         } else if (ld_vol(&C.fs[f].state) == ST_DONE) {
             C.fs[f].reported = 1;
         }
+        C.tag0[f] = cmd == CMD_INIT ? 1u : ((unsigned)ld_vol(&C.fs[f].n_evals) + 1u) & TAG_MASK;
     }
     __syncthreads();
     rebuild_active(frames, n_frames, C);
@@ -1397,8 +1411,9 @@ __device__ __forceinline__ void control_step(const d2ic_frame_t *frames, const d
 }
 
 // The active list (n_active = na <= FCACHE) with its prefix sums and each frame's candidate
-// rule, copied into the block's shared memory (whole block).
-__device__ __forceinline__ void load_list(Ctl &C, int lb, int na, int *s_cpre, int *s_gpre, int *s_act, FRule *s_fi) {
+// rule after `rounds` completed rounds, copied into the block's shared memory (whole block).
+__device__ __forceinline__ void load_list(Ctl &C, int lb, int na, int rounds, int *s_cpre, int *s_gpre, int *s_act,
+                                          FRule *s_fi) {
     if (na > FCACHE) return;
     for (int s = threadIdx.x; s <= na; s += NT) {
         s_cpre[s] = __ldcg(C.cp(lb) + s);
@@ -1407,7 +1422,7 @@ __device__ __forceinline__ void load_list(Ctl &C, int lb, int na, int *s_cpre, i
     for (int s = threadIdx.x; s < na; s += NT) {
         const int f = checked_index(__ldcg(C.act(lb) + s), C.n, C.h);
         s_act[s] = f;
-        s_fi[s] = make_rule(frame_info(C.fs + f));
+        s_fi[s] = make_rule(frame_info(C, f, rounds));
     }
 }
 
@@ -1469,7 +1484,7 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
     // descriptors of the active frames (na <= FS) without their tensor maps and reserved words
     constexpr int FS_N = ONE ? 1 : FS, FS_WORDS = (FRAME_END - FRAME_BEGIN) / 8;
     __shared__ __align__(16) unsigned long long s_frame[FS_N * FS_WORDS];
-    __shared__ unsigned s_tag0[FS_N];                // direct rounds: a frame's tag less the rounds completed
+    __shared__ unsigned s_tag0[FS_N];                // direct rounds: a frame's tag in the launch's first round
     __shared__ FrameState s_state;                   // ONE: the state in the control step (one warp of the grid)
     __shared__ int2 s_range[NWARP];                  // each warp's chunk range (one active frame)
     __shared__ int s_hdr[10];                         // n_active, total_chunks, total_groups, abort, slice stop,
@@ -1571,11 +1586,11 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
         s_hdr[8] = 0;
     }
     __syncthreads();
-    load_list(C, s_hdr[7], s_hdr[0], s_cpre, s_gpre, s_act, s_fi);
+    load_list(C, s_hdr[7], s_hdr[0], 0, s_cpre, s_gpre, s_act, s_fi);
     __syncthreads();
     if (!ONE && s_hdr[0] <= FS) {
         keep_frames(s_hdr[0]);
-        if ((int)threadIdx.x < s_hdr[0]) s_tag0[threadIdx.x] = s_fi[threadIdx.x].tag;
+        if ((int)threadIdx.x < s_hdr[0]) s_tag0[threadIdx.x] = __ldcg(C.tag0 + s_act[threadIdx.x]);
         __syncthreads();
     }
     if (!ONE) kept = s_hdr[0] <= FS;
@@ -1669,7 +1684,7 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                     w.flags = (unsigned)m.flags;
                     if (lane < cnt) {
                         const d2ic_frame_t &F = frame(m.f);
-                        const FInfo fi = kept ? s_fi[m.f].info() : cached ? s_fi[slot_of(g0 + lane * cs)].info() : frame_info(C.fs + m.f);
+                        const FInfo fi = kept ? s_fi[m.f].info() : cached ? s_fi[slot_of(g0 + lane * cs)].info() : frame_info(C, m.f, round);
                         const Cand cand = make_cand(F, fi);
                         w.tag = fi.tag;
                         const int nd[4] = {m.nd.x, m.nd.y, m.nd.z, m.nd.w};
@@ -1751,7 +1766,7 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                         checked_index(g, 0, C.h);
                         continue;
                     }
-                    const FInfo fi = cached ? s_fi[s].info() : frame_info(C.fs + f);
+                    const FInfo fi = cached ? s_fi[s].info() : frame_info(C, f, round);
                     const NodePre pre = node_pre(F, fi, g * GN + lane);   // independent of the pixel pass
                     SlotSums slots;
                     if (!gather_slots(F, g * GN + lane, __ldg(F.group_need + g), fi.tag, C.h, slots)) break;
@@ -1823,7 +1838,7 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                     }
                 } else if (blockred && cslot < na) {
                     cf = ONE ? 0 : cached ? s_act[cslot] : checked_index(__ldcg(C.act(lb) + cslot), n_frames, C.h);
-                    ctag = cached ? s_fi[cslot].tag : frame_info(C.fs + cf).tag;
+                    ctag = cached ? s_fi[cslot].tag : frame_tag(C, cf, round);
                     cs_slot = cslot;
                     cslot += nw;
                 } else {
@@ -1936,31 +1951,25 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
         if (s_hdr[5] != REFRESH_NONE && !s_hdr[3]) {    // rules from the frame states; a changed list is reloaded
             if (s_hdr[5] == REFRESH_RULES) {
                 if (na <= FCACHE)
-                    for (int s = threadIdx.x; s < na; s += NT) s_fi[s] = make_rule(frame_info(C.fs + s_act[s]));
+                    for (int s = threadIdx.x; s < na; s += NT) s_fi[s] = make_rule(frame_info(C, s_act[s], s_hdr[6]));
             } else if (s_hdr[0] > 0) {
                 // after direct rounds the rules are the records' (the states may still be on their way); the
                 // new list's frames are among the old one's
                 const int n2 = s_hdr[0], t = (int)threadIdx.x;
                 FRule rule{};
-                unsigned tag0 = 0;
-                bool have = false;
-                if (direct && t < n2) {
+                const bool have = direct && t < n2;
+                if (have) {
                     const int f = checked_index(__ldcg(C.act(s_hdr[7]) + t), C.n, C.h);
-                    for (int o = 0; o < na; ++o)
-                        if (s_act[o] == f) {
-                            tag0 = s_tag0[o];
-                            have = true;
-                        }
                     const uint4 r = ld_record(C.rule + f);
-                    rule = FRule{__uint_as_float(r.z), __uint_as_float(r.w), r.y, (tag0 + r.x) & TAG_MASK};
+                    rule = FRule{__uint_as_float(r.z), __uint_as_float(r.w), r.y, frame_tag(C, f, (int)r.x)};
                 }
                 __syncthreads();
-                load_list(C, s_hdr[7], n2, s_cpre, s_gpre, s_act, s_fi);
+                load_list(C, s_hdr[7], n2, s_hdr[6], s_cpre, s_gpre, s_act, s_fi);
                 if (have) s_fi[t] = rule;                // written by this thread in load_list, too
                 __syncthreads();
                 if (!ONE && n2 <= FS) {
                     keep_frames(n2);
-                    if (t < n2) s_tag0[t] = have ? tag0 : s_fi[t].tag - (unsigned)s_hdr[6];
+                    if (t < n2) s_tag0[t] = __ldcg(C.tag0 + s_act[t]);
                     __syncthreads();
                 }
                 if (!ONE) kept = n2 <= FS;
@@ -2108,8 +2117,8 @@ using namespace d2ic;
 
 extern "C" size_t d2ic_cg_control_bytes(int n_frames) {
     if (n_frames < 1) n_frames = 1;
-    size_t a, b, c, d, e;
-    return ctl_layout(n_frames, &a, &b, &c, &d, &e);
+    size_t a, b, c, d, e, t;
+    return ctl_layout(n_frames, &a, &b, &c, &d, &e, &t);
 }
 
 // Workspace of one frame: 7 node buffers (u x2, g x3, dir x2), the K gradient
