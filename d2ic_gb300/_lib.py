@@ -123,6 +123,7 @@ _SIGS = {
     "d2ic_grid_springs": (i32, [vp, vp, i32, vp, vp, vp]),
     "d2ic_structured_assign": (i32, [vp, ctypes.c_longlong, vp, i32, vp, i32, vp, vp, vp]),
     "d2ic_pcg_work_bytes": (szt, [i32, i32, i32]),
+    "d2ic_pcg_plan": (i32, [i32, i32, i32, vp]),
     "d2ic_pcg_solve_op": (i32, [vp, i32, i32, vp, vp, vp, vp, i32, f64, i32, vp, szt, vp, vp]),
     "d2ic_hessian_prepare": (i32, [vp, i32, i32, i32, vp, f32, f32, vp, szt, vp, vp, vp]),
     "d2ic_hessian_check": (i32, [vp, i32, i32, vp]),

@@ -955,7 +955,19 @@ __global__ void pcg_blocks_df(const double *__restrict__ Minv, int n, float2 *__
     M[i] = make_float2(v.hi, v.lo);
 }
 
-// Columns per launch and blocks of pcg_resident; 0 columns: the vectors do not fit on the chip.
+// The most launches of pcg_resident for one solve.  On large meshes few columns fit on the chip at a time, and
+// every launch reads the whole operator each iteration, once for its columns; the form with its vectors in memory
+// reads it once for all.  Per iteration, on the chip (launches) and in memory, in us:
+//     nodes     K = 16           32            48             64             96             128            256
+//     131,044   123 (4) 608   239 (8) 637   358 (12) 712   494 (16) 722   714 (24) 888   953 (32) 1075  1967 (64) 1943
+//     263,169   314 (8) 1209  620 (16) 1248 1005 (24) 1386 1259 (32) 1411 1911 (48) 1738 2684 (64) 2098 4894 (128) 3862
+//     330,625   609 (16) 1518 1212 (32) 1560 1831 (48) 1726 2435 (64) 1749 3653 (96) 2161
+//     580,644  1285 (16) 2612 2567 (32) 2693 3840 (48) 2997 5134 (64) 3046
+// and at 7,569 nodes 23.5 (1) against 75.3 with 64 columns, 167 (8) against 307 with 512.
+constexpr int PR_LAUNCHES = 32;
+
+// Columns per launch and blocks of pcg_resident; 0 columns: the vectors do not fit on the chip, or its launches
+// are too many.
 struct PrPlan {
     int cols, blocks, staged;
     size_t smem;
@@ -967,7 +979,7 @@ static PrPlan pr_plan(int n_nodes, int K, int sms) {
     int cols = K < PR_COLS ? K : PR_COLS;
     const long long per_all = (n_nodes + sms - 1) / sms;      // nodes per block on the whole chip
     if (per_all * cols > pairs_max) cols = (int)(pairs_max / per_all);
-    if (cols < 1) return p;
+    if (cols < 1 || (K + cols - 1) / cols > PR_LAUNCHES) return p;
     const long long pairs = (long long)n_nodes * cols;
     // one block where it fits (no grid hops); else blocks of at least a pair per thread
     long long blocks = pairs <= PR_ONE_BLOCK ? 1 : (pairs + PR_T - 1) / PR_T;
@@ -1135,6 +1147,12 @@ extern "C" size_t d2ic_pcg_work_bytes(int n_nodes, int K, int node_chunk_k) {
     return a > b ? a : b;
 }
 
+extern "C" int d2ic_pcg_plan(int n_nodes, int K, int num_sms, int *blocks) {
+    const PrPlan p = n_nodes >= 1 && K >= 1 ? pr_plan(n_nodes, K, num_sms < 1024 ? num_sms : 1024) : PrPlan{0, 0, 0, 0};
+    if (blocks) *blocks = p.blocks;
+    return p.cols;
+}
+
 // op: an assembled operator, or null: assembled from chunk_hess into the work buffer first
 static int pcg_solve(const d2ic_frame_t *frame_dev, int n_chunks, int n_nodes, int node_chunk_k,
                      const float *chunk_hess, float inv_np, float alpha_reg, const void *op, const double *Minv,
@@ -1157,7 +1175,8 @@ static int pcg_solve(const d2ic_frame_t *frame_dev, int n_chunks, int n_nodes, i
     if (de == cudaSuccess) de = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
     if (de != cudaSuccess) return cuda_status(de, "d2ic_pcg_solve: device attributes");
     const PrPlan plan = pr_plan(n_nodes, K, sms < 1024 ? sms : 1024);
-    // the vectors on the chip wherever a column of them fits (547,000 nodes on 152 SMs), else in memory
+    // the vectors on the chip where a column of them fits (547,000 nodes on 152 SMs) and few launches take all
+    // columns (pr_plan), else in memory
     if (plan.cols > 0 && coop && (size_t)PR_BYTES + sizeof(PrShared) <= (size_t)smem) {
         PrWork r;
         pr_carve(n_nodes, K, node_chunk_k, (char *)work, &r);
