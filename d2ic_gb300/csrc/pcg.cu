@@ -141,21 +141,39 @@ __global__ void __launch_bounds__(256) hop_merge(const d2ic_frame_t *__restrict_
 }
 
 // The block-Jacobi preconditioner: the inverse of each node's diagonal block (FP64, row-major 2x2), zero
-// and inactive where the node has no block or one without a positive determinant.
-__global__ void hop_diagonal(const int *__restrict__ idx, const float4 *__restrict__ blk, int n_nodes,
-                             double *__restrict__ Minv, unsigned char *__restrict__ active) {
+// and inactive where the node has no block or one without a positive determinant.  One thread per node sums
+// the block in FP64 from the node's slots and springs: the operator's merged block is an FP32 sum, whose
+// rounding decides the sign of the determinant where the image varies along one direction only.  The
+// determinant's products are rounded before the difference, so that equal products cancel to zero.
+__global__ void hop_diagonal(const d2ic_frame_t *__restrict__ fp, const int *__restrict__ sids,
+                             const float4 *__restrict__ sblk, float inv_np, float alpha, double *__restrict__ Minv,
+                             unsigned char *__restrict__ active) {
+    const d2ic_frame_t &F = *fp;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= n_nodes) return;
-    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int q = 0; q < HOP; ++q) {
-        const int j = __ldg(idx + (size_t)n * HOP + q);
-        if (j < 0) break;
-        if (j == n) {
-            b = __ldg(blk + (size_t)n * HOP + q);
-            break;
-        }
+    if (n >= F.n_nodes) return;
+    const size_t Nn = F.n_nodes;
+    double xx = 0.0, xy = 0.0, yy = 0.0;
+    for (int s = 0; s < F.node_chunk_k; ++s) {
+        const size_t e = (size_t)s * Nn + n;
+        const int4 j = __ldg(reinterpret_cast<const int4 *>(sids) + e);   // -1: slot not owned by a chunk
+        const int jj[4] = {j.x, j.y, j.z, j.w};
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+            if (jj[b] == n) {
+                const float4 v = __ldg(sblk + 4 * e + b);
+                xx += (double)(inv_np * v.x);
+                xy += (double)(inv_np * v.y);
+                yy += (double)(inv_np * v.z);
+            }
     }
-    const double xx = b.x, xy = b.y, yy = b.z, det = xx * yy - xy * xy;
+    double w = 0.0;
+    for (int q = 0; q < F.max_deg; ++q) {
+        if (__ldg(F.nbr_index + (size_t)q * Nn + n) < 0) break;
+        w += (double)__ldg(F.nbr_weight + (size_t)q * Nn + n);
+    }
+    xx += (double)alpha * w;
+    yy += (double)alpha * w;
+    const double det = __dsub_rn(__dmul_rn(xx, yy), __dmul_rn(xy, xy));
     const bool on = fabs(xx) + fabs(xy) + fabs(yy) > 0.0 && det > 0.0;
     double *m = Minv + 4 * (size_t)n;
     m[0] = on ? yy / det : 0.0;
@@ -1317,7 +1335,7 @@ extern "C" int d2ic_hessian_prepare(const d2ic_frame_t *frame_dev, int n_chunks,
     HopView hv;
     int st = assemble(frame_dev, n_chunks, n_nodes, node_chunk_k, chunk_hess, inv_np, alpha_reg, (char *)op, s, &hv);
     if (st) return st;
-    hop_diagonal<<<(n_nodes + 127) / 128, 128, 0, s>>>(hv.idx, hv.blk, n_nodes, Minv, active);
+    hop_diagonal<<<(n_nodes + 127) / 128, 128, 0, s>>>(frame_dev, hv.sids, hv.sblk, inv_np, alpha_reg, Minv, active);
     D2IC_CHECK_LAUNCH("hop_diagonal");
     return D2IC_OK;
 }
