@@ -559,8 +559,15 @@ __global__ void __launch_bounds__(PT) pcg_dir(int n_nodes, int K, const double *
 // The vectors and the sums are double-floats (48 bits) instead of FP64: GB300 issues an FP64
 // instruction per SM every 16 cycles, so the 12 FP64 operations per vector entry and iteration cost 20 us
 // at 7,396 nodes x 64 columns, the same in double-float 3 us; the product with H is FP32 either way.
-// Columns are scaled by a power of two to a largest entry in [1, 2), so that FP32's exponent range
-// suffices.  Errors against an FP64 solve are those of the FP32 operator, 1.8e-6, as before.
+// Columns are scaled by a power of two to a largest entry in [1, 2), and the preconditioner by the one that
+// halves the exponent of its largest entry, so that FP32's exponent range suffices wherever the FP32 operator's
+// does: with H of size h, P is of size h^-1/2, H P of size h^1/2 and X, kept as h X, of size 1.  (CG with a scaled
+// preconditioner gives the same iterates; powers of two change no bits.)  Errors against CG with FP64 products of the same operator are
+// those of the FP32 products, with these vectors and with FP64 ones: 30 meshes of 330 to 4,212 nodes and 1 to
+// 47 columns, 0.9 to 2.2e-7 of the solution's norm at rtol 1e-7, 0.8 to 1.2e-7 at 1e-10 and at 1e-13, each pair alike to
+// three digits and with the same iteration counts.  (Against FP64 vectors with the same FP32 products the solution
+// differs by 4e-13 to 1e-9 of its norm up to 3,000 nodes; CG amplifies any rounding, in 103 iterations on 22,801 nodes
+// to 1e-8, and FP64 vectors with another order of the sums to 5e-9.)
 //
 // Bound by the hops at few columns (two sums and a barrier, about 6 us) and by the double-float
 // arithmetic and the latency of the neighbours' values at many.  Per iteration, five kernels before ->
@@ -579,7 +586,8 @@ struct PrArgs {
     const int *idx;                        // the operator
     const float4 *blk;
     const int *overflow;                   // the assembly's error flag
-    const float2 *M;                       // inverse diagonal blocks, 4 double-floats per node
+    const double *Minv;                    // inverse diagonal blocks
+    float2 *M;                             // the same, scaled, as 4 double-floats per node (unless staged)
     const unsigned char *act;
     const double *B;
     double *X;
@@ -621,6 +629,7 @@ struct PrShared {
     DF a[PR_COLS], rz[PR_COLS];
     double thr[PR_COLS];
     int scale[PR_COLS];                    // biased FP64 exponent of the column's largest entry
+    int mexp;                              // exponent of the preconditioner's scale
     int stop;                              // a wait ran out somewhere
 };
 extern __shared__ __align__(16) unsigned char pr_dyn[];
@@ -784,7 +793,6 @@ __global__ void __launch_bounds__(PR_T, 1) pcg_resident(const PrArgs A) {
     if (A.staged == 2)
         for (int i = tid; i < nn * HOP; i += PR_T) sblk[i] = __ldg(A.blk + (size_t)n0 * HOP + i);
     if (A.staged) {
-        for (int i = tid; i < nn * 2; i += PR_T) sM[i] = __ldg(reinterpret_cast<const float4 *>(A.M) + 2 * (size_t)n0 + i);
         for (int i = tid; i < nn * HOP; i += PR_T) sidx[i] = A.act[n0 + i / HOP] ? __ldg(A.idx + (size_t)n0 * HOP + i) : -1;
     }
     if (tid == 0) S.stop = 0;
@@ -797,8 +805,9 @@ __global__ void __launch_bounds__(PR_T, 1) pcg_resident(const PrArgs A) {
     auto ld = [](float2 v) { return DF{v.x, v.y}; };
     auto st = [](DF v) { return make_float2(v.hi, v.lo); };
     auto precond = [&](int n, DF r0, DF r1, DF &z0, DF &z1) {
-        const float4 m0 = A.staged ? sM[2 * (n - n0)] : __ldg(reinterpret_cast<const float4 *>(A.M) + 2 * (size_t)n);
-        const float4 m1 = A.staged ? sM[2 * (n - n0) + 1] : __ldg(reinterpret_cast<const float4 *>(A.M) + 2 * (size_t)n + 1);
+        // written by this block: plain loads
+        const float4 m0 = A.staged ? sM[2 * (n - n0)] : reinterpret_cast<const float4 *>(A.M)[2 * (size_t)n];
+        const float4 m1 = A.staged ? sM[2 * (n - n0) + 1] : reinterpret_cast<const float4 *>(A.M)[2 * (size_t)n + 1];
         z0 = df_add(df_mul(DF{m0.x, m0.y}, r0), df_mul(DF{m0.z, m0.w}, r1));
         z1 = df_add(df_mul(DF{m1.x, m1.y}, r0), df_mul(DF{m1.z, m1.w}, r1));
     };
@@ -807,8 +816,10 @@ __global__ void __launch_bounds__(PR_T, 1) pcg_resident(const PrArgs A) {
         o[0] = p0.hi;
         o[Kb] = p1.hi;
     };
-    // the columns' scales
-    int e = 0;
+    // the columns' scales and the preconditioner's largest entry
+    int e = 0, em = 0;
+    if (tid < T)
+        for (int i = tid; i < 4 * nn; i += T) em = max(em, (__double2hiint(A.Minv[4 * (size_t)n0 + i]) >> 20) & 0x7ff);
     pairs([&](int n, int) {
         const size_t i0 = (size_t)n * 2 * A.K + A.k0 + k;
         if (A.act[n]) {
@@ -816,14 +827,29 @@ __global__ void __launch_bounds__(PR_T, 1) pcg_resident(const PrArgs A) {
             e = max(e, (__double2hiint(A.B[i0 + A.K]) >> 20) & 0x7ff);
         }
     });
-    DF v[2] = {DF{__int_as_float(e), 0.f}, DF{0.f, 0.f}};
-    if (!pr_reduce<1, PrMax>(v, A, S, T, rows, ++tag)) return;
+    DF v[2] = {DF{__int_as_float(e), 0.f}, DF{__int_as_float(em), 0.f}};
+    if (!pr_reduce<2, PrMax>(v, A, S, T, rows, ++tag)) return;
     if (tid < Kb) {
         const int m = __float_as_int(S.tot[tid].hi);
         S.scale[tid] = m == 0 || m == 0x7ff ? 1023 : min(m, 2045);
     }
+    if (tid == 0) {                                      // half of its exponent off the blocks (see above)
+        int m = 0;
+        for (int i = 0; i < Kb; ++i) m = max(m, __float_as_int(S.tot[Kb + i].hi));
+        S.mexp = m == 0 || m == 0x7ff ? 0 : -min(max((m - 1023) / 2, -100), 100);
+    }
+    __syncthreads();
+    {
+        const double by = __hiloint2double((1023 + S.mexp) << 20, 0);
+        float2 *M = A.staged ? reinterpret_cast<float2 *>(sM) : A.M + 4 * (size_t)n0;
+        for (int i = tid; i < 4 * nn; i += PR_T) {
+            const DF m = df_from(A.Minv[4 * (size_t)n0 + i] * by);
+            M[i] = make_float2(m.hi, m.lo);
+        }
+    }
     __syncthreads();
     const double up = __hiloint2double(min(max(2046 - S.scale[k], 1), 2046) << 20, 0);   // 2^(1023 - scale)
+    const float ms = __int_as_float((127 + S.mexp) << 23);   // the preconditioner's scale
     // X = 0, R = B, Z = M R, P = Z
     v[0] = v[1] = DF{0.f, 0.f};
     pairs([&](int n, int i) {
@@ -919,11 +945,11 @@ __global__ void __launch_bounds__(PR_T, 1) pcg_resident(const PrArgs A) {
         if (tid < Kb) S.a[tid] = S.tot[tid].hi > 0.f ? df_div(S.rz[tid], S.tot[tid]) : DF{0.f, 0.f};
         __syncthreads();
         // X += a P, R -= a AP, R.R and R.Z
-        const DF a = S.a[k];
+        const DF a = S.a[k], ax = {a.hi * ms * ms, a.lo * ms * ms};
         v[0] = v[1] = DF{0.f, 0.f};
         pairs([&](int n, int i) {
-            x[i] = st(df_add(ld(x[i]), df_mul(a, ld(p[i]))));
-            x[cap + i] = st(df_add(ld(x[cap + i]), df_mul(a, ld(p[cap + i]))));
+            x[i] = st(df_add(ld(x[i]), df_mul(ax, ld(p[i]))));
+            x[cap + i] = st(df_add(ld(x[cap + i]), df_mul(ax, ld(p[cap + i]))));
             const DF r0 = df_add(ld(r[i]), df_neg(df_mul_f(a, ap[i])));
             const DF r1 = df_add(ld(r[cap + i]), df_neg(df_mul_f(a, ap[cap + i])));
             r[i] = st(r0);
@@ -956,21 +982,14 @@ __global__ void __launch_bounds__(PR_T, 1) pcg_resident(const PrArgs A) {
         });
         if (!pr_barrier(A, S, ++phase)) return;
     }
-    const double down = __hiloint2double(S.scale[k] << 20, 0);   // 2^(scale - 1023)
+    // 2^(scale - 1023) and the square of the preconditioner's scale
+    const double down = __hiloint2double(S.scale[k] << 20, 0), msq = __hiloint2double((1023 - 2 * S.mexp) << 20, 0);
     pairs([&](int n, int i) {
         const size_t i0 = (size_t)n * 2 * A.K + A.k0 + k;
-        A.X[i0] = df_to_double(ld(x[i])) * down;
-        A.X[i0 + A.K] = df_to_double(ld(x[cap + i])) * down;
+        A.X[i0] = df_to_double(ld(x[i])) * msq * down;
+        A.X[i0 + A.K] = df_to_double(ld(x[cap + i])) * msq * down;
     });
     if (blockIdx.x == 0 && tid == 0) atomicMax(A.out, it);
-}
-
-// the inverse diagonal blocks as double-floats
-__global__ void pcg_blocks_df(const double *__restrict__ Minv, int n, float2 *__restrict__ M) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const DF v = df_from(Minv[i]);
-    M[i] = make_float2(v.hi, v.lo);
 }
 
 // The most launches of pcg_resident for one solve.  On large meshes few columns fit on the chip at a time, and
@@ -1200,8 +1219,6 @@ static int pcg_solve(const d2ic_frame_t *frame_dev, int n_chunks, int n_nodes, i
         pr_carve(n_nodes, K, node_chunk_k, (char *)work, &r);
         int st = get_operator(r.op, s, &hv);
         if (st) return st;
-        pcg_blocks_df<<<(unsigned)((4 * (size_t)n_nodes + 255) / 256), 256, 0, s>>>(Minv, 4 * n_nodes, r.M);
-        D2IC_CHECK_LAUNCH("pcg_blocks_df");
         cudaError_t e = cudaMemsetAsync(r.out, 0, 2 * sizeof(int), s);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(pcg_resident, cudaFuncAttributeMaxDynamicSharedMemorySize, PR_BYTES);
@@ -1211,6 +1228,7 @@ static int pcg_solve(const d2ic_frame_t *frame_dev, int n_chunks, int n_nodes, i
             A.idx = hv.idx;
             A.blk = hv.blk;
             A.overflow = hv.err;
+            A.Minv = Minv;
             A.M = r.M;
             A.act = active;
             A.B = B;
