@@ -12,13 +12,15 @@
 //   * the products are a register-blocked correlation: a thread makes
 //     2 x R offsets (two rows of R), and per template value reads two patch
 //     values and one template value from shared memory for 2 R multiply-adds;
-//   * the two sums come from separable running sums in double-float, so that
-//     v = sum d^2 - (sum d)^2 / n is exact to FP32 (rows are rounded to FP32
-//     once, 6e-8 relative).
-// A window whose mean lies more than 8 standard deviations from c would lose
-// digits in v; it is scored by the two-pass form (mean first, then centred
-// sums), as is every window of a patch with values that are not finite or
-// beyond 1e15.
+//   * the two sums come from separable running sums in double-float, rounded to
+//     FP32 once per row; v = sum d^2 - (sum d)^2 / n in double-float.
+// With s = sum d^2 / v = 1 + (mean - c)^2 / variance of a window, the rows' rounding is amplified s-fold in v and
+// the rounding of sum d t sqrt(s)-fold; the two-pass form (mean first, then centred sums, one after the other in
+// FP32) has errors that grow with the window.  Simulated RMS errors of the score, correlations 0.3 and 0.99, against
+// those of the two-pass form: win 5 1.0 at s = 2, 1.3 at 5; win 11 0.95 at 5, 1.2 at 10; win 21 0.9 at 10, 1.2 at 37;
+// win 41 0.9 at 17, 1.0 at 62.  Windows with s above 0.15 win^1.5 (or 65) are therefore scored in two passes, by a
+// thread each, or by a warp each where they are few; so is every window of a patch with values that are not finite
+// or beyond 1e15.
 //
 // Bound by FP32 issue and shared-memory reads.  9,216 centres at win 41,
 // search 24 (2401 offsets x 1681 pixels): 14.2 ms with one offset per thread in
@@ -45,6 +47,64 @@ __device__ __forceinline__ float zncc_two_pass(const float *w0, int ps, const fl
             cr += d * tpl[i * win + j];
         }
     return cr / (sqrtf(v / n) + 1e-12f) / n;
+}
+
+// the same by a whole warp
+__device__ __forceinline__ float zncc_two_pass_warp(const float *w0, int ps, const float *tpl, int win, int lane) {
+    const int n = win * win;
+    auto pixels = [&](auto &&f) {
+        for (int p = lane, r = 0, q = lane; p < n; p += 32, q += 32) {
+            while (q >= win) {
+                q -= win;
+                ++r;
+            }
+            f(w0[r * ps + q], p);
+        }
+    };
+    float s = 0.f;
+    pixels([&](float d, int) { s += d; });
+    const float mw = warp_sum_f(s) / (float)n;
+    float v = 0.f, cr = 0.f;
+    pixels([&](float x, int p) {
+        const float d = x - mw;
+        v += d * d;
+        cr += d * tpl[p];
+    });
+    v = warp_sum_f(v);
+    return warp_sum_f(cr) / (sqrtf(v / (float)n) + 1e-12f) / (float)n;
+}
+
+// The offsets of a block with var < 0, in two passes: listed over the means, then a warp each where they are fewer than
+// the warps times the steps that a warp saves, else a thread each.  Updates the thread's best score and its
+// offset.  (Out of line: inlined, it changes how the correlation is compiled, 6 % of the whole at win 41.)
+__device__ __noinline__ void zncc_left_over(const float *pat, int ps, const float *tpl, int win, int npa, const float *var,
+                                            int *list, int *count, float &best, int &bidx) {
+    const int n = win * win, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    auto better = [&](float sc, int o) {                   // not visited in order
+        if (sc > best || (sc == best && o < bidx)) {
+            best = sc;
+            bidx = o;
+        }
+    };
+    __syncthreads();                                       // every thread has read its means
+    if (threadIdx.x == 0) *count = 0;
+    __syncthreads();
+    for (int o = threadIdx.x; o < npa * npa; o += blockDim.x)
+        if (var[o] < 0.f) list[atomicAdd(count, 1)] = o;
+    __syncthreads();
+    const int left = *count;
+    if ((long long)left * 64 <= (long long)nw * n) {
+        for (int i = wid; i < left; i += nw) {
+            const int o = list[i];
+            const float sc = zncc_two_pass_warp(pat + (o / npa) * ps + o % npa, ps, tpl, win, lane);
+            if (lane == 0) better(sc, o);
+        }
+    } else {
+        for (int i = threadIdx.x; i < left; i += blockDim.x) {
+            const int o = list[i];
+            better(zncc_two_pass(pat + (o / npa) * ps + o % npa, ps, tpl, win), o);
+        }
+    }
 }
 
 // a float added to a double-float whose low word collects the rounding errors
@@ -162,6 +222,7 @@ __global__ void __launch_bounds__(ZNCC_MAX_THREADS) zncc_kernel(const float *__r
         if ((int)threadIdx.x < R) pat[ps * ps + threadIdx.x] = 0.f;
         __syncthreads();
         const int segs = (npa + ZNCC_SEG - 1) / ZNCC_SEG;
+        const float most = fminf(0.15f * (float)win * sqrtf((float)win), 65.f);   // of sum d^2 / v
         // rows: sums over win columns (a thread: one row, ZNCC_SEG columns; neighbouring threads take
         // neighbouring rows)
         for (int t = threadIdx.x; t < 2 * ps * segs; t += blockDim.x) {
@@ -185,6 +246,7 @@ __global__ void __launch_bounds__(ZNCC_MAX_THREADS) zncc_kernel(const float *__r
         // columns: the window sums, kept in registers until every thread has read its rows (mean and var
         // lie over the rows).  A task is one column, ZNCC_SEG rows; at most ZNCC_TPT per thread.
         float wm[ZNCC_TPT][ZNCC_SEG], wv[ZNCC_TPT][ZNCC_SEG];
+        bool two_pass = false;
 #pragma unroll
         for (int h = 0; h < ZNCC_TPT; ++h) {
             const int task = threadIdx.x + h * blockDim.x, kx = task % npa, ky0 = (task / npa) * ZNCC_SEG;
@@ -203,7 +265,7 @@ __global__ void __launch_bounds__(ZNCC_MAX_THREADS) zncc_kernel(const float *__r
                     const DF d = df_add(s2, DF{-sq.hi, -(sq.lo + m * (lo + rest))});
                     const float v = d.hi + d.lo;
                     wm[h][q] = m;
-                    wv[h][q] = v * 65.f >= s2.hi + s2.lo ? fmaxf(v, 0.f) : -1.f;
+                    wv[h][q] = v * most >= s2.hi + s2.lo ? fmaxf(v, 0.f) : -1.f;
                     if (ky0 + q + 1 < npa && q + 1 < ZNCC_SEG) {
                         df_acc(s1, -row1[(ky0 + q) * npa + kx]);
                         df_acc(s1, row1[(ky0 + q + win) * npa + kx]);
@@ -223,9 +285,10 @@ __global__ void __launch_bounds__(ZNCC_MAX_THREADS) zncc_kernel(const float *__r
                     if (ky0 + q < npa) {
                         mean[(ky0 + q) * npa + kx] = wm[h][q];
                         var[(ky0 + q) * npa + kx] = wv[h][q];
+                        two_pass |= wv[h][q] < 0.f;
                     }
         }
-        __syncthreads();
+        two_pass = __syncthreads_or(two_pass);
         // the correlation: 2 rows x R columns of offsets per thread
         const int nbx = (npa + R - 1) / R, nby = (npa + 1) / 2;
         for (int t = threadIdx.x; t < nbx * nby; t += blockDim.x) {
@@ -248,9 +311,18 @@ __global__ void __launch_bounds__(ZNCC_MAX_THREADS) zncc_kernel(const float *__r
                     for (int o = 0; o < R; ++o) acc[o] = pair_fma(w[(q + o) % R], tv, acc[o]);
                 };
                 int j = 0;
-                for (; j + R <= win; j += R)
+                // R = 7 unrolled takes 4 % more with many centres (9,216 at 41 / 24: 2.16 ms), 3 % less with 625; the
+                // others take 1 to 20 % less unrolled (49 centres at 41 / 12: 49 and 60 us)
+                if constexpr (R == 7) {
+#pragma unroll 1
+                    for (; j + R <= win; j += R)
 #pragma unroll
-                    for (int q = 0; q < R; ++q) column(j + q, q);
+                        for (int q = 0; q < R; ++q) column(j + q, q);
+                } else {
+                    for (; j + R <= win; j += R)
+#pragma unroll
+                        for (int q = 0; q < R; ++q) column(j + q, q);
+                }
 #pragma unroll
                 for (int q = 0; q < R - 1; ++q)             // the last win % R columns
                     if (j + q < win) column(j + q, q);
@@ -263,14 +335,14 @@ __global__ void __launch_bounds__(ZNCC_MAX_THREADS) zncc_kernel(const float *__r
                         if (kx0 + q < npa) {
                             const int o = (ky + h * nby) * npa + kx0 + q;
                             const float v = var[o], cr = (h == 0 ? pair_lo(acc[q]) : pair_hi(acc[q])) - mean[o] * t1;
-                            float sc = cr / (sqrtf(v / (float)n) + 1e-12f) / (float)n;
-                            if (v < 0.f) sc = zncc_two_pass(pat + (ky + h * nby) * ps + kx0 + q, ps, tpl, win);
-                            if (sc > best || (sc == best && o < bidx)) {   // offsets are not visited in order
+                            const float sc = cr / (sqrtf(v / (float)n) + 1e-12f) / (float)n;
+                            if (v >= 0.f && (sc > best || (sc == best && o < bidx))) {   // not visited in order
                                 best = sc;
                                 bidx = o;
                             }
                         }
         }
+        if (two_pass) zncc_left_over(pat, ps, tpl, win, npa, var, reinterpret_cast<int *>(mean), s_idx, best, bidx);
     }
     // block argmax: larger score, then smaller index
 #pragma unroll
@@ -528,13 +600,15 @@ extern "C" int d2ic_zncc_match(const float *ref, int Hr, int Wr, const float *de
     // for the blocked form's running sums: below 24,000 pixels x offsets per centre (10,000 centres, win 11: search 4
     // 64 us wide, 129 us blocked; search 6 124 and 149; search 8 203 and 153), or, with fewer centres than SMs,
     // below 300,000 (49 centres, win 21: search 6 27 and 32 us, win 31: search 8 40 and 44, search 12 54 and 41).
+    // Windows below 9 pixels, most of which go through the two-pass form anyway: wide (speckle, 10,000 centres,
+    // search 24: win 5 469 us wide, 738 us blocked; win 7 660 and 754; win 9 917 and 695).
     int dev = 0, sms = 0;
     cudaError_t de = cudaGetDevice(&dev);
     if (de == cudaSuccess) de = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (de != cudaSuccess) return cuda_status(de, "d2ic_zncc_match");
     const long long work = (long long)npa * npa * win * win;
     const bool little = work < 24000 || (n_centers <= sms && work < 300000);
-    if (!little && smem <= 200 * 1024 && npa * ((npa + ZNCC_SEG - 1) / ZNCC_SEG) <= ZNCC_TPT * threads) {
+    if (win >= 9 && !little && smem <= 200 * 1024 && npa * ((npa + ZNCC_SEG - 1) / ZNCC_SEG) <= ZNCC_TPT * threads) {
         auto launch = [&](auto kernel) {
             if (smem > 48 * 1024) {
                 cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
