@@ -118,6 +118,9 @@ class ImplicitAdjoint:
         return prepare_coefficients(img.to(torch.float32).contiguous(), _lib.INTERP_CUBIC)
 
     MIXED_BATCH = 32   # images per launch of the batched prefilter and mixed term
+    # scratch of mixed_T's fields in one launch: 14 fields of 1024 x 1024, one of 4096 x 4096, whose pixels fill the
+    # chip by themselves
+    MIXED_T_BYTES = 128 << 20
 
     def mixed(self, dI: torch.Tensor) -> torch.Tensor:
         """(d grad_u J / dI2) dI_k for images dI (K, H, W) -> (Nn, 2, K): the images' B-spline
@@ -145,11 +148,13 @@ class ImplicitAdjoint:
         return self._mixed_T(lam, self.inv_np)
 
     def _mixed_T(self, lam: torch.Tensor, scale: float) -> torch.Tensor:
-        """``scale`` times the unscaled adjoint, up to MIXED_BATCH fields per launch."""
+        """``scale`` times the unscaled adjoint, as many fields per launch as MIXED_T_BYTES of scratch hold
+        (one at least, MIXED_BATCH at most)."""
         L = self.L
         K = lam.shape[2]
         out = torch.empty((K, L.H, L.W), dtype=torch.float32, device=self.dev)
-        B = min(self.MIXED_BATCH, max(K, 1))
+        field_bytes = 4 * L.cpitch * (2 * L.H + 2 * PAD)
+        B = max(1, min(self.MIXED_BATCH, K, self.MIXED_T_BYTES // field_bytes))
         gco = torch.empty((B, L.H + 2 * PAD, L.cpitch), dtype=torch.float32, device=self.dev)
         tmp = torch.empty((B, L.H, L.cpitch), dtype=torch.float32, device=self.dev)
         s = _lib.stream_handle()
