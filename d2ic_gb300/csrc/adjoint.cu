@@ -332,6 +332,7 @@ __global__ void __launch_bounds__(32 * MIX_WARPS, 2) mixed_chunks(const d2ic_fra
     if (tiled)
         for (int j = 0; j < per && w * per + j < n_images; ++j)
             load_tile(tiles + j * MIX_TILE, dcoeff + (size_t)(w * per + j) * coeff_stride + origin);
+    bool inside = true;                                        // of the window
     if ((int)threadIdx.x < n) {
         const int i = threadIdx.x;
         const ChunkPix q = unpack(__ldg(reinterpret_cast<const uint4 *>(F.pix) + pb + i));
@@ -346,15 +347,23 @@ __global__ void __launch_bounds__(32 * MIX_WARPS, 2) mixed_chunks(const d2ic_fra
         s_r[i] = sample_cubic(im, ix, iy, tx, ty, gx, gy) - q.I1;
         s_gx[i] = gx;
         s_gy[i] = gy;
-        // tiled: s_ix is the first tap's element of the window, inside it; limited as a guard of the bounds
-        s_ix[i] = tiled ? min(max((iy - 1 + F.pad - y0) * tw + ix - 1 + F.pad - x0, 0), (th - 4) * tw + tw - 4) : ix;
+        const int lx = ix - 1 + F.pad - x0, ly = iy - 1 + F.pad - y0;
+        inside = (unsigned)lx <= (unsigned)(tw - 4) && (unsigned)ly <= (unsigned)(th - 4);
+        s_ix[i] = tiled ? ly * tw + lx : ix;                   // tiled: the first tap's element of the window
         s_iy[i] = iy;
         s_tx[i] = tx;
         s_ty[i] = ty;
 #pragma unroll
         for (int a = 0; a < 4; ++a) s_N[a][i] = q.N[a];
     }
-    __syncthreads();
+    // every pixel of an element lies inside; one beyond it (a caller's own shape functions) may not: global memory
+    if (!__syncthreads_and(inside) && tiled) {
+        tiled = false;
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        const int i = threadIdx.x;
+        if (i < n) s_ix[i] += x0 + 1 - F.pad - (s_iy[i] - 1 + F.pad - y0) * tw;
+        __syncthreads();
+    }
     for (int b0 = w * per; b0 < n_images; b0 += MIX_WARPS * per) {
         const int nb = min(per, n_images - b0);
         float v[8 * MIX];                            // node sums: image j's x of node a at 8 j + 2 a, its y after it

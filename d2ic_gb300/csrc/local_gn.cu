@@ -131,7 +131,6 @@ __global__ void __launch_bounds__(32 * LGN_WARPS, 2) lgn_chunks_kernel(const d2i
                 __syncwarp();
             }
         }
-        const int limit = (th - 4) * tw + tw - 4;
         float acc[4][5];
 #pragma unroll
         for (int a = 0; a < 4; ++a)
@@ -154,9 +153,10 @@ __global__ void __launch_bounds__(32 * LGN_WARPS, 2) lgn_chunks_kernel(const d2i
             split_coord(x, dx, ix, tx);
             split_coord(y, dy, iy, ty);
             float r, gx, gy;
-            if (KIND == D2IC_INTERP_CUBIC && tiled) {
-                // already inside the window; limited to it as a guard of the shared-memory bounds
-                const int at = min(max((iy - 1 - y0) * tw + ix - 1 - x0, 0), limit);
+            const int lx = ix - 1 - x0, ly = iy - 1 - y0;
+            // inside for any pixel of its element; a pixel beyond it (a caller's own shape functions) may lie outside
+            if (KIND == D2IC_INTERP_CUBIC && tiled && (unsigned)lx <= (unsigned)(tw - 4) && (unsigned)ly <= (unsigned)(th - 4)) {
+                const int at = ly * tw + lx;
                 r = tile_value(tile + at, tw, tx, ty) - I1;
                 gx = tile_value(tile + LGN_TILE + at, tw, tx, ty);
                 gy = tile_value(tile + 2 * LGN_TILE + at, tw, tx, ty);
