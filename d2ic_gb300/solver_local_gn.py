@@ -122,10 +122,10 @@ class LocalGaussNewtonSolver(SolverBase):
         hist = torch.full((max(n_sweeps, 1), 2), float("nan"), dtype=torch.float64, device=dev)
         alpha = float(state.config.reg_strength)
         _lib.call("d2ic_local_gn_run", ptr(self._desc), L.n_pix, L.n_chunks, nn, L.node_chunk_k, L.kind, ptr(self._cgx),
-                  ptr(self._cgy), ptr(u), ptr(v), n_sweeps, ptr(self._slots), ptr(self._r2), ptr(self._has_pix),
+                  ptr(self._cgy), ptr(u), ptr(v), max(n_sweeps, 0), ptr(self._slots), ptr(self._r2), ptr(self._has_pix),
                   ptr(self._nbr), ptr(self._nbw), self._md, ptr(self._rho), self._lam, self._max_step, alpha, self._omega,
                   ptr(self._st), ptr(hist), _lib.stream_handle())
-        if n_sweeps % 2:
+        if n_sweeps > 0 and n_sweeps % 2:
             u = v
         u_host = u.cpu().numpy()
         save_history = bool(getattr(state.config, "save_history", False))
