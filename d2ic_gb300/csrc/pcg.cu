@@ -579,7 +579,10 @@ constexpr int PR_BLOCK_BYTES = 16 * HOP;       // the operator's blocks of a nod
 constexpr int PR_BYTES = 212 * 1024;       // dynamic shared memory per block at most
 constexpr int PR_COLS = 64;                // columns per launch
 constexpr int PR_POLL = 5;                 // records a lane polls at a time: 160 blocks in one round trip
-constexpr int PR_ONE_BLOCK = 2048;         // systems of at most this many pairs run in one block
+// Systems of at most two pairs per thread run in one block: no grid hops, but every pair of a thread adds to the
+// iteration.  One block and several, us per iteration: 529 nodes x 1 column 8.7 and 9.2, 1,024 x 1 11.2 and 11.1,
+// 2,025 x 1 20.9 and 11.3; 256 x 6 9.9 and 8.9, 400 x 6 13.7 and 8.7; 25 x 64 8.1 and 8.5, 49 x 64 12.9 and 9.4.
+constexpr int PR_ONE_BLOCK = 2 * PR_T;
 constexpr unsigned long long PR_WAIT_NS = 5ull * 1000ull * 1000ull * 1000ull;
 
 struct PrArgs {

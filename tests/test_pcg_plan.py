@@ -29,5 +29,10 @@ def test_many_launches_go_to_memory(plan, nodes, columns):
     assert plan(nodes, columns)[0] == 0
 
 
+@pytest.mark.parametrize("nodes,columns,blocks", [(16, 64, 1), (1_024, 1, 1), (1_025, 1, 3), (171, 6, 3), (1_681, 6, 20)])
+def test_one_block_up_to_two_pairs_per_thread(plan, nodes, columns, blocks):
+    assert plan(nodes, columns) == (columns, blocks)
+
+
 def test_arguments_without_a_plan(plan):
     assert plan(100, 1, 0) == (0, 0) and plan(0, 1) == (0, 0) and plan(1, 0) == (0, 0)
