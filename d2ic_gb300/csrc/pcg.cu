@@ -1215,7 +1215,7 @@ static int pcg_solve(const d2ic_frame_t *frame_dev, int n_chunks, int n_nodes, i
     if (de == cudaSuccess) de = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
     if (de != cudaSuccess) return cuda_status(de, "d2ic_pcg_solve: device attributes");
     const PrPlan plan = pr_plan(n_nodes, K, sms < 1024 ? sms : 1024);
-    // the vectors on the chip where a column of them fits (547,000 nodes on 152 SMs) and few launches take all
+    // the vectors on the chip where a column of them fits (589,000 nodes on 152 SMs) and few launches take all
     // columns (pr_plan), else in memory
     if (plan.cols > 0 && coop && (size_t)PR_BYTES + sizeof(PrShared) <= (size_t)smem) {
         PrWork r;

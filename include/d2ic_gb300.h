@@ -179,7 +179,7 @@ D2IC_API size_t d2ic_pcg_work_bytes(int n_nodes, int K, int node_chunk_k);
  * inverse diagonal blocks (zero for inactive dofs), active (n_nodes) 0/1 mask.  Stops when every
  * column of a launch (up to 64 columns) has ||R|| <= rtol ||B|| or after max_iter iterations
  * (*iters_out: the most of any launch).  The vectors stay on the chip as double-floats where a
- * column of them fits (547,000 nodes on 152 SMs) and few launches take all columns (d2ic_pcg_plan), else
+ * column of them fits (589,000 nodes on 152 SMs) and few launches take all columns (d2ic_pcg_plan), else
  * in memory as FP64.  Blocks wait for one another (a cooperative launch): D2IC_WAIT_TIMEOUT if a wait runs
  * out. */
 D2IC_API int d2ic_pcg_solve(const d2ic_frame_t *frame_dev, int n_chunks, int n_nodes, int node_chunk_k,

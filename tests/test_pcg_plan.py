@@ -29,6 +29,12 @@ def test_many_launches_go_to_memory(plan, nodes, columns):
     assert plan(nodes, columns)[0] == 0
 
 
+@pytest.mark.parametrize("nodes,sms,cols", [(589_000, 152, 1), (589_001, 152, 0), (644_809, 152, 0), (3_875, 1, 1), (3_876, 1, 0)])
+def test_a_column_of_the_largest_mesh(plan, nodes, sms, cols):
+    """3,875 pairs of 56 bytes in the shared memory of an SM."""
+    assert plan(nodes, 1, sms)[0] == cols
+
+
 @pytest.mark.parametrize("nodes,columns,blocks", [(16, 64, 1), (1_024, 1, 1), (1_025, 1, 3), (171, 6, 3), (1_681, 6, 20)])
 def test_one_block_up_to_two_pairs_per_thread(plan, nodes, columns, blocks):
     assert plan(nodes, columns) == (columns, blocks)
