@@ -118,9 +118,9 @@ class ImplicitAdjoint:
         return prepare_coefficients(img.to(torch.float32).contiguous(), _lib.INTERP_CUBIC)
 
     MIXED_BATCH = 32   # images per launch of the batched prefilter and mixed term
-    # scratch of mixed_T's fields in one launch: 14 fields of 1024 x 1024, one of 4096 x 4096, whose pixels fill the
-    # chip by themselves
-    MIXED_T_BYTES = 128 << 20
+    # scratch of mixed_T's fields in one launch: 32 fields of 1024 x 1024, 3 of 4096 x 4096 (six fields there take
+    # 3.6 ms one at a time, 2.6 ms together)
+    MIXED_T_BYTES = 512 << 20
 
     def mixed(self, dI: torch.Tensor) -> torch.Tensor:
         """(d grad_u J / dI2) dI_k for images dI (K, H, W) -> (Nn, 2, K): the images' B-spline
@@ -149,14 +149,22 @@ class ImplicitAdjoint:
 
     def _mixed_T(self, lam: torch.Tensor, scale: float) -> torch.Tensor:
         """``scale`` times the unscaled adjoint, as many fields per launch as MIXED_T_BYTES of scratch hold
-        (one at least, MIXED_BATCH at most)."""
+        (one at least, MIXED_BATCH at most; fewer where the device has no room)."""
         L = self.L
         K = lam.shape[2]
         out = torch.empty((K, L.H, L.W), dtype=torch.float32, device=self.dev)
         field_bytes = 4 * L.cpitch * (2 * L.H + 2 * PAD)
         B = max(1, min(self.MIXED_BATCH, K, self.MIXED_T_BYTES // field_bytes))
-        gco = torch.empty((B, L.H + 2 * PAD, L.cpitch), dtype=torch.float32, device=self.dev)
-        tmp = torch.empty((B, L.H, L.cpitch), dtype=torch.float32, device=self.dev)
+        while True:
+            gco = tmp = None
+            try:
+                gco = torch.empty((B, L.H + 2 * PAD, L.cpitch), dtype=torch.float32, device=self.dev)
+                tmp = torch.empty((B, L.H, L.cpitch), dtype=torch.float32, device=self.dev)
+                break
+            except torch.cuda.OutOfMemoryError:
+                if B == 1:
+                    raise
+                B = (B + 1) // 2
         s = _lib.stream_handle()
         for k0 in range(0, K, B):
             nb = min(B, K - k0)

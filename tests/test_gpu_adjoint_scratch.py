@@ -1,4 +1,5 @@
-"""Scratch of the adjoint of the mixed term (GPU): bounded by bytes, whatever the image size and field count."""
+"""Scratch of the adjoint of the mixed term (GPU): bounded by bytes, whatever the image size and field count, and by
+what the device has left."""
 from __future__ import annotations
 
 import pytest
@@ -7,9 +8,9 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("side,K,most", [(2048, 9, 128 << 20), (4300, 2, 152 << 20), (256, 40, 128 << 20)])
+@pytest.mark.parametrize("side,K,most", [(2048, 20, 512 << 20), (4300, 5, 512 << 20), (256, 40, 512 << 20)])
 def test_mixed_transpose_scratch(cuda, side, K, most):
-    """2048: 35 MB a field, 3 per launch; 4300: 151 MB a field, one per launch; 256: 32 fields per launch."""
+    """2048: 35 MB a field, 15 per launch; 4300: 150 MB a field, 3 per launch; 256: 32 fields per launch."""
     from test_gpu_pcg_sizes import _adjoint
     adj = _adjoint(cuda, side, 64)
     g = torch.Generator(device=cuda).manual_seed(side)
@@ -25,3 +26,25 @@ def test_mixed_transpose_scratch(cuda, side, K, most):
     for k in (0, K - 1):
         one = adj.mixed_T(lam[:, :, k:k + 1])[0]
         assert float((out[k] - one).abs().max()) <= 1e-5 * float(one.abs().max())
+
+
+def test_fewer_fields_where_the_device_has_no_room(cuda):
+    """A limit that leaves room for the result and two fields: the call that fits one at a time still runs."""
+    from test_gpu_pcg_sizes import _adjoint
+    side, K = 1500, 16
+    adj = _adjoint(cuda, side, 64)
+    g = torch.Generator(device=cuda).manual_seed(1)
+    lam = torch.randn((adj.L.n_nodes, 2, K), generator=g, device=cuda)
+    want = adj.mixed_T(lam)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    field = 4 * adj.L.cpitch * (2 * side + 64)
+    room = torch.cuda.memory_reserved(cuda) + want.numel() * 4 + 2 * field + (44 << 20)
+    total = torch.cuda.get_device_properties(cuda).total_memory
+    torch.cuda.set_per_process_memory_fraction(room / total, cuda)
+    try:
+        got = adj.mixed_T(lam)
+        torch.cuda.synchronize()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0, cuda)
+    assert float((got - want).abs().max()) <= 1e-5 * float(want.abs().max())
