@@ -37,10 +37,12 @@ __device__ __forceinline__ float zncc_two_pass(const float *w0, int ps, const fl
     const float n = (float)(win * win);
     float s = 0.f;
     for (int i = 0; i < win; ++i)
+#pragma unroll 4
         for (int j = 0; j < win; ++j) s += w0[i * ps + j];
     const float mw = s / n;
     float v = 0.f, cr = 0.f;
     for (int i = 0; i < win; ++i)
+#pragma unroll 4
         for (int j = 0; j < win; ++j) {
             const float d = w0[i * ps + j] - mw;
             v += d * d;
@@ -599,7 +601,10 @@ extern "C" int d2ic_zncc_match(const float *ref, int Hr, int Wr, const float *de
     // (search <= 34 at win 41); the wide form, one offset per thread, beyond, and where there is too little to do
     // for the blocked form's running sums: below 24,000 pixels x offsets per centre (10,000 centres, win 11: search 4
     // 64 us wide, 129 us blocked; search 6 124 and 149; search 8 203 and 153), or, with fewer centres than SMs,
-    // below 300,000 (49 centres, win 21: search 6 27 and 32 us, win 31: search 8 40 and 44, search 12 54 and 41).
+    // below 300,000 (49 centres, win 21: search 6 27 and 32 us, win 31: search 8 40 and 44, search 12 54 and 41); with
+    // windows up to 15 pixels also for more centres, up to 300,000 per SM (speckle, 289 centres: win 11 search 12 27 and
+    // 31 us, win 15 search 10 26 and 32; 625: win 11 search 8 26 and 35, search 10 28 and 37, win 15 search 10 42 and 41;
+    // 1,225: win 11 search 8 34 and 36, search 10 47 and 39).
     // Windows below 9 pixels, most of which go through the two-pass form anyway: wide (speckle, 10,000 centres,
     // search 24: win 5 469 us wide, 738 us blocked; win 7 660 and 754; win 9 917 and 695).
     int dev = 0, sms = 0;
@@ -607,7 +612,8 @@ extern "C" int d2ic_zncc_match(const float *ref, int Hr, int Wr, const float *de
     if (de == cudaSuccess) de = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (de != cudaSuccess) return cuda_status(de, "d2ic_zncc_match");
     const long long work = (long long)npa * npa * win * win;
-    const bool little = work < 24000 || (n_centers <= sms && work < 300000);
+    const bool little =
+        work < 24000 || (work < 300000 && (n_centers <= sms || (win <= 15 && work * n_centers < 300000ll * sms)));
     if (win >= 9 && !little && smem <= 200 * 1024 && npa * ((npa + ZNCC_SEG - 1) / ZNCC_SEG) <= ZNCC_TPT * threads) {
         auto launch = [&](auto kernel) {
             if (smem > 48 * 1024) {
