@@ -131,18 +131,19 @@ struct Ctl {
     int *gpre;     // two copies of n_frames + 1
     FrameState *fs;
     uint4 *rule;   // n_frames: candidate rule of the next round, as a tagged record (direct rounds)
-    unsigned *tag0;   // n_frames: tag of the evaluation of the launch's first round, constant while it runs
     int n;         // n_frames
     __device__ __forceinline__ int *act(int b) const { return active + b * n; }
     __device__ __forceinline__ int *cp(int b) const { return cpre + b * (n + 1); }
     __device__ __forceinline__ int *gp(int b) const { return gpre + b * (n + 1); }
+    // n_frames: tag of the evaluation of the launch's first round, constant while it runs
+    __device__ __forceinline__ unsigned *tag0() const { return reinterpret_cast<unsigned *>(rule + n); }
 };
 
 __host__ __device__ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // control block: header | cmd | active | cpre | gpre | frame states | rule records | first tags
 __host__ __device__ inline size_t ctl_layout(int n, size_t *o_active, size_t *o_cpre, size_t *o_gpre, size_t *o_fs,
-                                             size_t *o_rule, size_t *o_tag) {
+                                             size_t *o_rule) {
     size_t off = align256(sizeof(CtlHeader));
     off = align256(off + sizeof(int) * (size_t)n);          // cmd
     *o_active = off;                                        // two copies of each list array
@@ -154,15 +155,13 @@ __host__ __device__ inline size_t ctl_layout(int n, size_t *o_active, size_t *o_
     *o_fs = off;
     off = (off + sizeof(FrameState) * (size_t)n + 15) & ~(size_t)15;
     *o_rule = off;
-    off += sizeof(uint4) * (size_t)n;
-    *o_tag = off;
-    off = align256(off + sizeof(unsigned) * (size_t)n);
+    off = align256(off + (sizeof(uint4) + sizeof(unsigned)) * (size_t)n);   // Ctl::tag0 behind the records
     return off;
 }
 
 __device__ inline Ctl make_ctl(char *base, int n) {
-    size_t oa, oc, og, of, orl, ot;
-    ctl_layout(n, &oa, &oc, &og, &of, &orl, &ot);
+    size_t oa, oc, og, of, orl;
+    ctl_layout(n, &oa, &oc, &og, &of, &orl);
     Ctl c;
     c.h = (CtlHeader *)base;
     c.cmd = (int *)(base + align256(sizeof(CtlHeader)));
@@ -172,7 +171,6 @@ __device__ inline Ctl make_ctl(char *base, int n) {
     c.n = n;
     c.fs = (FrameState *)(base + of);
     c.rule = (uint4 *)(base + orl);
-    c.tag0 = (unsigned *)(base + ot);
     return c;
 }
 
@@ -246,10 +244,13 @@ constexpr unsigned TAG_MASK = 0x0fffffffu;
 // rounds completed.  It is not read from the state: a block that has no work of the frame waits for none of the
 // frame's control steps and may read a state that is already an evaluation ahead.  The rest of such a rule is
 // never used (a list in which the block has work of the frame is followed by another read), a tag kept from it
-// would stay wrong.
+// would stay wrong.  With STATE_TAG it is read from the state: a launch of one frame, whose list does not change,
+// so that a block without work stays without (read from the control block there, an evaluation at 2048 x 2048 takes
+// 0.6 % longer: other code for the pixel pass).
 __device__ __forceinline__ unsigned frame_tag(const Ctl &C, int f, int rounds) {
-    return (__ldcg(C.tag0 + f) + (unsigned)rounds) & TAG_MASK;
+    return (__ldcg(C.tag0() + f) + (unsigned)rounds) & TAG_MASK;
 }
+template <bool STATE_TAG = false>
 __device__ __forceinline__ FInfo frame_info(const Ctl &C, int f, int rounds) {
     const FrameState *S = C.fs + f;
     FInfo fi;
@@ -261,7 +262,7 @@ __device__ __forceinline__ FInfo frame_info(const Ctl &C, int f, int rounds) {
     fi.alpha = __ldcg(&S->alpha);
     fi.beta = __ldcg(&S->beta);
     fi.mode = (st == ST_EVAL) ? 0 : ((rs || k == 0) ? 2 : 1);
-    fi.tag = frame_tag(C, f, rounds);
+    fi.tag = STATE_TAG ? ((unsigned)__ldcg(&S->n_evals) + 1u) & TAG_MASK : frame_tag(C, f, rounds);
     return fi;
 }
 
@@ -568,7 +569,8 @@ struct ChunkWork {
 
 // The sum over the warp of values v >= 0 (or NaN): the values as 54-bit fixed-point numbers relative to
 // the largest, summed by integer warp reductions (a double-float butterfly takes five dependent steps of
-// two shuffles and an 11-operation sum).  Error: 2^-47 of the sum.
+// two shuffles and an 11-operation sum).  Error: below 2^-47 of the sum, and at most 2^-48.0 in 12,000 simulated sums
+// of values of equal and very different size, where the butterfly's is up to 2^-47.0 (RMS 2^-50 to 2^-52 both).
 __device__ __forceinline__ DF warp_sum_nonneg(float v) {
     const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(v)), e = m >> 23;
     if (e < 27u || e >= 255u) return df_warp_sum(DF{v, 0.f});          // tiny, infinite or NaN: the same for all lanes
@@ -1107,7 +1109,7 @@ __device__ void r_init(const d2ic_frame_t *frames, int n_frames, Ctl &C) {
         } else if (ld_vol(&C.fs[f].state) == ST_DONE) {
             C.fs[f].reported = 1;
         }
-        C.tag0[f] = cmd == CMD_INIT ? 1u : ((unsigned)ld_vol(&C.fs[f].n_evals) + 1u) & TAG_MASK;
+        C.tag0()[f] = cmd == CMD_INIT ? 1u : ((unsigned)ld_vol(&C.fs[f].n_evals) + 1u) & TAG_MASK;
     }
     __syncthreads();
     rebuild_active(frames, n_frames, C);
@@ -1412,6 +1414,7 @@ __device__ __forceinline__ void control_step(const d2ic_frame_t *frames, const d
 
 // The active list (n_active = na <= FCACHE) with its prefix sums and each frame's candidate
 // rule after `rounds` completed rounds, copied into the block's shared memory (whole block).
+template <bool STATE_TAG>
 __device__ __forceinline__ void load_list(Ctl &C, int lb, int na, int rounds, int *s_cpre, int *s_gpre, int *s_act,
                                           FRule *s_fi) {
     if (na > FCACHE) return;
@@ -1422,7 +1425,7 @@ __device__ __forceinline__ void load_list(Ctl &C, int lb, int na, int rounds, in
     for (int s = threadIdx.x; s < na; s += NT) {
         const int f = checked_index(__ldcg(C.act(lb) + s), C.n, C.h);
         s_act[s] = f;
-        s_fi[s] = make_rule(frame_info(C, f, rounds));
+        s_fi[s] = make_rule(frame_info<STATE_TAG>(C, f, rounds));
     }
 }
 
@@ -1432,7 +1435,8 @@ __device__ __forceinline__ void load_list(Ctl &C, int lb, int na, int rounds, in
 // a 512 x 512 frame, and 80 against 64 chunks per SM at 2048 x 2048).  Blocks whose warps reduce node
 // groups (group gi: warp gi), and the last block, which runs the control step, take LEAD_PIXELS pixels
 // less than the others: a block's pixel work of about 2.5 us, the time of the node work that comes
-// before the wait for a group's chunks.  (Without it a 512 x 512 round takes 13.8 instead of 12.5 us.)
+// before the wait for a group's chunks.  (Without it an evaluation at 512 x 512 takes 12.2 instead of 10.2 us, at
+// 1024 x 1024 15.6 instead of 14.0, at 2048 x 2048 28.3 instead of 27.0; half of it: 11.6, 14.2 and 27.6.)
 constexpr int LEAD_PIXELS = 2304;
 __device__ __forceinline__ int2 chunk_share(const d2ic_frame_t &F, int total, int tg, int wid) {
     const int nb = (int)gridDim.x, b = (int)blockIdx.x, rb = (tg + NWARP - 1) / NWARP, full = nb - rb - 1;
@@ -1586,11 +1590,11 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
         s_hdr[8] = 0;
     }
     __syncthreads();
-    load_list(C, s_hdr[7], s_hdr[0], 0, s_cpre, s_gpre, s_act, s_fi);
+    load_list<ONE>(C, s_hdr[7], s_hdr[0], 0, s_cpre, s_gpre, s_act, s_fi);
     __syncthreads();
     if (!ONE && s_hdr[0] <= FS) {
         keep_frames(s_hdr[0]);
-        if ((int)threadIdx.x < s_hdr[0]) s_tag0[threadIdx.x] = __ldcg(C.tag0 + s_act[threadIdx.x]);
+        if ((int)threadIdx.x < s_hdr[0]) s_tag0[threadIdx.x] = __ldcg(C.tag0() + s_act[threadIdx.x]);
         __syncthreads();
     }
     if (!ONE) kept = s_hdr[0] <= FS;
@@ -1951,7 +1955,7 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
         if (s_hdr[5] != REFRESH_NONE && !s_hdr[3]) {    // rules from the frame states; a changed list is reloaded
             if (s_hdr[5] == REFRESH_RULES) {
                 if (na <= FCACHE)
-                    for (int s = threadIdx.x; s < na; s += NT) s_fi[s] = make_rule(frame_info(C, s_act[s], s_hdr[6]));
+                    for (int s = threadIdx.x; s < na; s += NT) s_fi[s] = make_rule(frame_info<ONE>(C, s_act[s], s_hdr[6]));
             } else if (s_hdr[0] > 0) {
                 // after direct rounds the rules are the records' (the states may still be on their way); the
                 // new list's frames are among the old one's
@@ -1964,12 +1968,12 @@ __global__ void __launch_bounds__(NT, D2IC_ENGINE_MINB) cg_engine(const d2ic_fra
                     rule = FRule{__uint_as_float(r.z), __uint_as_float(r.w), r.y, frame_tag(C, f, (int)r.x)};
                 }
                 __syncthreads();
-                load_list(C, s_hdr[7], n2, s_hdr[6], s_cpre, s_gpre, s_act, s_fi);
+                load_list<ONE>(C, s_hdr[7], n2, s_hdr[6], s_cpre, s_gpre, s_act, s_fi);
                 if (have) s_fi[t] = rule;                // written by this thread in load_list, too
                 __syncthreads();
                 if (!ONE && n2 <= FS) {
                     keep_frames(n2);
-                    if (t < n2) s_tag0[t] = __ldcg(C.tag0 + s_act[t]);
+                    if (t < n2) s_tag0[t] = __ldcg(C.tag0() + s_act[t]);
                     __syncthreads();
                 }
                 if (!ONE) kept = n2 <= FS;
@@ -2117,8 +2121,8 @@ using namespace d2ic;
 
 extern "C" size_t d2ic_cg_control_bytes(int n_frames) {
     if (n_frames < 1) n_frames = 1;
-    size_t a, b, c, d, e, t;
-    return ctl_layout(n_frames, &a, &b, &c, &d, &e, &t);
+    size_t a, b, c, d, e;
+    return ctl_layout(n_frames, &a, &b, &c, &d, &e);
 }
 
 // Workspace of one frame: 7 node buffers (u x2, g x3, dir x2), the K gradient
