@@ -15,7 +15,7 @@
 // write and one read of node_chunk_k * Nn * 2 * K floats per product).
 //
 // PCG: one cooperative launch runs all iterations of up to 64 columns with the vectors in shared memory
-// (pcg_resident).  Meshes whose vectors do not fit on the chip keep them in memory and run five kernels
+// (pcg_resident).  Meshes whose vectors do not fit on the chip, or only a few columns of many, keep them in memory and run five kernels
 // per iteration: AP = H P with the block partials of P.AP, their column sums, the update of X, R, Z with
 // the partials of R.R and R.Z, their column sums (one warp per column, blocks summed in a fixed order:
 // deterministic) and the new direction; the last block of the second column sum decides convergence
@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(PT) pcg_dir(int n_nodes, int K, const double *
 //
 // Bound by the hops at few columns (two sums and a barrier, about 6 us) and by the double-float
 // arithmetic and the latency of the neighbours' values at many.  Per iteration, five kernels before ->
-// now: 7,569 nodes x 64 columns 66 -> 26 us, 4,331 x 6 55 -> 12 us, 1,089 x 1 (one block) 27 -> 12 us.
+// now: 7,569 nodes x 64 columns 66 -> 26 us, 4,331 x 6 55 -> 12 us, 1,089 x 1 27 -> 11 us.
 constexpr int PR_T = 512;                  // threads per block
 constexpr int PR_PAIR_BYTES = 7 * 8;       // x, r, p (two components, double-float) and two floats of H P
 constexpr int PR_NODE_BYTES = 4 * HOP + 32;   // the operator's column nodes and the preconditioner block
@@ -1356,7 +1356,8 @@ extern "C" int d2ic_hessian_prepare(const d2ic_frame_t *frame_dev, int n_chunks,
     HopView hv;
     int st = assemble(frame_dev, n_chunks, n_nodes, node_chunk_k, chunk_hess, inv_np, alpha_reg, (char *)op, s, &hv);
     if (st) return st;
-    hop_diagonal<<<(n_nodes + 127) / 128, 128, 0, s>>>(frame_dev, hv.sids, hv.sblk, inv_np, alpha_reg, Minv, active);
+    // one warp per block: the FP64 sums and divisions of 7,569 nodes on every SM
+    hop_diagonal<<<(n_nodes + 31) / 32, 32, 0, s>>>(frame_dev, hv.sids, hv.sblk, inv_np, alpha_reg, Minv, active);
     D2IC_CHECK_LAUNCH("hop_diagonal");
     return D2IC_OK;
 }
