@@ -360,8 +360,8 @@ __global__ void __launch_bounds__(32 * MIX_WARPS, 2) mixed_chunks(const d2ic_fra
     if (!__syncthreads_and(inside) && tiled) {
         tiled = false;
         asm volatile("cp.async.wait_all;" ::: "memory");
-        const int i = threadIdx.x;
-        if (i < n) s_ix[i] += x0 + 1 - F.pad - (s_iy[i] - 1 + F.pad - y0) * tw;
+        const int i = threadIdx.x, xo = (int)(origin % F.cpitch), yo = (int)(origin / F.cpitch);   // x0, y0
+        if (i < n) s_ix[i] += xo + 1 - F.pad - (s_iy[i] - 1 + F.pad - yo) * tw;
         __syncthreads();
     }
     for (int b0 = w * per; b0 < n_images; b0 += MIX_WARPS * per) {

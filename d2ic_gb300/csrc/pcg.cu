@@ -152,24 +152,43 @@ __global__ void hop_diagonal(const d2ic_frame_t *__restrict__ fp, const int *__r
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= F.n_nodes) return;
     const size_t Nn = F.n_nodes;
-    double xx = 0.0, xy = 0.0, yy = 0.0;
-    for (int s = 0; s < F.node_chunk_k; ++s) {
-        const size_t e = (size_t)s * Nn + n;
-        const int4 j = __ldg(reinterpret_cast<const int4 *>(sids) + e);   // -1: slot not owned by a chunk
-        const int jj[4] = {j.x, j.y, j.z, j.w};
+    const int K = F.node_chunk_k, md = F.max_deg;
+    double xx = 0.0, xy = 0.0, yy = 0.0, w = 0.0;
+    // loads of a batch in flight together
+    constexpr int QS = 4, QN = 8;
+    for (int s0 = 0; s0 < K; s0 += QS) {
+        int4 j[QS];
 #pragma unroll
-        for (int b = 0; b < 4; ++b)
-            if (jj[b] == n) {
-                const float4 v = __ldg(sblk + 4 * e + b);
-                xx += (double)(inv_np * v.x);
-                xy += (double)(inv_np * v.y);
-                yy += (double)(inv_np * v.z);
-            }
+        for (int t = 0; t < QS; ++t)                       // -1: slot not owned by a chunk
+            j[t] = s0 + t < K ? __ldg(reinterpret_cast<const int4 *>(sids) + (size_t)(s0 + t) * Nn + n)
+                              : make_int4(-1, -1, -1, -1);
+#pragma unroll
+        for (int t = 0; t < QS; ++t) {
+            const int jj[4] = {j[t].x, j[t].y, j[t].z, j[t].w};
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+                if (jj[b] == n) {
+                    const float4 v = __ldg(sblk + 4 * ((size_t)(s0 + t) * Nn + n) + b);
+                    xx += (double)(inv_np * v.x);
+                    xy += (double)(inv_np * v.y);
+                    yy += (double)(inv_np * v.z);
+                }
+        }
     }
-    double w = 0.0;
-    for (int q = 0; q < F.max_deg; ++q) {
-        if (__ldg(F.nbr_index + (size_t)q * Nn + n) < 0) break;
-        w += (double)__ldg(F.nbr_weight + (size_t)q * Nn + n);
+    bool alive = true;                                     // entries after the first -1 are padding
+    for (int q0 = 0; q0 < md && alive; q0 += QN) {
+        int i[QN];
+        float v[QN];
+#pragma unroll
+        for (int t = 0; t < QN; ++t) {
+            i[t] = q0 + t < md ? __ldg(F.nbr_index + (size_t)(q0 + t) * Nn + n) : -1;
+            v[t] = q0 + t < md ? __ldg(F.nbr_weight + (size_t)(q0 + t) * Nn + n) : 0.f;
+        }
+#pragma unroll
+        for (int t = 0; t < QN; ++t) {
+            alive = alive && i[t] >= 0;
+            if (alive) w += (double)v[t];
+        }
     }
     xx += (double)alpha * w;
     yy += (double)alpha * w;

@@ -133,9 +133,11 @@ __global__ void strain_jvp_kernel(const double *__restrict__ du, int K, const do
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int k0 = blockIdx.y * JD, nk = min(JD, K - k0);
     if (i >= n) return;
-    const double *v = du + 2 * (size_t)k0 * n;
+    const double *v1 = du + 2 * (size_t)k0 * n;
+    const double2 *v2 = reinterpret_cast<const double2 *>(v1);
     auto at = [&](size_t e) {
-        return WIDE ? __ldg(reinterpret_cast<const double2 *>(v) + e) : make_double2(__ldg(v + 2 * e), __ldg(v + 2 * e + 1));
+        if constexpr (WIDE) return v2[e];
+        else return make_double2(v1[2 * e], v1[2 * e + 1]);
     };
     const double2 xi = X[i];
     const int d = min(deg[i], md);
