@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(32 * MIX_WARPS, 2) mixed_chunks(const d2ic_fra
                                                                   float2 *__restrict__ slots, size_t coeff_stride,
                                                                   size_t slot_stride, int n_images) {
     extern __shared__ __align__(16) float mix_smem[];
-    __shared__ int s_ix[D2IC_CHUNK_MAX], s_iy[D2IC_CHUNK_MAX];
+    __shared__ int s_at[D2IC_CHUNK_MAX], s_ix[D2IC_CHUNK_MAX], s_iy[D2IC_CHUNK_MAX];
     __shared__ float s_tx[D2IC_CHUNK_MAX], s_ty[D2IC_CHUNK_MAX];
     __shared__ float s_r[D2IC_CHUNK_MAX], s_gx[D2IC_CHUNK_MAX], s_gy[D2IC_CHUNK_MAX];
     __shared__ float s_N[4][D2IC_CHUNK_MAX];
@@ -349,7 +349,8 @@ __global__ void __launch_bounds__(32 * MIX_WARPS, 2) mixed_chunks(const d2ic_fra
         s_gy[i] = gy;
         const int lx = ix - 1 + F.pad - x0, ly = iy - 1 + F.pad - y0;
         inside = (unsigned)lx <= (unsigned)(tw - 4) && (unsigned)ly <= (unsigned)(th - 4);
-        s_ix[i] = tiled ? ly * tw + lx : ix;                   // tiled: the first tap's element of the window
+        s_at[i] = ly * tw + lx;                                // the first tap's element of the window
+        s_ix[i] = ix;
         s_iy[i] = iy;
         s_tx[i] = tx;
         s_ty[i] = ty;
@@ -357,13 +358,7 @@ __global__ void __launch_bounds__(32 * MIX_WARPS, 2) mixed_chunks(const d2ic_fra
         for (int a = 0; a < 4; ++a) s_N[a][i] = q.N[a];
     }
     // every pixel of an element lies inside; one beyond it (a caller's own shape functions) may not: global memory
-    if (!__syncthreads_and(inside) && tiled) {
-        tiled = false;
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        const int i = threadIdx.x, xo = (int)(origin % F.cpitch), yo = (int)(origin / F.cpitch);   // x0, y0
-        if (i < n) s_ix[i] += xo + 1 - F.pad - (s_iy[i] - 1 + F.pad - yo) * tw;
-        __syncthreads();
-    }
+    if (!__syncthreads_and(inside)) tiled = false;
     for (int b0 = w * per; b0 < n_images; b0 += MIX_WARPS * per) {
         const int nb = min(per, n_images - b0);
         float v[8 * MIX];                            // node sums: image j's x of node a at 8 j + 2 a, its y after it
@@ -386,7 +381,7 @@ __global__ void __launch_bounds__(32 * MIX_WARPS, 2) mixed_chunks(const d2ic_fra
                 bspline_w(pair(s_ty[ia], s_ty[ib]), wy, dwy);
                 const Pair r = pair(ga * s_r[ia], gb * s_r[ib]);
                 const Pair gx = pair(ga * s_gx[ia], gb * s_gx[ib]), gy = pair(ga * s_gy[ia], gb * s_gy[ib]);
-                const float *pa = tiles + s_ix[ia], *pc = tiles + s_ix[ib];
+                const float *pa = tiles + s_at[ia], *pc = tiles + s_at[ib];
 #pragma unroll
                 for (int j = 0; j < MIX; ++j) {
                     if (j >= nb) break;
@@ -446,6 +441,7 @@ __global__ void __launch_bounds__(32 * MIX_WARPS, 2) mixed_chunks(const d2ic_fra
         if (j < nb)
             reinterpret_cast<float *>(slots + (size_t)(b0 + j) * slot_stride + (size_t)sla * F.n_nodes + nda)[lane & 1] = v[0];
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");       // windows of a chunk that did without them
 }
 
 // Few images: one image per warp, from global memory, with more blocks per SM and no windows to copy.  The same bits.
