@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(PT) pcg_dir(int n_nodes, int K, const double *
 // halves the exponent of its largest entry, so that FP32's exponent range suffices wherever the FP32 operator's
 // does: with H of size h, P is of size h^-1/2, H P of size h^1/2 and X, kept as h X, of size 1.  (CG with a scaled
 // preconditioner gives the same iterates; powers of two change no bits.)  Errors against CG with FP64 products of the same operator are
-// those of the FP32 products, with these vectors and with FP64 ones: 30 meshes of 330 to 4,212 nodes and 1 to
+// those of the FP32 products, with these vectors and with FP64 ones: 28 meshes of 330 to 4,212 nodes and 1 to
 // 47 columns, 0.9 to 2.2e-7 of the solution's norm at rtol 1e-7, 0.8 to 1.2e-7 at 1e-10 and at 1e-13, each pair alike to
 // three digits and with the same iteration counts.  (Against FP64 vectors with the same FP32 products the solution
 // differs by 4e-13 to 1e-9 of its norm up to 3,000 nodes; CG amplifies any rounding, in 103 iterations on 22,801 nodes
